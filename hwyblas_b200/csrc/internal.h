@@ -123,7 +123,8 @@ enum WorkspaceSlot : int {
   kWsResidual = 32,    // hwyblas_dresidual_dd partial sums
   kWsMixedInv = 33,    // mixed Cholesky: the inverse of a diagonal block
   kWsTrsmBarrier = 34, // cooperative TRSM: its grid barrier counter
-  kNumWorkspaceSlots = 35
+  kWsLuMoves = 35,     // LU panels' lists of moved rows
+  kNumWorkspaceSlots = 36
 };
 
 // Makes `to` wait for the work enqueued on `from` so far.
@@ -189,6 +190,9 @@ size_t DgemmSplitBytes(int m, int n, int k);
 // FP32 (chunks of 384), FFMA on the CUDA cores.
 void Sgemm(int m, int n, int k, float alpha, View<float> a, View<float> b,
            float beta, float* c, int ldc, Part part = kAll, Tri tri = kTriNone);
+// The same without a triangular operand (gemm_f32.cu).
+void SgemmTiles(int m, int n, int k, float alpha, View<float> a, View<float> b, float beta,
+                float* c, int ldc, Part part);
 // C := beta*C on `part` (beta == 0 writes zeros without reading C).
 template <typename T>
 void ScaleMatrix(int m, int n, T beta, T* c, int ldc, Part part = kAll);
@@ -219,6 +223,19 @@ void AdjustPivots(int* ipiv, int begin, int end, int delta);
 template <typename T>
 void GetrfLeaf(int m, int n, T* a, int lda, int* ipiv, int* info, int info_base,
                int leaf_w = 16);
+// Getrf2 of an m x n panel (n <= 64, m >= n) in one launch (lu_panel.cu), if a
+// cluster can hold it; false (and nothing done) otherwise. ipiv gets the
+// panel-relative pivots plus ipiv_add. moves (device, may be null; 2 +
+// kPanelMoves ints, the first zero): the rows that the interchanges moved.
+constexpr int kPanelMoves = 256;
+template <typename T>
+bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,
+                int* moves);
+// The interchanges of the panel at (j, j) of a, jb columns wide, from its list
+// of moved rows, on columns [0, left) and [c0, c0 + nc), and the solve with the
+// panel's unit lower triangle on the latter.
+template <typename T>
+void PanelSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const int* moves);
 // Sets the poll limit of the cooperative leaf's exchange on the current
 // device (0: the default); returns the previous one.
 unsigned int SetLeafWaitLimit(unsigned int polls);

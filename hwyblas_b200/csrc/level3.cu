@@ -789,6 +789,10 @@ void TrsmRec(bool left, View<T> tri, bool lower, bool unit, int r, int other,
 
 void Sgemm(int m, int n, int k, float alpha, View<float> a, View<float> b,
            float beta, float* c, int ldc, Part part, Tri tri) {
+  if (tri == kTriNone) {
+    SgemmTiles(m, n, k, alpha, a, b, beta, c, ldc, part);
+    return;
+  }
   const dim3 grid((m + kSB - 1) / kSB, (n + kSB - 1) / kSB);
   SgemmKernel<<<grid, 256, 0, Ctx().stream>>>(m, n, k, alpha, a, b, beta, c, ldc,
                                               static_cast<int>(part),
