@@ -33,6 +33,7 @@ T* At(T* a, int lda, int i, int j) {
 template <typename T>
 void GetrfRec(int m, int n, T* a, int lda, int* ipiv, int* info, int col0) {
   if (m == 0 || n == 0) return;
+  if (GetrfPanel<T>(m, n, a, lda, ipiv, 0, info, col0, nullptr)) return;
   if (std::min(m, n) <= 16) {
     GetrfLeaf<T>(m, n, a, lda, ipiv, info, col0);
     return;
@@ -82,41 +83,63 @@ void Getrf(int m, int n, T* a, int lda, int* ipiv, int* info) {
   // The context stream's persistent GEMMs leave kSideSms SMs free, so that
   // the side stream's panel runs beside them rather than after them.
   const int cap = side.ok ? std::max(1, ctx.num_sms - kSideSms) : 0;
-  // The trailing work of panel j on columns [c0, c0 + nc).
-  const auto update = [&](int j, int jb, int c0, int nc) {
-    Laswp<T>(nc, At(a, lda, 0, c0), lda, j + 1, j + jb, ipiv, 1);
-    TrsmFull<T>(true, true, false, true, jb, nc, T(1), At(a, lda, j, j), lda,
-                At(a, lda, j, c0), lda);
-    if (j + jb < m) {
+  // Panel j in one launch leaves a list of the rows that its interchanges
+  // moved, which the interchanges and the triangular solve of the other
+  // columns then take in one launch too; a panel that is too tall for it is
+  // factored by the recursion and followed by LASWP and TRSM.
+  constexpr int kList = 2 + kPanelMoves;
+  const size_t list_bytes = sizeof(int) * kList * static_cast<size_t>((mn + nb - 1) / nb);
+  int* lists = static_cast<int*>(Workspace(kWsLuMoves, list_bytes));
+  if (lists == nullptr) return;
+  cudaMemsetAsync(lists, 0, list_bytes, main);
+  bool listed = false;  // whether the panel last factored left its list
+  const auto panel = [&](int j, int jb) {
+    T* at = At(a, lda, j, j);
+    listed = GetrfPanel<T>(m - j, jb, at, lda, ipiv + j, j, info, j, lists + j / nb * kList);
+    if (!listed) {
+      GetrfRec<T>(m - j, jb, at, lda, ipiv + j, info, j);
+      AdjustPivots(ipiv, j, j + jb, j);
+    }
+  };
+  // The trailing work of panel j on columns [c0, c0 + nc); `left` columns left
+  // of the panel take its interchanges.
+  const auto update = [&](int j, int jb, int left, int c0, int nc, bool list) {
+    if (list) {
+      PanelSwapTrsm<T>(j, jb, left, c0, nc, a, lda, lists + j / nb * kList);
+    } else {
+      Laswp<T>(left, a, lda, j + 1, j + jb, ipiv, 1);
+      if (nc > 0) {
+        Laswp<T>(nc, At(a, lda, 0, c0), lda, j + 1, j + jb, ipiv, 1);
+        TrsmFull<T>(true, true, false, true, jb, nc, T(1), At(a, lda, j, j), lda,
+                    At(a, lda, j, c0), lda);
+      }
+    }
+    if (nc > 0 && j + jb < m) {
       GemmFull<T>(false, false, m - j - jb, nc, jb, T(-1), At(a, lda, j + jb, j), lda,
                   At(a, lda, j, c0), lda, T(1), At(a, lda, j + jb, c0), lda);
     }
   };
   StreamAfter(side.to_side, main, look);
-  OnSide([&] { GetrfRec<T>(m, std::min(nb, mn), a, lda, ipiv, info, 0); });
+  OnSide([&] { panel(0, std::min(nb, mn)); });
   for (int j = 0; j < mn; j += nb) {
     const int jb = std::min(mn - j, nb);
     const int right = n - j - jb;               // columns right of the panel
     const int next = std::min(nb, right);       // the next panel's columns
     const int jb2 = std::min(mn - j - jb, nb);  // the next panel's width
+    const bool list = listed;
     StreamAfter(side.to_side, main, look);
-    OnSide([&] { AdjustPivots(ipiv, j, std::min(m, j + jb), j); });
     StreamAfter(side.to_main, look, main);
     if (next > 0) {
       OnSide([&] {
         ctx.side_leaf = side.ok;
-        update(j, jb, j + jb, next);
-        if (jb2 > 0) GetrfRec<T>(m - j - jb, jb2, At(a, lda, j + jb, j + jb), lda,
-                                 ipiv + j + jb, info, j + jb);
+        update(j, jb, 0, j + jb, next, list);
+        if (jb2 > 0) panel(j + jb, jb2);
         ctx.side_leaf = false;
       });
     }
-    Laswp<T>(j, a, lda, j + 1, j + jb, ipiv, 1);
-    if (right > next) {
-      ctx.sm_cap = cap;
-      update(j, jb, j + jb + next, right - next);
-      ctx.sm_cap = 0;
-    }
+    ctx.sm_cap = right > next ? cap : 0;
+    update(j, jb, j, j + jb + next, std::max(0, right - next), list);
+    ctx.sm_cap = 0;
   }
   StreamAfter(side.to_main, look, main);
 }

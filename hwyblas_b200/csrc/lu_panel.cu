@@ -1,0 +1,647 @@
+// The LU panel (at most 64 columns) in one launch, and the interchanges and
+// triangular solve that follow it.
+//
+// GetrfPanelKernel factors an m x w panel (w <= 64, m >= w) with the
+// reference's recursion (src/lapack/getrf.cc:112-207: halves down to leaves of
+// at most 16 columns, factor_kernels.cc:79-183) and each element's operations
+// in the reference's order. It is bound by the latency of its w dependent
+// pivot searches, so everything between two of them stays on the chip: a
+// thread-block cluster holds the panel in shared memory, one row a thread,
+// and a leaf's 16 columns in registers. Rows are never interchanged: each
+// thread keeps the position its row has after the interchanges so far (ties
+// of the pivot search go to the first position), and the rows go to their
+// positions when the panel is written. Per column: the warps' maxima by
+// redux on the bits of |x|, one block barrier, the block's candidate row sent
+// to every CTA of the cluster by st.async (one one-way trip; the receiving
+// mbarrier counts the bytes), and every warp picks the winner by itself.
+// After a leaf, every CTA collects its pivot rows' other columns and solves
+// the small triangles for itself.
+#include <algorithm>
+#include <cstdio>
+
+#include "device.cuh"
+#include "internal.h"
+#include "ref_order.cuh"
+
+namespace hb {
+namespace {
+
+constexpr int kPanelW = 64;        // columns
+constexpr int kPanelLeaf = 16;     // src/lapack/factor_kernels.h:27
+constexpr int kPanelThreads = 512;  // rows of a CTA at most
+constexpr int kPanelCtas = 16;
+// Polls of a wait for the other CTAs' candidates: each lasts up to the
+// hardware's suspend time, far above any real wait in total.
+constexpr uint32_t kPanelPolls = 1u << 20;
+
+// A CTA's candidate of one column: the row's leaf columns, the reciprocal of
+// its pivot, its key, position and place in the panel.
+template <typename T>
+struct __align__(16) PanelSlot {
+  T row[kPanelLeaf];
+  unsigned long long key;
+  int pos, place;
+  T rinv;
+};
+
+template <typename T>
+struct PanelArgs {
+  int m, w, R, lanes;  // R: rows of a CTA
+  T* a;
+  long long lda;
+  int* ipiv;
+  int ipiv_add;
+  int* info;
+  int info_base;
+  int* moves;  // count, unused, then (position, row) of every row that moved
+  int* timeout_flag;
+};
+
+// Order of the pivot search: larger |x|, NaN below everything (0).
+__device__ __forceinline__ unsigned long long PivotKey(double x) {
+  const double v = fabs(x);
+  return isnan(v) ? 0ull : static_cast<unsigned long long>(__double_as_longlong(v)) + 1;
+}
+__device__ __forceinline__ unsigned long long PivotKey(float x) {
+  const float v = fabsf(x);
+  return isnan(v) ? 0ull : static_cast<unsigned long long>(__float_as_uint(v)) + 1;
+}
+
+// The warp's largest key and the smallest position holding it.
+template <typename T>
+__device__ __forceinline__ void WarpBest(unsigned long long& key, int& pos) {
+  const unsigned lo = static_cast<unsigned>(key), hi = static_cast<unsigned>(key >> 32);
+  unsigned mhi = 0;
+  bool top = true;
+  if constexpr (sizeof(T) == 8) {
+    mhi = __reduce_max_sync(0xffffffffu, hi);
+    top = hi == mhi;
+  }
+  const unsigned mlo = __reduce_max_sync(0xffffffffu, top ? lo : 0u);
+  pos = __reduce_min_sync(0xffffffffu, top && lo == mlo ? pos : 0x7fffffff);
+  key = (static_cast<unsigned long long>(mhi) << 32) | mlo;
+}
+
+__device__ __forceinline__ uint32_t MapRank(uint32_t addr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+// 16 bytes to another CTA's shared memory, counted on its mbarrier.
+__device__ __forceinline__ void StAsync16(uint32_t dst, ulonglong2 v, uint32_t bar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];"
+      :
+      : "r"(dst), "l"(v.x), "l"(v.y), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ double LoadRemote(uint32_t addr, double) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float LoadRemote(uint32_t addr, float) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void ClusterBarrier() {
+  asm volatile(
+      "barrier.cluster.arrive.release.aligned;\n\t"
+      "barrier.cluster.wait.acquire.aligned;" ::
+          : "memory");
+}
+
+// U := L^-1 U for the n1 pivot rows at `rows` (stride kPanelW; L unit lower in
+// their columns [0, n1), U in columns [n1, n1 + n2)): one column a lane, each
+// element's chain over q ascending (src/trsm-inl.h:107-174).
+template <typename T, int N>
+__device__ __forceinline__ void PanelSolve(T* rows, int n1, int n2) {
+  const int c = threadIdx.x;
+  if (c >= n2) return;
+  T y[N];
+#pragma unroll
+  for (int s = 0; s < N; ++s) y[s] = s < n1 ? rows[s * kPanelW + n1 + c] : T(0);
+#pragma unroll
+  for (int q = 0; q + 1 < N; ++q) {
+    if (q + 1 >= n1) break;
+#pragma unroll
+    for (int s = q + 1; s < N; ++s)
+      if (s < n1) y[s] = fma(-y[q], rows[s * kPanelW + q], y[s]);
+  }
+#pragma unroll
+  for (int s = 0; s < N; ++s)
+    if (s < n1) rows[s * kPanelW + n1 + c] = y[s];
+}
+
+// Four consecutive elements from shared memory, 16-byte loads if aligned.
+template <typename T, bool kVec>
+__device__ __forceinline__ void Load4Shared(const T* p, T (&v)[4]) {
+  if constexpr (kVec && sizeof(T) == 8) {
+    const double2 x = reinterpret_cast<const double2*>(p)[0];
+    const double2 y = reinterpret_cast<const double2*>(p)[1];
+    v[0] = x.x, v[1] = x.y, v[2] = y.x, v[3] = y.y;
+  } else if constexpr (kVec) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = p[i];
+  }
+}
+
+// Two rows of the trailing update: X(r, c) = -sum_q L(r, q) U(q, c) + X(r, c)
+// for cw (8 or 16) columns, each sum one chain over q (alpha -1, beta 1).
+template <typename T, bool kVec>
+__device__ __forceinline__ void PanelUpdate(const T* l, T* x, int R, const T* u, int n1, int nc,
+                                            int cw, int ra, int rb, bool ina, bool inb) {
+  T acc[2][kPanelLeaf];
+#pragma unroll
+  for (int c = 0; c < kPanelLeaf; ++c) acc[0][c] = acc[1][c] = T(0);
+  for (int q = 0; q < n1; ++q) {
+    const T la = l[q * R + ra], lb = l[q * R + rb];
+#pragma unroll
+    for (int c4 = 0; c4 < kPanelLeaf / 4; ++c4) {
+      if (c4 >= 2 && cw <= 8) break;
+      T uv[4];
+      Load4Shared<T, kVec>(u + q * kPanelW + c4 * 4, uv);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        acc[0][c4 * 4 + e] = fma(la, uv[e], acc[0][c4 * 4 + e]);
+        acc[1][c4 * 4 + e] = fma(lb, uv[e], acc[1][c4 * 4 + e]);
+      }
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < kPanelLeaf; ++c) {
+    if (c >= nc) continue;
+    if (ina) x[c * R + ra] = T(-1) * acc[0][c] + x[c * R + ra];
+    if (inb) x[c * R + rb] = T(-1) * acc[1][c] + x[c * R + rb];
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p) {
+  extern __shared__ __align__(16) unsigned char panel_smem[];
+  const int P = gridDim.x, cta = blockIdx.x, R = p.R, w = p.w;
+  PanelSlot<T>* slots = reinterpret_cast<PanelSlot<T>*>(panel_smem);  // [2][kPanelCtas]
+  T* prow = reinterpret_cast<T*>(slots + 2 * kPanelCtas);            // [w][kPanelW] pivot rows
+  T* S = prow + w * kPanelW;                                         // [w][R] this CTA's rows
+  __shared__ PanelSlot<T> s_mine;
+  __shared__ unsigned long long s_wkey[2][kPanelThreads / 32];
+  __shared__ int s_wpos[2][kPanelThreads / 32];
+  __shared__ int s_place[kPanelW], s_pos[kPanelThreads], s_op[7][4];
+  __shared__ __align__(8) uint64_t s_bar[2];
+  __shared__ int s_ops;
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, nwarps = blockDim.x / 32;
+  const int place = cta * R + tid;
+  const bool valid = tid < R && place < p.m;
+  int pos = place;
+
+  if (tid == 0) {
+    MbarInit(&s_bar[0], 1);
+    MbarInit(&s_bar[1], 1);
+    FenceBarrierInit();
+    // The recursion's steps: leaves (columns c0.., n) and, between the halves
+    // of a block (n1 and n2 columns), its solve and update.
+    int ops = 0;
+    const auto op = [&](int leaf, int c0, int n1, int n2) {
+      s_op[ops][0] = leaf, s_op[ops][1] = c0, s_op[ops][2] = n1, s_op[ops][3] = n2;
+      ++ops;
+    };
+    const auto half = [&](int c0, int n) {
+      if (n <= kPanelLeaf) {
+        op(1, c0, n, 0);
+      } else {
+        const int n1 = n / 2;
+        op(1, c0, n1, 0);
+        op(0, c0, n1, n - n1);
+        op(1, c0 + n1, n - n1, 0);
+      }
+    };
+    if (w <= kPanelLeaf) {
+      op(1, 0, w, 0);
+    } else {
+      half(0, w / 2);
+      op(0, 0, w / 2, w - w / 2);
+      half(w / 2, w - w / 2);
+    }
+    s_ops = ops;
+  }
+  if (valid) {
+    const T* src = p.a + place;
+#pragma unroll 1
+    for (int c0 = 0; c0 < w; c0 += 16) {
+      T v[16];
+#pragma unroll
+      for (int c = 0; c < 16; ++c)
+        if (c0 + c < w) v[c] = src[(c0 + c) * p.lda];
+#pragma unroll
+      for (int c = 0; c < 16; ++c)
+        if (c0 + c < w) S[(c0 + c) * R + tid] = v[c];
+    }
+  }
+  // Every CTA's mbarriers are ready before any candidate is sent.
+  if (P > 1) ClusterBarrier();
+  else __syncthreads();
+
+  // A wait that gives up: the CTA skips the rest but keeps taking part in the
+  // cluster's barriers, so that no CTA exits while others read its rows.
+  bool timed_out = false, alive = true;
+  for (int op = 0; op < s_ops; ++op) {
+    const int c0 = s_op[op][1], n1 = s_op[op][2], n2 = s_op[op][3];
+    if (s_op[op][0] != 0) {
+      T x[kPanelLeaf];
+#pragma unroll
+      for (int k = 0; k < kPanelLeaf; ++k)
+        x[k] = valid && k < n1 ? S[(c0 + k) * R + tid] : T(0);
+#pragma unroll
+      for (int j = 0; j < kPanelLeaf; ++j) {
+        if (j >= n1 || !alive) break;
+        const int jc = c0 + j, par = jc & 1;
+        // The warp's candidate among the rows not yet taken (position >= jc). A
+        // NaN at position jc wins, as the reference's search starts from it.
+        const bool in = valid && pos >= jc;
+        unsigned long long key = in ? PivotKey(x[j]) : 0ull;
+        if (in && pos == jc && key == 0) key = sizeof(T) == 8 ? ~0ull : 0xffffffffull;
+        int best = pos;
+        WarpBest<T>(key, best);
+        if (lane == 0) {
+          s_wkey[par][warp] = key;
+          s_wpos[par][warp] = best;
+        }
+        const T rinv = T(1) / x[j];
+        if (__syncthreads_or(timed_out)) {
+          alive = false;
+          break;
+        }
+        // The block's, found by every warp; the warp that holds the row sends it.
+        key = lane < nwarps ? s_wkey[par][lane] : 0ull;
+        best = lane < nwarps ? s_wpos[par][lane] : 0x7fffffff;
+        WarpBest<T>(key, best);
+        const bool mine = in && key != 0 && pos == best;
+        if (__any_sync(0xffffffffu, mine) || (key == 0 && warp == 0)) {
+          if (mine) {
+#pragma unroll
+            for (int k = 0; k < kPanelLeaf; ++k) s_mine.row[k] = x[k];
+            s_mine.rinv = rinv;
+            s_mine.place = place;
+          }
+          if (mine || (key == 0 && lane == 0)) {
+            s_mine.key = key;
+            s_mine.pos = best;
+          }
+          __syncwarp();
+          if (P > 1) {
+            constexpr int kPieces = sizeof(PanelSlot<T>) / 16;
+            const ulonglong2* src = reinterpret_cast<const ulonglong2*>(&s_mine);
+            const uint32_t dst = SmemAddr(&slots[par * kPanelCtas + cta]);
+            const uint32_t bar = SmemAddr(&s_bar[par]);
+            for (int i = lane; i < P * kPieces; i += 32) {
+              const int to = i / kPieces, e = i % kPieces;
+              StAsync16(MapRank(dst + 16 * e, to), src[e], MapRank(bar, to));
+            }
+          }
+        }
+        const PanelSlot<T>* win = &s_mine;
+        if (P > 1) {
+          if (tid == 0)
+            MbarArriveExpectTx(&s_bar[par], P * static_cast<uint32_t>(sizeof(PanelSlot<T>)));
+          uint32_t polls = 0;
+          while (!MbarTryWait(&s_bar[par], (jc >> 1) & 1)) {
+            if (++polls >= kPanelPolls) {
+              atomicExch(p.timeout_flag, 1);
+              timed_out = true;  // every thread learns of it at the next block barrier
+              break;
+            }
+          }
+          key = lane < P ? slots[par * kPanelCtas + lane].key : 0ull;
+          best = lane < P ? slots[par * kPanelCtas + lane].pos : 0x7fffffff;
+          const unsigned long long own_key = key;
+          const int own_pos = best;
+          WarpBest<T>(key, best);
+          const unsigned hit = __ballot_sync(0xffffffffu, own_key == key && own_pos == best);
+          win = &slots[par * kPanelCtas + ((__ffs(hit) - 1) & (kPanelCtas - 1))];
+        } else {
+          __syncthreads();
+        }
+        const int piv = win->pos;
+        const T pivot = win->row[j];
+        if (tid < n1) prow[jc * kPanelW + c0 + tid] = win->row[tid];
+        if (tid == 0) {
+          s_place[jc] = win->place;
+          if (cta == 0) {
+            p.ipiv[jc] = piv + 1 + p.ipiv_add;
+            if (pivot == T(0) && *p.info == 0) *p.info = p.info_base + jc + 1;
+          }
+        }
+        // A zero pivot is at position jc already.
+        if (pos == piv) pos = jc;
+        else if (pos == jc) pos = piv;
+        if (valid && pos > jc) {
+          // The column below the pivot times its reciprocal (divided if the
+          // pivot is below the safe minimum, kept if it is zero), then the
+          // rank-1 update of the leaf's later columns.
+          if (pivot != T(0))
+            x[j] = !(fabs(pivot) >= Sfmin<T>()) ? x[j] / pivot : x[j] * win->rinv;
+          const int len = p.m - jc - 1;
+#pragma unroll
+          for (int k = j + 1; k < kPanelLeaf; ++k)
+            x[k] = Axpy(x[k], -win->row[k], x[j], len, p.lanes);
+        }
+      }
+      if (valid && pos >= c0 + n1) {
+#pragma unroll
+        for (int k = 0; k < kPanelLeaf; ++k)
+          if (k < n1) S[(c0 + k) * R + tid] = x[k];
+      }
+      s_pos[tid] = valid ? pos : -1;
+      if (w > n1) {
+        // The leaf's pivot rows' other columns, from the CTAs that hold them
+        // (these rows change no more).
+        if (__syncthreads_or(timed_out)) alive = false;
+        if (P > 1) ClusterBarrier();
+        const int other = w - n1;
+        for (int i = tid; alive && i < n1 * other; i += blockDim.x) {
+          const int s = i / other, cc = i % other, col = cc < c0 ? cc : cc + n1;
+          const int from = s_place[c0 + s], owner = from / R;
+          const T* at = S + col * R + (from - owner * R);
+          prow[(c0 + s) * kPanelW + col] =
+              P > 1 ? LoadRemote(MapRank(SmemAddr(at), owner), T(0)) : *at;
+        }
+        __syncthreads();
+      }
+    } else if (alive) {
+      T* rows = prow + c0 * kPanelW + c0;
+      if (warp == 0) {
+        if (n1 <= kPanelLeaf) PanelSolve<T, 16>(rows, n1, n2);
+        else PanelSolve<T, 32>(rows, n1, n2);
+      }
+      __syncthreads();
+      // Half the threads take the first cw columns of two rows each, the other
+      // half the rest.
+      const int cw = n2 > 16 ? 16 : 8, half = (R + 1) / 2;
+      const int blk = tid >= half ? 1 : 0, ra = tid - blk * half;
+      const int rb = min(ra + half, R - 1), nc = min(cw, n2 - blk * cw);
+      if (ra < half && nc > 0) {
+        const int cb = n1 + blk * cw;
+        const bool ina = s_pos[ra] >= c0 + n1;
+        const bool inb = ra + half < R && s_pos[rb] >= c0 + n1;
+        if ((c0 + cb) % (16 / static_cast<int>(sizeof(T))) == 0)
+          PanelUpdate<T, true>(S + c0 * R, S + (c0 + cb) * R, R, rows + cb, n1, nc, cw, ra, rb,
+                               ina, inb);
+        else
+          PanelUpdate<T, false>(S + c0 * R, S + (c0 + cb) * R, R, rows + cb, n1, nc, cw, ra, rb,
+                                ina, inb);
+      }
+      __syncthreads();
+    }
+  }
+  if (!__syncthreads_or(timed_out) && alive) {
+    for (int c = cta; c < w; c += P)
+      for (int r = tid; r < w; r += blockDim.x) p.a[r + c * p.lda] = prow[r * kPanelW + c];
+    if (valid && pos >= w) {
+      T* dst = p.a + pos;
+#pragma unroll 4
+      for (int c = 0; c < w; ++c) dst[c * p.lda] = S[c * R + tid];
+    }
+    if (valid && pos != place && p.moves != nullptr) {
+      const int e = atomicAdd(p.moves, 1);
+      p.moves[2 + 2 * e] = pos;
+      p.moves[3 + 2 * e] = place;
+    }
+  }
+  // No CTA exits while another may read or write its shared memory.
+  if (P > 1) ClusterBarrier();
+}
+
+template <typename T>
+size_t PanelSmem(int w, int R) {
+  return 2 * kPanelCtas * sizeof(PanelSlot<T>) +
+         sizeof(T) * static_cast<size_t>(w) * (kPanelW + R);
+}
+
+constexpr size_t kPanelSmemMax = 227 * 1024 - 8 * 1024;  // beside the static arrays
+
+// CTAs and rows a CTA for an m x w panel; false if it does not fit a cluster
+// of at most `most` CTAs.
+template <typename T>
+bool PanelShape(int m, int w, int most, int* ctas, int* rows) {
+  int fit = kPanelThreads;
+  while (fit > 0 && PanelSmem<T>(w, fit) > kPanelSmemMax) fit -= 32;
+  if (fit <= 0) return false;
+  const int least = (m + fit - 1) / fit;
+  if (least > most) return false;
+  // A row a thread: about 256 rows a CTA balance the exchange (more CTAs) with
+  // the updates (more rows).
+  const int want = std::max(least, std::min(most, (m + 255) / 256));
+  *ctas = want;
+  *rows = (m + want - 1) / want;
+  return true;
+}
+
+// Interchanges as a list of moved rows (position, row), applied to a block of
+// columns, and for the columns right of a panel the solve with its unit lower
+// triangle L (jb x jb, jb <= 64): B := L^-1 P B on the panel's rows
+// (src/lapack/getrf.cc:28-81, src/trsm.cc:87-135). Bound by latency: a CTA owns
+// kSwapCols columns, a warp kSwapCols / 8 of them, a lane one of a column's
+// rows, and the solved values go round by shuffles, so that a solve of 32
+// rows is 32 steps whatever the width.
+constexpr int kSwapThreads = 256, kSwapCols = 16, kMovesMax = 2 * kPanelW;
+
+template <typename T>
+struct SwapArgs {
+  int jb, left, nc;  // columns [0, left) only move; [c0, c0 + nc) are solved too
+  T* a;              // row j of the matrix
+  long long lda, c0;
+  const T* l;        // the panel's triangle, leading dimension lda
+  const int* moves;
+};
+
+// 32-row solves and products of one warp's two columns, lane = row; st: the
+// row's part of the triangle, st[q] for column q.
+template <typename T>
+__device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[2]) {
+  const int lane = threadIdx.x % 32;
+  for (int q = 0; q + 1 < r; ++q) {
+    const T l = lrow[q];
+    const T y0 = __shfl_sync(0xffffffffu, y[0], q), y1 = __shfl_sync(0xffffffffu, y[1], q);
+    if (lane > q) {
+      y[0] = fma(-y0, l, y[0]);
+      y[1] = fma(-y1, l, y[1]);
+    }
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kSwapThreads) PanelSwapTrsmKernel(SwapArgs<T> p) {
+  constexpr int kLd = kPanelW + 1;
+  __shared__ int s_dst[kMovesMax], s_src[kMovesMax], s_top[kPanelW];
+  __shared__ T s_l[kPanelW * kLd];
+  __shared__ T s_b[kSwapCols][kLd];
+  const int tid = threadIdx.x, jb = p.jb;
+  const int cnt = min(p.moves[0], kMovesMax);
+  const int left_blocks = (p.left + kSwapCols - 1) / kSwapCols;
+  const bool solve = static_cast<int>(blockIdx.x) >= left_blocks;
+  const int first = (solve ? blockIdx.x - left_blocks : blockIdx.x) * kSwapCols;
+  const int cols = min(kSwapCols, (solve ? p.nc : p.left) - first);
+  T* b = p.a + (solve ? p.c0 + first : first) * p.lda;
+  if (tid < cnt) {
+    s_dst[tid] = p.moves[2 + 2 * tid];
+    s_src[tid] = p.moves[3 + 2 * tid];
+  }
+  if (tid < kPanelW) s_top[tid] = tid;
+  if (solve) {
+    for (int i = tid; i < jb * jb; i += kSwapThreads) {
+      const int r = i % jb, c = i / jb;
+      s_l[r * kLd + c] = p.l[r + c * p.lda];
+    }
+  }
+  __syncthreads();
+  if (solve && tid < cnt && s_dst[tid] < jb) s_top[s_dst[tid]] = s_src[tid];
+  __syncthreads();
+  // Every value that moves is read before any is written.
+  constexpr int kPer = kMovesMax * kSwapCols / kSwapThreads;
+  T v[kPer];
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int e = (tid + i * kSwapThreads) % kMovesMax, c = (tid + i * kSwapThreads) / kMovesMax;
+    if (e < cnt && c < cols && !(solve && s_dst[e] < jb)) v[i] = b[s_src[e] + c * p.lda];
+  }
+  if (solve) {
+    for (int i = tid; i < kPanelW * kSwapCols; i += kSwapThreads) {
+      const int r = i % kPanelW, c = i / kPanelW;
+      s_b[c][r] = r < jb && c < cols ? b[s_top[r] + c * p.lda] : T(0);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int e = (tid + i * kSwapThreads) % kMovesMax, c = (tid + i * kSwapThreads) / kMovesMax;
+    if (e < cnt && c < cols && !(solve && s_dst[e] < jb)) b[s_dst[e] + c * p.lda] = v[i];
+  }
+  if (!solve) return;
+  // The recursion's split (src/trsm.cc:87-135): 32 rows, the product, the rest.
+  const int r1 = min(jb, 32), r2 = jb - r1, lane = tid % 32, c = tid / 32 * 2;
+  static_assert(kSwapCols == 2 * (kSwapThreads / 32), "two columns a warp");
+  const T* l1 = s_l + min(lane, jb - 1) * kLd;
+  T y[2] = {s_b[c][lane], s_b[c + 1][lane]};
+  LaneSolve<T>(l1, r1, y);
+  T z[2] = {T(0), T(0)};
+  if (r2 > 0) {
+    const T* l2 = s_l + min(32 + lane, jb - 1) * kLd;
+    T acc[2] = {T(0), T(0)};
+#pragma unroll 4
+    for (int q = 0; q < 32; ++q) {
+      const T l = l2[q];
+      acc[0] = fma(l, __shfl_sync(0xffffffffu, y[0], q), acc[0]);
+      acc[1] = fma(l, __shfl_sync(0xffffffffu, y[1], q), acc[1]);
+    }
+    z[0] = T(-1) * acc[0] + s_b[c][32 + lane];
+    z[1] = T(-1) * acc[1] + s_b[c + 1][32 + lane];
+    LaneSolve<T>(l2 + 32, r2, z);
+  }
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {
+    if (c + d >= cols) continue;
+    T* col = b + (c + d) * p.lda;
+    if (lane < r1) col[lane] = y[d];
+    if (lane < r2) col[32 + lane] = z[d];
+  }
+}
+
+}  // namespace
+
+template <typename T>
+bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,
+                int* moves) {
+  Context& ctx = Ctx();
+  PanelArgs<T> args;
+  int ctas = 0;
+  if (n < 1 || n > kPanelW || m < n) return false;
+  static const int max_cluster = [] {
+    const void* fn = reinterpret_cast<const void*>(GetrfPanelKernel<T>);
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kPanelSmemMax)) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kPanelCtas);
+    cfg.blockDim = dim3(kPanelThreads);
+    cfg.dynamicSmemBytes = kPanelSmemMax;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = kPanelCtas;
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int size = 0;
+    if (cudaOccupancyMaxPotentialClusterSize(&size, fn, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      size = 1;
+    }
+    return std::min(size, kPanelCtas);
+  }();
+  // Beside a capped trailing update a cluster of at most 8 CTAs finds its SMs
+  // in one GPC soonest; larger panels take what they need.
+  if (!PanelShape<T>(m, n, std::min(max_cluster, 8), &ctas, &args.R) &&
+      !PanelShape<T>(m, n, max_cluster, &ctas, &args.R))
+    return false;
+  args.m = m;
+  args.w = n;
+  args.lanes = sizeof(T) == 8 ? RefLanesDouble() : 2 * RefLanesDouble();
+  args.a = a;
+  args.lda = lda;
+  args.ipiv = ipiv;
+  args.ipiv_add = ipiv_add;
+  args.info = info;
+  args.info_base = info_base;
+  args.moves = moves;
+  args.timeout_flag = ctx.dev_status;
+  cudaEvent_t t0 = KernelTimerStart(kFamilyLuLeaf, ctx.stream);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3((args.R + 31) / 32 * 32);
+  cfg.dynamicSmemBytes = PanelSmem<T>(n, args.R);
+  cfg.stream = ctx.stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ctas;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  Failed(cudaLaunchKernelEx(&cfg, GetrfPanelKernel<T>, args), "getrf panel");
+  KernelTimerStop(t0, ctx.stream);
+  CountLaunch();
+  LaunchFailed("getrf panel");
+  return true;
+}
+template bool GetrfPanel<double>(int, int, double*, int, int*, int, int*, int, int*);
+template bool GetrfPanel<float>(int, int, float*, int, int*, int, int*, int, int*);
+
+template <typename T>
+void PanelSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const int* moves) {
+  const int blocks = (left + kSwapCols - 1) / kSwapCols + (nc + kSwapCols - 1) / kSwapCols;
+  if (blocks == 0) return;
+  SwapArgs<T> args;
+  args.jb = jb;
+  args.left = left;
+  args.nc = nc;
+  args.a = a + j;
+  args.lda = lda;
+  args.c0 = c0;
+  args.l = a + j + static_cast<long long>(j) * lda;
+  args.moves = moves;
+  PanelSwapTrsmKernel<T><<<blocks, kSwapThreads, 0, Ctx().stream>>>(args);
+  CountLaunch();
+  LaunchFailed("panel interchanges");
+}
+template void PanelSwapTrsm<double>(int, int, int, int, int, double*, int, const int*);
+template void PanelSwapTrsm<float>(int, int, int, int, int, float*, int, const int*);
+
+}  // namespace hb
