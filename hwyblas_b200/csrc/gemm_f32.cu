@@ -41,47 +41,64 @@ __device__ __forceinline__ void CpAsyncF32(float* dst, const float* src, bool in
   }
 }
 
-// One slab of an operand: s[q * LD + x] = op(x0 + x, k0 + q) for x < B and
-// q < 16, zero outside (extent, k). xs, qs: the strides of x and q in memory.
-// vec: x is contiguous and every group of four x (x0 + x a multiple of 4) is
-// 16-byte aligned.
-template <int B, int LD, int Threads>
-__device__ __forceinline__ void LoadSlab(float* s, const float* p, long long xs, long long qs,
-                                         int x0, int k0, int extent, int k, bool vec) {
-  if (vec) {
+// How an operand's slabs are copied: groups of four x (x contiguous and
+// 16-byte aligned), single x (contiguous), single q (q contiguous; transposed on
+// the way in).
+enum SlabMode : int { kSlabVec = 0, kSlabX = 1, kSlabQ = 2 };
+
+// One operand's slabs: s[q * LD + x] = op(x0 + x, k0 + q) for x < B and
+// q < 16, zero outside. A thread's first element is fixed and the steps between
+// its elements are constants, so a slab costs a pointer and one address a copy.
+template <int Mode, int B, int LD, int Threads>
+struct SlabLoader {
+  static constexpr int kPer = Mode == kSlabVec ? 4 : 1;
+  static constexpr int kCopies = B * kF32Kb / Threads / kPer;
+  static constexpr int kDx = Mode == kSlabQ ? Threads / kF32Kb : 0;
+  static constexpr int kDq = Mode == kSlabQ ? 0 : Threads * kPer / B;
+  const float* p;  // this thread's first element of the next slab
+  int left;        // elements of the operand from its first x on
+
+  static __device__ __forceinline__ int X() {
+    return Mode == kSlabQ ? threadIdx.x / kF32Kb : threadIdx.x % (B / kPer) * kPer;
+  }
+  static __device__ __forceinline__ int Q() {
+    return Mode == kSlabQ ? threadIdx.x % kF32Kb : threadIdx.x / (B / kPer);
+  }
+  __device__ __forceinline__ SlabLoader(const float* data, long long ld, int x0, int n)
+      : p(Mode == kSlabQ ? data + (x0 + X()) * ld + Q() : data + (x0 + X()) + Q() * ld),
+        left(n - x0 - X()) {}
+  // kend: rows of the slab that exist (16 but for the last). `safe` is an
+  // address for copies that read nothing.
+  __device__ __forceinline__ void Load(float* s, int kend, long long ld, const float* safe) {
+    float* dst = s + Q() * LD + X();
 #pragma unroll
-    for (int l = 0; l < B * kF32Kb / 4 / Threads; ++l) {
-      const int idx = threadIdx.x + l * Threads;
-      const int x = idx % (B / 4) * 4, q = idx / (B / 4);
-      float* dst = s + q * LD + x;
-      const bool row = k0 + q < k;
-      if (x0 + x + 3 < extent || !row) {
-        const float* src = p + (x0 + x) + (k0 + q) * qs;
-        CpAsyncF32<16>(dst, row ? src : p, row);
-      } else {
+    for (int l = 0; l < kCopies; ++l) {
+      const float* src = p + (Mode == kSlabQ ? l * kDx * ld : l * kDq * ld);
+      float* to = dst + l * (kDq * LD + kDx);
+      const bool row = Q() + l * kDq < kend;
+      if constexpr (Mode == kSlabVec) {
+        if (left >= 4) {
+          CpAsyncF32<16>(to, row ? src : safe, row);
+        } else {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const bool in = x0 + x + e < extent;
-          CpAsyncF32<4>(dst + e, in ? p + (x0 + x + e) + (k0 + q) * qs : p, in);
+          for (int e = 0; e < 4; ++e)
+            CpAsyncF32<4>(to + e, row && e < left ? src + e : safe, row && e < left);
         }
+      } else {
+        const bool in = row && l * kDx < left;
+        CpAsyncF32<4>(to, in ? src : safe, in);
       }
     }
-    return;
+    p += Mode == kSlabQ ? kF32Kb : kF32Kb * ld;
   }
-  const bool along_x = xs == 1;
-#pragma unroll
-  for (int l = 0; l < B * kF32Kb / Threads; ++l) {
-    const int idx = threadIdx.x + l * Threads;
-    const int x = along_x ? idx % B : idx / kF32Kb, q = along_x ? idx / B : idx % kF32Kb;
-    const bool in = x0 + x < extent && k0 + q < k;
-    CpAsyncF32<4>(s + q * LD + x, in ? p + (x0 + x) * xs + (k0 + q) * qs : p, in);
-  }
-}
+};
 
-__device__ __forceinline__ unsigned long long Pack2(float lo, float hi) {
-  unsigned long long v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-  return v;
+__device__ __forceinline__ unsigned long long Swap2(unsigned long long v) {
+  unsigned long long r;
+  asm("{\n\t.reg .b32 lo, hi;\n\tmov.b64 {lo, hi}, %1;\n\tmov.b64 %0, {hi, lo};\n\t}"
+      : "=l"(r)
+      : "l"(v));
+  return r;
 }
 // Two IEEE FMAs (round to nearest) at once.
 __device__ __forceinline__ void Fma2(unsigned long long& d, unsigned long long a,
@@ -102,10 +119,11 @@ __device__ __forceinline__ bool CrossingTileF32(int part, int m, int n, int i, i
   return !(i0 + mr - 1 < j0);
 }
 
-template <int WM, int WN, bool kPart>
+template <int WM, int WN, bool kPart, int ModeA, int ModeB>
 __global__ void __launch_bounds__(F32Tile<WM, WN>::kThreads, 512 / F32Tile<WM, WN>::kThreads)
-    SgemmTileKernel(int m, int n, int k, float alpha, View<float> a, View<float> b, float beta,
-                    float* c, long long ldc, int part, int veca, int vecb, const int* guard) {
+    SgemmTileKernel(int m, int n, int k, float alpha, const float* a, long long lda,
+                    const float* b, long long ldb, float beta, float* c, long long ldc, int part,
+                    const int* guard) {
   using Cfg = F32Tile<WM, WN>;
   constexpr int BM = Cfg::kBM, BN = Cfg::kBN, SA = Cfg::kSA, SB = Cfg::kSB;
   if (guard != nullptr && *guard != 0) return;
@@ -118,16 +136,20 @@ __global__ void __launch_bounds__(F32Tile<WM, WN>::kThreads, 512 / F32Tile<WM, W
   // likewise with 16.
   const int row0 = warp % WM * 64 + lane % 8 * 4, col0 = warp / WM * 32 + lane / 8 * 4;
   const int slabs = (k + kF32Kb - 1) / kF32Kb;
+  SlabLoader<ModeA, BM, SA, Cfg::kThreads> la(a, lda, m0, m);
+  SlabLoader<ModeB, BN, SB, Cfg::kThreads> lb(b, ldb, n0, n);
   const auto load = [&](int slab) {
     if (slab < slabs) {
       float* sa = f32_smem + slab % kF32Stages * Cfg::kStage;
-      LoadSlab<BM, SA, Cfg::kThreads>(sa, a.data, a.rs, a.cs, m0, slab * kF32Kb, m, k, veca);
-      LoadSlab<BN, SB, Cfg::kThreads>(sa + kF32Kb * SA, b.data, b.cs, b.rs, n0, slab * kF32Kb,
-                                      n, k, vecb);
+      la.Load(sa, k - slab * kF32Kb, lda, a);
+      lb.Load(sa + kF32Kb * SA, k - slab * kF32Kb, ldb, b);
     }
     CpAsyncCommit();
   };
-  unsigned long long acc[4][8];  // row pairs x columns
+  // acc[r][j], rows 2 r and 2 r + 1 of the thread's: the first with column j,
+  // the second with column j ^ 1, so that a packed FMA takes B's columns as
+  // they lie or swapped.
+  unsigned long long acc[4][8];
 #pragma unroll
   for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -143,15 +165,18 @@ __global__ void __launch_bounds__(F32Tile<WM, WN>::kThreads, 512 / F32Tile<WM, W
     const auto step = [&](int q) {
       const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(sa + q * SA);
       const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(sa + q * SA + 32);
-      const float4 b0 = *reinterpret_cast<const float4*>(sb + q * SB);
-      const float4 b1 = *reinterpret_cast<const float4*>(sb + q * SB + 16);
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(sb + q * SB);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(sb + q * SB + 16);
       const unsigned long long av[4] = {a0.x, a0.y, a1.x, a1.y};
-      const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+      const unsigned long long bv[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const unsigned long long bb = Pack2(bv[j], bv[j]);
+      for (int j = 0; j < 4; ++j) {
+        const unsigned long long swapped = Swap2(bv[j]);
 #pragma unroll
-        for (int r = 0; r < 4; ++r) Fma2(acc[r][j], av[r], bb);
+        for (int r = 0; r < 4; ++r) {
+          Fma2(acc[r][2 * j], av[r], bv[j]);
+          Fma2(acc[r][2 * j + 1], av[r], swapped);
+        }
       }
     };
     const int k0 = slab * kF32Kb;
@@ -182,7 +207,7 @@ __global__ void __launch_bounds__(F32Tile<WM, WN>::kThreads, 512 / F32Tile<WM, W
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const int di = e / 4 * 32 + e % 4;
-          const unsigned long long pair = acc[e / 4 * 2 + e % 4 / 2][jj + d];
+          const unsigned long long pair = acc[e / 4 * 2 + e % 4 / 2][(jj + d) ^ (e % 2)];
           const float r =
               alpha * __uint_as_float(static_cast<unsigned>(e % 2 == 0 ? pair : pair >> 32));
           float v;
@@ -201,36 +226,63 @@ __global__ void __launch_bounds__(F32Tile<WM, WN>::kThreads, 512 / F32Tile<WM, W
   }
 }
 
-template <int WM, int WN, bool kPart>
-void LaunchTile(int m, int n, int k, float alpha, View<float> a, View<float> b, float beta,
-                float* c, int ldc, Part part) {
+struct TileCall {
+  int m, n, k;
+  float alpha;
+  View<float> a, b;
+  float beta;
+  float* c;
+  int ldc;
+  Part part;
+};
+
+template <int WM, int WN, bool kPart, int ModeA, int ModeB>
+void LaunchModes(const TileCall& t) {
   using Cfg = F32Tile<WM, WN>;
   static const cudaError_t attr =
-      cudaFuncSetAttribute(SgemmTileKernel<WM, WN, kPart>,
+      cudaFuncSetAttribute(SgemmTileKernel<WM, WN, kPart, ModeA, ModeB>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
   if (Failed(attr, "sgemm attributes")) return;
-  const auto aligned = [](const float* p, long long stride) {
-    return reinterpret_cast<uintptr_t>(p) % 16 == 0 && stride % 4 == 0;
-  };
-  const int veca = a.rs == 1 && aligned(a.data, a.cs), vecb = b.cs == 1 && aligned(b.data, b.rs);
-  const dim3 grid((m + Cfg::kBM - 1) / Cfg::kBM, (n + Cfg::kBN - 1) / Cfg::kBN);
-  SgemmTileKernel<WM, WN, kPart><<<grid, Cfg::kThreads, Cfg::kSmem, Ctx().stream>>>(
-      m, n, k, alpha, a, b, beta, c, ldc, static_cast<int>(part), veca, vecb, Ctx().guard);
+  const dim3 grid((t.m + Cfg::kBM - 1) / Cfg::kBM, (t.n + Cfg::kBN - 1) / Cfg::kBN);
+  SgemmTileKernel<WM, WN, kPart, ModeA, ModeB>
+      <<<grid, Cfg::kThreads, Cfg::kSmem, Ctx().stream>>>(
+          t.m, t.n, t.k, t.alpha, t.a.data, t.a.ld(), t.b.data, t.b.ld(), t.beta, t.c, t.ldc,
+          static_cast<int>(t.part), Ctx().guard);
   CountLaunch();
   LaunchFailed("sgemm tile");
+}
+
+// The copy mode of an operand whose x has stride xs and whose q has stride qs.
+int ModeOf(const float* p, long long xs, long long qs) {
+  if (xs != 1) return kSlabQ;
+  return reinterpret_cast<uintptr_t>(p) % 16 == 0 && qs % 4 == 0 ? kSlabVec : kSlabX;
+}
+
+template <int WM, int WN, bool kPart, int ModeA>
+void LaunchModeA(const TileCall& t, int mode_b) {
+  if (mode_b == kSlabVec) LaunchModes<WM, WN, kPart, ModeA, kSlabVec>(t);
+  else if (mode_b == kSlabX) LaunchModes<WM, WN, kPart, ModeA, kSlabX>(t);
+  else LaunchModes<WM, WN, kPart, ModeA, kSlabQ>(t);
+}
+
+template <int WM, int WN, bool kPart>
+void LaunchTile(const TileCall& t) {
+  const int ma = ModeOf(t.a.data, t.a.rs, t.a.cs), mb = ModeOf(t.b.data, t.b.cs, t.b.rs);
+  if (ma == kSlabVec) LaunchModeA<WM, WN, kPart, kSlabVec>(t, mb);
+  else if (ma == kSlabX) LaunchModeA<WM, WN, kPart, kSlabX>(t, mb);
+  else LaunchModeA<WM, WN, kPart, kSlabQ>(t, mb);
 }
 
 }  // namespace
 
 void SgemmTiles(int m, int n, int k, float alpha, View<float> a, View<float> b, float beta,
                 float* c, int ldc, Part part) {
+  const TileCall t = {m, n, k, alpha, a, b, beta, c, ldc, part};
   const long long big = static_cast<long long>((m + 127) / 128) * ((n + 127) / 128);
   if (big >= Ctx().num_sms)
-    part == kAll ? LaunchTile<2, 4, false>(m, n, k, alpha, a, b, beta, c, ldc, part)
-                 : LaunchTile<2, 4, true>(m, n, k, alpha, a, b, beta, c, ldc, part);
+    part == kAll ? LaunchTile<2, 4, false>(t) : LaunchTile<2, 4, true>(t);
   else
-    part == kAll ? LaunchTile<1, 2, false>(m, n, k, alpha, a, b, beta, c, ldc, part)
-                 : LaunchTile<1, 2, true>(m, n, k, alpha, a, b, beta, c, ldc, part);
+    part == kAll ? LaunchTile<1, 2, false>(t) : LaunchTile<1, 2, true>(t);
 }
 
 }  // namespace hb
