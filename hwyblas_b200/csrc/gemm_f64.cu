@@ -26,6 +26,7 @@
 // phase hit 8 distinct chunks), and MMA column g takes tile column
 // [0,2,4,6,1,3,5,7][g] of its 8-column block (the 16 lanes of each 64-bit
 // load phase hit 16 distinct 8-byte slots).
+#include <cooperative_groups.h>
 #include <cuda.h>
 
 #include <algorithm>
@@ -838,6 +839,131 @@ __global__ void __launch_bounds__(256)
   p.c[i + j * p.ldc] = cv;
 }
 
+// Small products (few tiles of 32 x 32): bound by latency, so the operands are
+// staged in shared memory by wide cp.async slabs of 64 k (8 bytes a copy: any
+// alignment and either order of an operand) and the chains run on the tensor
+// pipe, one 16 x 8 tile a warp; the KC chunks of k, whose chains are
+// independent, are dealt to the CTAs of a cluster, which then merge them in
+// order through distributed shared memory. One thread an element from global
+// memory (DgemmDirectKernel) waited on every term: 33 x 47 x 65 11 us,
+// 64 x 64 x 1000 45 us.
+constexpr int kSmT = 32, kSmK = 64, kSmLd = kSmT + 4, kSmThreads = 256, kSmCluster = 8;
+constexpr int kSmStage = 2 * kSmK * kSmLd;  // doubles
+constexpr int kSmMaxParts = 16;             // chunks a CTA at most
+
+// One slab of an operand: s[q * kSmLd + x] = op(x0 + x, k0 + q), kend of its 64 q
+// exist. Past them: `fill` (A -0, B +0, so that the products are -0 and leave
+// every sum as it is).
+__device__ __forceinline__ void SmallSlab(double* s, const double* p, long long xs, long long qs,
+                                          int left, int kend, double fill) {
+  const bool along_x = xs == 1;
+#pragma unroll
+  for (int l = 0; l < kSmT * kSmK / kSmThreads; ++l) {
+    const int idx = threadIdx.x + l * kSmThreads;
+    const int x = along_x ? idx % kSmT : idx / kSmK, q = along_x ? idx / kSmT : idx % kSmK;
+    double* to = s + q * kSmLd + x;
+    if (x < left && q < kend) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(SmemAddr(to)),
+                   "l"(p + x * xs + q * qs)
+                   : "memory");
+    } else {
+      *to = fill;
+    }
+  }
+}
+
+// Merges chunk c's sum (already times alpha) into an element, as the reference
+// merges its KC chunks.
+__device__ __forceinline__ double SmallMerge(const GemmParams& p, int i, int j, int c, double r,
+                                             double cv) {
+  if (c != 0) return r + cv;
+  if (p.beta == 0.0) return r;
+  const double cin = p.c[i + j * p.ldc];
+  if (p.beta == 1.0) return r + cin;
+  if (p.part != kAll && InCrossingTile(p.part, p.m, p.n, i, j)) return r + p.beta * cin;
+  return fma(cin, p.beta, r);
+}
+
+__global__ void __launch_bounds__(kSmThreads, 3)
+    DgemmSmallKernel(GemmParams p, View<double> a, View<double> b, int S) {
+  if (p.guard != nullptr && *p.guard != 0) return;
+  extern __shared__ __align__(16) double sm_smem[];
+  double* parts = sm_smem + 2 * kSmStage;  // [chunk / S][column][row]
+  const int rank = blockIdx.x % S, tile = blockIdx.x / S;
+  const int mt = (p.m + kSmT - 1) / kSmT;
+  const int m0 = tile % mt * kSmT, n0 = tile / mt * kSmT;
+  // A tile wholly outside the triangle has nothing to do (nor has its cluster).
+  if (p.part == kLower && m0 + kSmT - 1 < n0) return;
+  if (p.part == kUpper && m0 > n0 + kSmT - 1) return;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane >> 2, t = lane & 3;
+  const int wr = warp % 2, wc = warp / 2;  // tile rows 16 wr, columns 8 wc
+  const double* pa = a.data + m0 * a.rs;
+  const double* pb = b.data + n0 * b.cs;
+  // This CTA's slabs in turn: chunks rank, rank + S, ..., 64 k at a time.
+  const auto next = [&](int k0) {
+    k0 += kSmK;
+    return k0 % 256 == 0 ? k0 + (S - 1) * 256 : k0;
+  };
+  const auto load = [&](int k0, int buf) {
+    if (k0 < p.k) {
+      double* s = sm_smem + buf * kSmStage;
+      SmallSlab(s, pa + k0 * a.cs, a.rs, a.cs, p.m - m0, p.k - k0, -0.0);
+      SmallSlab(s + kSmK * kSmLd, pb + k0 * b.rs, b.cs, b.rs, p.n - n0, p.k - k0, 0.0);
+    }
+    CpAsyncCommit();
+  };
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  int buf = 0, part = 0;
+  load(rank * 256, 0);
+  for (int k0 = rank * 256; k0 < p.k; k0 = next(k0), buf ^= 1) {
+    load(next(k0), buf ^ 1);
+    CpAsyncWait<1>();
+    __syncthreads();
+    const double* sa = sm_smem + buf * kSmStage + t * kSmLd + wr * 16 + g;
+    const double* sb = sm_smem + buf * kSmStage + (kSmK + t) * kSmLd + wc * 8 + g;
+    const int steps = (min(kSmK, p.k - k0) + 7) / 8;
+#pragma unroll 2
+    for (int ks = 0; ks < steps; ++ks) {
+      const double* fa = sa + ks * 8 * kSmLd;
+      const double* fb = sb + ks * 8 * kSmLd;
+      asm volatile(
+          "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
+          "{%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+          : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
+          : "d"(fa[0]), "d"(fa[8]), "d"(fa[4 * kSmLd]), "d"(fa[4 * kSmLd + 8]), "d"(fb[0]),
+            "d"(fb[4 * kSmLd]));
+    }
+    __syncthreads();
+    if (S > 1 && (k0 + kSmK) % 256 != 0 && k0 + kSmK < p.k) continue;
+    if (S == 1 && k0 + kSmK < p.k) continue;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int i = wr * 16 + g + (e >> 1) * 8, j = wc * 8 + 2 * t + (e & 1);
+      if (S > 1) {
+        parts[part * kSmT * kSmT + j * kSmT + i] = acc[e];
+      } else if (m0 + i < p.m && n0 + j < p.n && InPart(p, m0 + i, n0 + j)) {
+        p.c[m0 + i + (n0 + j) * p.ldc] = SmallMerge(p, m0 + i, n0 + j, 0, p.alpha * acc[e], 0.0);
+      }
+      acc[e] = 0.0;
+    }
+    ++part;
+  }
+  if (S == 1) return;
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  cluster.sync();
+  for (int e = rank * kSmThreads + threadIdx.x; e < kSmT * kSmT; e += S * kSmThreads) {
+    const int i = m0 + e % kSmT, j = n0 + e / kSmT;
+    if (i >= p.m || j >= p.n || !InPart(p, i, j)) continue;
+    double cv = 0.0;
+#pragma unroll 4
+    for (int c = 0; c < p.nchunks; ++c)
+      cv = SmallMerge(p, i, j, c,
+                      p.alpha * cluster.map_shared_rank(parts, c % S)[c / S * kSmT * kSmT + e], cv);
+    p.c[i + j * p.ldc] = cv;
+  }
+  cluster.sync();  // no CTA exits while another reads its sums
+}
+
 // Copies op(X) (rows x cols, strided view) into a dense column-major buffer
 // with leading dimension ld, through a 32 x 32 shared tile so that both the
 // read (along X's contiguous dimension) and the write are coalesced.
@@ -965,10 +1091,65 @@ size_t DgemmSplitBytes(int m, int n, int k) {
                                                                                      : 0;
 }
 
+namespace {
+// Products for DgemmSmallKernel: those of at most a few million multiply-adds
+// or with a side below 32, and larger ones whose (tile, chunk) pairs still fit
+// the SMs about twice.
+bool SmallTakes(int m, int n, int k, bool small) {
+  const int nchunks = (k + 255) / 256, S = std::min(nchunks, kSmCluster);
+  const long long ctas = static_cast<long long>((m + kSmT - 1) / kSmT) * ((n + kSmT - 1) / kSmT) * S;
+  if ((nchunks + S - 1) / S > kSmMaxParts || ctas > (1LL << 30)) return false;
+  return small || ctas <= 2LL * Ctx().num_sms;
+}
+
+void DgemmSmall(int m, int n, int k, double alpha, View<double> a, View<double> b, double beta,
+                double* c, int ldc, Part part) {
+  Context& ctx = Ctx();
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      DgemmSmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      static_cast<int>(sizeof(double)) * (2 * kSmStage + kSmMaxParts * kSmT * kSmT));
+  if (Failed(attr, "dgemm small attributes")) return;
+  GemmParams p = {};
+  p.m = m;
+  p.n = n;
+  p.k = k;
+  p.alpha = alpha;
+  p.beta = beta;
+  p.c = c;
+  p.ldc = ldc;
+  p.part = part;
+  p.tri = kTriNone;
+  p.nchunks = (k + 255) / 256;
+  p.timeout_flag = ctx.dev_status;
+  p.guard = ctx.guard;
+  const int S = std::min(p.nchunks, kSmCluster), parts = S > 1 ? (p.nchunks + S - 1) / S : 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>((m + kSmT - 1) / kSmT) * ((n + kSmT - 1) / kSmT) * S);
+  cfg.blockDim = dim3(kSmThreads);
+  cfg.dynamicSmemBytes = sizeof(double) * (2 * kSmStage + parts * kSmT * kSmT);
+  cfg.stream = ctx.stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = S;
+  at.val.clusterDim.y = 1;
+  at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = S > 1 ? 1 : 0;
+  Failed(cudaLaunchKernelEx(&cfg, DgemmSmallKernel, p, a, b, S), "dgemm small");
+  CountLaunch();
+  LaunchFailed("dgemm small");
+}
+}  // namespace
+
 void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
            double beta, double* c, int ldc, Part part, Tri tri) {
   Context& ctx = Ctx();
-  if (static_cast<long long>(m) * n * k <= (1LL << 22) || m < 32 || n < 32) {
+  const bool small = static_cast<long long>(m) * n * k <= (1LL << 22) || m < 32 || n < 32;
+  if (tri == kTriNone && SmallTakes(m, n, k, small)) {
+    DgemmSmall(m, n, k, alpha, a, b, beta, c, ldc, part);
+    return;
+  }
+  if (small) {
     GemmParams p;
     p.m = m;
     p.n = n;
