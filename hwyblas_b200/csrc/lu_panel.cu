@@ -7,10 +7,13 @@
 // in the reference's order. It is bound by the latency of its w dependent
 // pivot searches, so everything between two of them stays on the chip: a
 // thread-block cluster holds the panel in shared memory, one row a thread,
-// and a leaf's 16 columns in registers. Rows are never interchanged: each
-// thread keeps the position its row has after the interchanges so far (ties
-// of the pivot search go to the first position), and the rows go to their
-// positions when the panel is written. Per column: the warps' maxima by
+// and a leaf's remaining columns in registers. Rows are never interchanged:
+// each thread keeps the position its row has after the interchanges so far
+// (ties of the pivot search go to the first position), and the rows go to
+// their positions when the panel is written. The column loop is rolled (the
+// update shifts the registers, so that the current column is always the
+// first): unrolled, its instructions came from L2 once per column, which took
+// longer than the column's work. Per column: the warps' maxima by
 // redux on the bits of |x|, one block barrier, the block's candidate row sent
 // to every CTA of the cluster by st.async (one one-way trip; the receiving
 // mbarrier counts the bytes), and every warp picks the winner by itself.
@@ -28,13 +31,17 @@ namespace {
 
 constexpr int kPanelW = 64;        // columns
 constexpr int kPanelLeaf = 16;     // src/lapack/factor_kernels.h:27
+// Row stride of the pivot rows: 16-byte aligned, few bank conflicts by column.
+template <typename T>
+constexpr int kPanelLd = kPanelW + 16 / static_cast<int>(sizeof(T));
 constexpr int kPanelThreads = 512;  // rows of a CTA at most
+constexpr int kPanelLeast = 256;   // threads at least: the solves share all warps
 constexpr int kPanelCtas = 16;
 // Polls of a wait for the other CTAs' candidates: each lasts up to the
 // hardware's suspend time, far above any real wait in total.
 constexpr uint32_t kPanelPolls = 1u << 20;
 
-// A CTA's candidate of one column: the row's leaf columns, the reciprocal of
+// A CTA's candidate of one column: the row from that column on, the reciprocal of
 // its pivot, its key, position and place in the panel.
 template <typename T>
 struct __align__(16) PanelSlot {
@@ -112,26 +119,38 @@ __device__ __forceinline__ void ClusterBarrier() {
           : "memory");
 }
 
-// U := L^-1 U for the n1 pivot rows at `rows` (stride kPanelW; L unit lower in
-// their columns [0, n1), U in columns [n1, n1 + n2)): one column a lane, each
-// element's chain over q ascending (src/trsm-inl.h:107-174).
-template <typename T, int N>
-__device__ __forceinline__ void PanelSolve(T* rows, int n1, int n2) {
-  const int c = threadIdx.x;
-  if (c >= n2) return;
-  T y[N];
-#pragma unroll
-  for (int s = 0; s < N; ++s) y[s] = s < n1 ? rows[s * kPanelW + n1 + c] : T(0);
-#pragma unroll
-  for (int q = 0; q + 1 < N; ++q) {
-    if (q + 1 >= n1) break;
-#pragma unroll
-    for (int s = q + 1; s < N; ++s)
-      if (s < n1) y[s] = fma(-y[q], rows[s * kPanelW + q], y[s]);
+// Solves with the unit lower triangle, two columns a warp, a lane one row: the
+// solved values go round by shuffles, so that r rows are r - 1 steps and each
+// element's chain runs over q ascending (src/trsm-inl.h:107-174). lrow: the
+// lane's row of the triangle.
+template <typename T>
+__device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[2]) {
+  const int lane = threadIdx.x % 32;
+#pragma unroll 4
+  for (int q = 0; q + 1 < r; ++q) {
+    const T l = lrow[q];
+    const T y0 = __shfl_sync(0xffffffffu, y[0], q), y1 = __shfl_sync(0xffffffffu, y[1], q);
+    if (lane > q) {
+      y[0] = fma(-y0, l, y[0]);
+      y[1] = fma(-y1, l, y[1]);
+    }
   }
-#pragma unroll
-  for (int s = 0; s < N; ++s)
-    if (s < n1) rows[s * kPanelW + n1 + c] = y[s];
+}
+
+// U := L^-1 U for the n1 <= 32 pivot rows at `rows` (stride kPanelLd; L unit
+// lower in their columns [0, n1), U in columns [n1, n1 + n2)).
+template <typename T>
+__device__ __forceinline__ void PanelSolve(T* rows, int n1, int n2) {
+  const int lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
+  T* row = rows + min(lane, n1 - 1) * kPanelLd<T>;
+  for (int c = 2 * (threadIdx.x / 32); c < n2; c += 2 * nwarps) {
+    T y[2] = {row[n1 + c], row[n1 + min(c + 1, n2 - 1)]};
+    LaneSolve<T>(row, n1, y);
+    if (lane < n1) {
+      row[n1 + c] = y[0];
+      if (c + 1 < n2) row[n1 + c + 1] = y[1];
+    }
+  }
 }
 
 // Four consecutive elements from shared memory, 16-byte loads if aligned.
@@ -164,7 +183,7 @@ __device__ __forceinline__ void PanelUpdate(const T* l, T* x, int R, const T* u,
     for (int c4 = 0; c4 < kPanelLeaf / 4; ++c4) {
       if (c4 >= 2 && cw <= 8) break;
       T uv[4];
-      Load4Shared<T, kVec>(u + q * kPanelW + c4 * 4, uv);
+      Load4Shared<T, kVec>(u + q * kPanelLd<T> + c4 * 4, uv);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         acc[0][c4 * 4 + e] = fma(la, uv[e], acc[0][c4 * 4 + e]);
@@ -185,8 +204,8 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
   extern __shared__ __align__(16) unsigned char panel_smem[];
   const int P = gridDim.x, cta = blockIdx.x, R = p.R, w = p.w;
   PanelSlot<T>* slots = reinterpret_cast<PanelSlot<T>*>(panel_smem);  // [2][kPanelCtas]
-  T* prow = reinterpret_cast<T*>(slots + 2 * kPanelCtas);            // [w][kPanelW] pivot rows
-  T* S = prow + w * kPanelW;                                         // [w][R] this CTA's rows
+  T* prow = reinterpret_cast<T*>(slots + 2 * kPanelCtas);            // [w][kPanelLd] pivot rows
+  T* S = prow + w * kPanelLd<T>;                                     // [w][R] this CTA's rows
   __shared__ PanelSlot<T> s_mine;
   __shared__ unsigned long long s_wkey[2][kPanelThreads / 32];
   __shared__ int s_wpos[2][kPanelThreads / 32];
@@ -255,14 +274,13 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
 #pragma unroll
       for (int k = 0; k < kPanelLeaf; ++k)
         x[k] = valid && k < n1 ? S[(c0 + k) * R + tid] : T(0);
-#pragma unroll
-      for (int j = 0; j < kPanelLeaf; ++j) {
-        if (j >= n1 || !alive) break;
+#pragma unroll 1
+      for (int j = 0; j < n1; ++j) {
         const int jc = c0 + j, par = jc & 1;
         // The warp's candidate among the rows not yet taken (position >= jc). A
         // NaN at position jc wins, as the reference's search starts from it.
         const bool in = valid && pos >= jc;
-        unsigned long long key = in ? PivotKey(x[j]) : 0ull;
+        unsigned long long key = in ? PivotKey(x[0]) : 0ull;
         if (in && pos == jc && key == 0) key = sizeof(T) == 8 ? ~0ull : 0xffffffffull;
         int best = pos;
         WarpBest<T>(key, best);
@@ -270,7 +288,7 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
           s_wkey[par][warp] = key;
           s_wpos[par][warp] = best;
         }
-        const T rinv = T(1) / x[j];
+        const T rinv = T(1) / x[0];
         if (__syncthreads_or(timed_out)) {
           alive = false;
           break;
@@ -326,8 +344,8 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
           __syncthreads();
         }
         const int piv = win->pos;
-        const T pivot = win->row[j];
-        if (tid < n1) prow[jc * kPanelW + c0 + tid] = win->row[tid];
+        const T pivot = win->row[0];
+        if (tid < n1 - j) prow[jc * kPanelLd<T> + jc + tid] = win->row[tid];
         if (tid == 0) {
           s_place[jc] = win->place;
           if (cta == 0) {
@@ -341,42 +359,41 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
         if (valid && pos > jc) {
           // The column below the pivot times its reciprocal (divided if the
           // pivot is below the safe minimum, kept if it is zero), then the
-          // rank-1 update of the leaf's later columns.
-          if (pivot != T(0))
-            x[j] = !(fabs(pivot) >= Sfmin<T>()) ? x[j] / pivot : x[j] * win->rinv;
+          // rank-1 update of the leaf's later columns, which move up by one.
+          T l = x[0];
+          if (pivot != T(0)) l = !(fabs(pivot) >= Sfmin<T>()) ? l / pivot : l * win->rinv;
+          S[jc * R + tid] = l;
           const int len = p.m - jc - 1;
+          if (len >= p.lanes) {
 #pragma unroll
-          for (int k = j + 1; k < kPanelLeaf; ++k)
-            x[k] = Axpy(x[k], -win->row[k], x[j], len, p.lanes);
+            for (int k = 1; k < kPanelLeaf; ++k) x[k - 1] = fma(l, -win->row[k], x[k]);
+          } else {
+#pragma unroll
+            for (int k = 1; k < kPanelLeaf; ++k)
+              x[k - 1] = Axpy(x[k], -win->row[k], l, len, p.lanes);
+          }
         }
       }
-      if (valid && pos >= c0 + n1) {
-#pragma unroll
-        for (int k = 0; k < kPanelLeaf; ++k)
-          if (k < n1) S[(c0 + k) * R + tid] = x[k];
-      }
       s_pos[tid] = valid ? pos : -1;
-      if (w > n1) {
-        // The leaf's pivot rows' other columns, from the CTAs that hold them
-        // (these rows change no more).
+      {
+        // The rest of the leaf's pivot rows (the candidates brought their columns
+        // from the pivot to the leaf's end), from the CTAs that hold them; these
+        // rows change no more.
         if (__syncthreads_or(timed_out)) alive = false;
         if (P > 1) ClusterBarrier();
-        const int other = w - n1;
-        for (int i = tid; alive && i < n1 * other; i += blockDim.x) {
-          const int s = i / other, cc = i % other, col = cc < c0 ? cc : cc + n1;
+        for (int i = tid; alive && i < n1 * w; i += blockDim.x) {
+          const int s = i / w, col = i - s * w;
+          if (col >= c0 + s && col < c0 + n1) continue;
           const int from = s_place[c0 + s], owner = from / R;
           const T* at = S + col * R + (from - owner * R);
-          prow[(c0 + s) * kPanelW + col] =
+          prow[(c0 + s) * kPanelLd<T> + col] =
               P > 1 ? LoadRemote(MapRank(SmemAddr(at), owner), T(0)) : *at;
         }
         __syncthreads();
       }
     } else if (alive) {
-      T* rows = prow + c0 * kPanelW + c0;
-      if (warp == 0) {
-        if (n1 <= kPanelLeaf) PanelSolve<T, 16>(rows, n1, n2);
-        else PanelSolve<T, 32>(rows, n1, n2);
-      }
+      T* rows = prow + c0 * kPanelLd<T> + c0;
+      PanelSolve<T>(rows, n1, n2);
       __syncthreads();
       // Half the threads take the first cw columns of two rows each, the other
       // half the rest.
@@ -399,7 +416,7 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
   }
   if (!__syncthreads_or(timed_out) && alive) {
     for (int c = cta; c < w; c += P)
-      for (int r = tid; r < w; r += blockDim.x) p.a[r + c * p.lda] = prow[r * kPanelW + c];
+      for (int r = tid; r < w; r += blockDim.x) p.a[r + c * p.lda] = prow[r * kPanelLd<T> + c];
     if (valid && pos >= w) {
       T* dst = p.a + pos;
 #pragma unroll 4
@@ -418,7 +435,7 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
 template <typename T>
 size_t PanelSmem(int w, int R) {
   return 2 * kPanelCtas * sizeof(PanelSlot<T>) +
-         sizeof(T) * static_cast<size_t>(w) * (kPanelW + R);
+         sizeof(T) * static_cast<size_t>(w) * (kPanelLd<T> + R);
 }
 
 constexpr size_t kPanelSmemMax = 227 * 1024 - 8 * 1024;  // beside the static arrays
@@ -457,21 +474,6 @@ struct SwapArgs {
   const T* l;        // the panel's triangle, leading dimension lda
   const int* moves;
 };
-
-// 32-row solves and products of one warp's two columns, lane = row; st: the
-// row's part of the triangle, st[q] for column q.
-template <typename T>
-__device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[2]) {
-  const int lane = threadIdx.x % 32;
-  for (int q = 0; q + 1 < r; ++q) {
-    const T l = lrow[q];
-    const T y0 = __shfl_sync(0xffffffffu, y[0], q), y1 = __shfl_sync(0xffffffffu, y[1], q);
-    if (lane > q) {
-      y[0] = fma(-y0, l, y[0]);
-      y[1] = fma(-y1, l, y[1]);
-    }
-  }
-}
 
 template <typename T>
 __global__ void __launch_bounds__(kSwapThreads) PanelSwapTrsmKernel(SwapArgs<T> p) {
@@ -605,7 +607,7 @@ bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info,
   cudaEvent_t t0 = KernelTimerStart(kFamilyLuLeaf, ctx.stream);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);
-  cfg.blockDim = dim3((args.R + 31) / 32 * 32);
+  cfg.blockDim = dim3(std::max(kPanelLeast, (args.R + 31) / 32 * 32));
   cfg.dynamicSmemBytes = PanelSmem<T>(n, args.R);
   cfg.stream = ctx.stream;
   cudaLaunchAttribute attr;
