@@ -163,12 +163,10 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 // TRSM base: solves X*T = B for independent rows of X (src/trsm-inl.h:107-174)
 // with T (r x r, r <= 32) read from a strided view. Columns are solved in
-// "solve order" s = 0..r-1 (column r-1-s for lower, s for upper), two per
-// pass: b_j0 -= x_q t(q, j0) and b_j1 -= x_q t(q, j1) as fma(-x_q, t, b) for
-// every solved q; x_j0 = b_j0 * (1/t(j0, j0)); b_j1 = fma(-x_j0, t(j0, j1), b_j1);
-// x_j1 = b_j1 * (1/t(j1, j1)). One thread owns one row of X; the row is kept
-// in registers indexed in solve order so all register indices are static.
-// Element (row, col q) of X is x[row * xs_row + q * xs_col].
+// "solve order" s = 0..r-1 (column r-1-s for lower, s for upper):
+// b_j -= x_q t(q, j) as fma(-x_q, t, b) for every solved q in that order, then
+// x_j = b_j * (1/t(j, j)). Element (row, col q) of X is
+// x[row * xs_row + q * xs_col].
 // The triangle of a base solve in shared memory, in solve order, and the
 // reciprocals of its diagonal (the CTA's threads share the loads).
 template <typename T>
@@ -206,53 +204,72 @@ __device__ __forceinline__ void StoreX(T* p, T v) {
   else *p = v;
 }
 
-template <typename T, bool kCg>
-__device__ __forceinline__ void BaseSolveRow(const T (*st)[33], const T* sinv, int lower,
-                                             int unit, int r, T* xr, long long xs_col) {
-  T y[32];
+// N rows of X solved by a warp, lane s holding the element of step s: at step q
+// lane q's element is final, goes round by shuffles, and every later lane takes
+// its term, so each element's chain is over q ascending, as above, but the
+// chains of a row run side by side. The loop is rolled: unrolled for one
+// thread a row, a launch fetched a thousand instructions to run each once
+// (10 us; 3 us so), and lanes along a column-major X read it coalesced.
+// xr[i]: row i's first element; rows with i >= n are not touched.
+template <typename T, bool kCg, int N>
+__device__ __forceinline__ void WarpSolve(const T (*st)[33], const T* sinv, int lower, int unit,
+                                          int r, T* const (&xr)[N], int n, long long xs_col) {
+  const int lane = threadIdx.x % 32;
+  const long long at = (lower ? r - 1 - lane : lane) * xs_col;
+  T y[N];
 #pragma unroll
-  for (int s = 0; s < 32; ++s) {
-    if (s < r) y[s] = LoadX<T, kCg>(xr + (lower ? r - 1 - s : s) * xs_col);
-  }
+  for (int i = 0; i < N; ++i) y[i] = i < n && lane < r ? LoadX<T, kCg>(xr[i] + at) : T(0);
+  const T inv = sinv[lane];
+#pragma unroll 2
+  for (int q = 0; q < r; ++q) {
+    const T l = st[q][lane];
 #pragma unroll
-  for (int step = 0; step + 1 < 32; step += 2) {
-    if (step + 2 <= r) {
-      T acc0 = y[step], acc1 = y[step + 1];
-#pragma unroll
-      for (int s = 0; s < step; ++s) {
-        acc0 = fma(-y[s], st[s][step], acc0);
-        acc1 = fma(-y[s], st[s][step + 1], acc1);
-      }
-      if (!unit) acc0 = acc0 * sinv[step];
-      y[step] = acc0;
-      acc1 = fma(-acc0, st[step][step + 1], acc1);
-      if (!unit) acc1 = acc1 * sinv[step + 1];
-      y[step + 1] = acc1;
-    } else if (step < r) {  // odd r: the last column alone
-      T acc = y[step];
-#pragma unroll
-      for (int s = 0; s < step; ++s) acc = fma(-y[s], st[s][step], acc);
-      if (!unit) acc = acc * sinv[step];
-      y[step] = acc;
+    for (int i = 0; i < N; ++i) {
+      const T yq = __shfl_sync(0xffffffffu, unit ? y[i] : y[i] * inv, q);
+      if (lane == q) y[i] = yq;
+      else if (lane > q) y[i] = fma(-yq, l, y[i]);
     }
   }
 #pragma unroll
-  for (int s = 0; s < 32; ++s) {
-    if (s < r) StoreX<T, kCg>(xr + (lower ? r - 1 - s : s) * xs_col, y[s]);
-  }
+  for (int i = 0; i < N; ++i)
+    if (i < n && lane < r) StoreX<T, kCg>(xr[i] + at, y[i]);
 }
 
+// A base solve of many rows: a CTA takes kBaseRows of them, two a warp. Rows
+// that are contiguous in memory across each other (right side) go through
+// shared memory, so that both sides read and write whole sectors.
+constexpr int kBaseThreads = 256, kBaseRows = 2 * kBaseThreads / 32;
 template <typename T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kBaseThreads)
     TrsmBaseKernel(View<T> tri, int lower, int unit, int r, int rows, T* x,
                    long long xs_row, long long xs_col, const int* guard) {
   if (guard != nullptr && *guard != 0) return;
   __shared__ T st[32][33];  // st[s][u] = T(col(s), col(u)) in solve order
   __shared__ T sinv[32];
+  __shared__ T xt[kBaseRows][33];
+  const int row0 = blockIdx.x * kBaseRows, n = min(kBaseRows, rows - row0);
+  const bool across = xs_row == 1;
+  x += row0 * xs_row;
+  if (across) {
+    for (int idx = threadIdx.x; idx < kBaseRows * r; idx += kBaseThreads) {
+      const int i = idx % kBaseRows, s = idx / kBaseRows;
+      if (i < n) xt[i][s] = x[i + s * xs_col];
+    }
+  }
   LoadBaseTriangle(tri, lower, unit, r, st, sinv);
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= rows) return;
-  BaseSolveRow<T, false>(st, sinv, lower, unit, r, x + row * xs_row, xs_col);
+  const int i0 = threadIdx.x / 32 * 2;
+  if (across) {
+    T* const xr[2] = {xt[i0], xt[i0 + 1]};
+    WarpSolve<T, false>(st, sinv, lower, unit, r, xr, n - i0, 1);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < kBaseRows * r; idx += kBaseThreads) {
+      const int i = idx % kBaseRows, s = idx / kBaseRows;
+      if (i < n) x[i + s * xs_col] = xt[i][s];
+    }
+  } else {
+    T* const xr[2] = {x + i0 * xs_row, x + (i0 + 1) * xs_row};
+    WarpSolve<T, false>(st, sinv, lower, unit, r, xr, n - i0, xs_col);
+  }
 }
 
 // Cooperative TRSM of a subtree of the recursion (at most kTcRows rows of
@@ -429,8 +446,6 @@ __global__ void __launch_bounds__(kTcThreads) TrsmCoopKernel(TrsmCoopArgs<T> p) 
   extern __shared__ __align__(16) unsigned char tc_smem[];
   T* sa = reinterpret_cast<T*>(tc_smem);   // kTcKMax x kTcRowsCta
   T* sb = sa + kTcKMax * kTcRowsCta;       // kTcKMax x kTcColsCta
-  const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  const long long nth = static_cast<long long>(gridDim.x) * blockDim.x;
   const auto col = [&](T* x, long long ld) {  // column-major, element (i, j) at x[i + j ld]
     View<T> v;
     v.data = x;
@@ -474,8 +489,12 @@ __global__ void __launch_bounds__(kTcThreads) TrsmCoopKernel(TrsmCoopArgs<T> p) 
         xb = p.b + static_cast<long long>(off) * p.ldb;
       }
       LoadBaseTriangle(t, lo, p.unit, rr, st, sinv);
-      for (long long row = tid; row < p.other; row += nth)
-        BaseSolveRow<T, true>(st, sinv, lo, p.unit, rr, xb + row * xs_row, xs_col);
+      // Rows go to the CTAs in turn, then to their warps.
+      for (long long row = blockIdx.x + static_cast<long long>(gridDim.x) * (threadIdx.x / 32);
+           row < p.other; row += static_cast<long long>(gridDim.x) * (blockDim.x / 32)) {
+        T* const xr[1] = {xb + row * xs_row};
+        WarpSolve<T, true>(st, sinv, lo, p.unit, rr, xr, 1, xs_col);
+      }
       --sp;
       if (!GridBarrier(p.barrier, gridDim.x, ++gen, p.timeout_flag)) return;
       continue;
@@ -673,9 +692,10 @@ __global__ void __launch_bounds__(kTcThreads) TrsmColsKernel(TrsmCoopArgs<double
       t.cs = rs;
       const int lo = !p.lower;
       LoadBaseTriangle(t, lo, p.unit, rr, st, sinv);
-      if (threadIdx.x < w)
-        BaseSolveRow<double, true>(st, sinv, lo, p.unit, rr,
-                                   xb + off + threadIdx.x * p.ldb, 1);
+      for (int j = threadIdx.x / 32; j < w; j += blockDim.x / 32) {
+        double* const xr[1] = {xb + off + j * p.ldb};
+        WarpSolve<double, true>(st, sinv, lo, p.unit, rr, xr, 1, 1);
+      }
       --sp;
       __syncthreads();
       continue;
@@ -820,10 +840,8 @@ void TrsmSolve(bool left, View<T> tri, bool lower, bool unit, int r, int other,
     xs_row = 1;
     xs_col = ldb;
   }
-  const int threads = 128;
-  TrsmBaseKernel<T><<<(other + threads - 1) / threads, threads, 0,
-                      Ctx().stream>>>(t, lo ? 1 : 0, unit ? 1 : 0, r, other, b,
-                                      xs_row, xs_col, Ctx().guard);
+  TrsmBaseKernel<T><<<(other + kBaseRows - 1) / kBaseRows, kBaseThreads, 0, Ctx().stream>>>(
+      t, lo ? 1 : 0, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
   CountLaunch();
   LaunchFailed("trsm base");
 }
