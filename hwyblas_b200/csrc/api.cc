@@ -91,6 +91,10 @@ void Init(ThreadState& st) {
   c.stream = c.own_stream;
   if (Failed(cudaMalloc(&c.dev_status, 4096), "status alloc")) return;
   cudaMemset(c.dev_status, 0, 4096);
+  if (Failed(cudaHostAlloc(&c.host_status, 256, cudaHostAllocMapped), "status alloc") ||
+      Failed(cudaHostGetDevicePointer(&c.wait_flag, c.host_status, 0), "status address"))
+    return;
+  memset(c.host_status, 0, 256);
   st.initialized = true;
 }
 
@@ -149,16 +153,11 @@ bool LaunchFailed(const char* what) { return Failed(cudaGetLastError(), what); }
 
 bool CheckDeviceStatus(const char* what) {
   Context& c = Ctx();
-  int flag = 0;
-  if (Failed(cudaMemcpyAsync(&flag, c.dev_status, sizeof(int),
-                             cudaMemcpyDeviceToHost, c.stream),
-             what) ||
-      Failed(cudaStreamSynchronize(c.stream), what)) {
-    return true;
-  }
-  if (flag != 0) {
+  if (Failed(cudaStreamSynchronize(c.stream), what)) return true;
+  volatile int* flag = c.host_status;
+  if (*flag != 0) {
     fprintf(stderr, "hwyblas_b200: a device wait timed out in %s\n", what);
-    cudaMemsetAsync(c.dev_status, 0, sizeof(int), c.stream);
+    *flag = 0;
     t_state.ctx.last_error = static_cast<int>(cudaErrorLaunchTimeout);
     return true;
   }
@@ -311,12 +310,11 @@ void ResetInfo() {
   cudaMemsetAsync(Ctx().dev_status + 1, 0, sizeof(int), Ctx().stream);
 }
 int ReadInfo() {
-  int v = 0;
-  Failed(cudaMemcpyAsync(&v, Ctx().dev_status + 1, sizeof(int),
-                         cudaMemcpyDeviceToHost, Ctx().stream),
+  Context& c = Ctx();
+  Failed(cudaMemcpyAsync(c.host_status + 1, c.dev_status + 1, sizeof(int),
+                         cudaMemcpyDeviceToHost, c.stream),
          "info out");
-  Failed(cudaStreamSynchronize(Ctx().stream), "sync");
-  return v;
+  return Failed(cudaStreamSynchronize(c.stream), "sync") ? 0 : c.host_status[1];
 }
 
 // ---------------------------------------------------------------------------

@@ -1495,7 +1495,7 @@ void ZGetrfLeaf(int m, int n, R* a, int lda, int* ipiv, int* info, int info_base
       Workspace(kWsLeaf, slot_bytes + sizeof(unsigned int) * 2 * kZLeafMaxP));
   if (args.xchg == nullptr) return;
   args.tags = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(args.xchg) + slot_bytes);
-  args.timeout_flag = ctx.dev_status;
+  args.timeout_flag = ctx.wait_flag;
   if (P > 1 && P <= max_cluster) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(P);

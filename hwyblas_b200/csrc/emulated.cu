@@ -833,7 +833,7 @@ int DgemmEmulated(int m, int n, int k, double alpha, View<double> a,
   p.w = (S > 4) ? static_cast<double*>(Workspace(ws_w, sizeof(double) *
                                                             static_cast<size_t>(m) * n))
                 : nullptr;
-  p.timeout_flag = ctx.dev_status;
+  p.timeout_flag = ctx.wait_flag;
   p.lower_only = lower_only ? 1 : 0;
   p.b_rows = n;
   p.b_off = 0;

@@ -805,7 +805,7 @@ void GetrfLeaf(int m, int n, T* a, int lda, int* ipiv, int* info, int info_base,
       Workspace(kWsLeaf, slot_bytes + sizeof(unsigned int) * 2 * kLeafMaxP));
   args.tags = reinterpret_cast<unsigned int*>(reinterpret_cast<char*>(args.xchg) +
                                               slot_bytes);
-  args.timeout_flag = ctx.dev_status;
+  args.timeout_flag = ctx.wait_flag;
   cudaEvent_t t0 = KernelTimerStart(kFamilyLuLeaf, ctx.stream);
   if (wide || (P > 1 && P <= max_cluster && (!ctx.side_leaf || P <= kLeafSideCluster))) {
     cudaLaunchConfig_t cfg = {};

@@ -1120,7 +1120,7 @@ void DgemmSmall(int m, int n, int k, double alpha, View<double> a, View<double> 
   p.part = part;
   p.tri = kTriNone;
   p.nchunks = (k + 255) / 256;
-  p.timeout_flag = ctx.dev_status;
+  p.timeout_flag = ctx.wait_flag;
   p.guard = ctx.guard;
   const int S = std::min(p.nchunks, kSmCluster), parts = S > 1 ? (p.nchunks + S - 1) / S : 0;
   cudaLaunchConfig_t cfg = {};
@@ -1160,7 +1160,7 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
     p.ldc = ldc;
     p.part = part;
     p.tri = tri;
-    p.timeout_flag = ctx.dev_status;
+    p.timeout_flag = ctx.wait_flag;
     p.guard = ctx.guard;
     const int nc = (k + 255) / 256;
     if (nc == 1) {
@@ -1211,7 +1211,7 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
     p.tri = tri;
     p.partial = nullptr;
     p.nchunks = 1;
-    p.timeout_flag = ctx.dev_status;
+    p.timeout_flag = ctx.wait_flag;
     p.guard = ctx.guard;
     const long long tiles =
         static_cast<long long>((m + kSkM - 1) / kSkM) * ((n + kSkN - 1) / kSkN);
@@ -1261,7 +1261,7 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
   p.tri = tri;
   p.partial = nullptr;
   p.nchunks = 1;
-  p.timeout_flag = ctx.dev_status;
+  p.timeout_flag = ctx.wait_flag;
   p.guard = ctx.guard;
   const long long tiles =
       static_cast<long long>((m + kBM - 1) / kBM) * ((n + kBN - 1) / kBN);

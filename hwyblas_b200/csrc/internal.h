@@ -50,10 +50,14 @@ struct Context {
   cudaStream_t own_stream = nullptr;
   int device = -1;
   int num_sms = 148;
-  // Device status words: [0] wait-timeout flag written by kernels whose
-  // bounded waits gave up; [1] LAPACK INFO of the running driver; the rest
-  // are grid-barrier counters and scratch ints.
+  // Device status words: [1] LAPACK INFO of the running driver; the rest are
+  // grid-barrier counters and scratch ints.
   int* dev_status = nullptr;
+  // Host words that kernels can write: [0] the wait-timeout flag, set by kernels
+  // whose bounded waits gave up, so that a call without a timeout has nothing
+  // to copy back for it; [1] where INFO is copied to.
+  int* host_status = nullptr;
+  int* wait_flag = nullptr;  // host_status[0] as the device sees it
   // If non-null, kernels return at once while *guard != 0 (used by drivers
   // that must stop after a failure, e.g. Cholesky's non-positive minor).
   const int* guard = nullptr;

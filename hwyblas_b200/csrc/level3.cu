@@ -580,7 +580,7 @@ bool TrsmCoop(bool left, View<T> tri, bool lower, bool unit, int r, int other, T
   a.b = b;
   a.ldb = ldb;
   a.barrier = bar;
-  a.timeout_flag = ctx.dev_status;
+  a.timeout_flag = ctx.wait_flag;
   a.guard = ctx.guard;
   void* args[] = {&a};
   if (cudaLaunchCooperativeKernel(reinterpret_cast<void*>(TrsmCoopKernel<T>), grid,
@@ -734,7 +734,7 @@ bool TrsmCols(View<double> tri, bool lower, bool unit, int r, int other, double*
   a.b = b;
   a.ldb = ldb;
   a.barrier = nullptr;
-  a.timeout_flag = ctx.dev_status;
+  a.timeout_flag = ctx.wait_flag;
   a.guard = ctx.guard;
   TrsmColsKernel<<<(other + kTsCols - 1) / kTsCols, kTcThreads, 0, ctx.stream>>>(a);
   CountLaunch();

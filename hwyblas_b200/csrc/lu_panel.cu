@@ -603,7 +603,7 @@ bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info,
   args.info = info;
   args.info_base = info_base;
   args.moves = moves;
-  args.timeout_flag = ctx.dev_status;
+  args.timeout_flag = ctx.wait_flag;
   cudaEvent_t t0 = KernelTimerStart(kFamilyLuLeaf, ctx.stream);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);

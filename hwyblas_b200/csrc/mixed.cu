@@ -926,7 +926,7 @@ bool ChainTrsv(bool lower, int n, int nrhs, const double* w, long long ldw,
   const int per_launch = std::max(1, std::min(chains, capacity / pmin));
   int nn = n;
   long long lw = ldw, lx = ldx;
-  int* tflag = ctx.dev_status;
+  int* tflag = ctx.wait_flag;
   unsigned int epoch = 1;
   const void* fn = lower ? reinterpret_cast<const void*>(ChainTrsvKernel<true>)
                          : reinterpret_cast<const void*>(ChainTrsvKernel<false>);
@@ -967,7 +967,7 @@ void BlockTrsv(bool lower, int n, int nrhs, const double* w, long long ldw,
   }
   int nn = n;
   long long lw = ldw, lx = ldx;
-  int* flag = ctx.dev_status;
+  int* flag = ctx.wait_flag;
   const void* fn = lower ? reinterpret_cast<const void*>(BlockTrsvKernel<true>)
                          : reinterpret_cast<const void*>(BlockTrsvKernel<false>);
   for (int q0 = 0; q0 < nrhs; q0 += kTrsvRhs) {

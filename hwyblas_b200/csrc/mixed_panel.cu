@@ -790,7 +790,7 @@ void TournamentLeaf(int m, int w, double* a, int lda, int* ipiv, int* info, int 
     epoch = 0;
   }
   p.epoch = ++epoch;
-  p.timeout_flag = ctx.dev_status;
+  p.timeout_flag = ctx.wait_flag;
   void* args[] = {&p};
   cudaEvent_t t0 = KernelTimerStart(kFamilyLuLeaf, ctx.stream);
   Failed(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(TournamentLeafKernel), c0,

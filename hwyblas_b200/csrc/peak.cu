@@ -113,11 +113,11 @@ double I8PeakTops() {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  kernel<<<ctx.num_sms, 64, kProbeSmem, ctx.stream>>>(64, ctx.dev_status);
+  kernel<<<ctx.num_sms, 64, kProbeSmem, ctx.stream>>>(64, ctx.wait_flag);
   float best = 1e30f;
   for (int r = 0; r < 3; ++r) {
     cudaEventRecord(e0, ctx.stream);
-    kernel<<<ctx.num_sms, 64, kProbeSmem, ctx.stream>>>(iters, ctx.dev_status);
+    kernel<<<ctx.num_sms, 64, kProbeSmem, ctx.stream>>>(iters, ctx.wait_flag);
     cudaEventRecord(e1, ctx.stream);
     cudaEventSynchronize(e1);
     float ms = 0.f;
