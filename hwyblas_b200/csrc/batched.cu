@@ -574,6 +574,7 @@ struct LuShared {
   T wv[32];
   int wi[32];
   int piv;
+  T pivot;
 };
 
 // LU leaf (min(m, n) <= 16) on an m x n block: partial pivoting with the
@@ -610,14 +611,18 @@ __device__ void CtaLeaf(int m, int n, Mat<T> a, int* ipiv, int* info, int col0, 
       }
       if (lane == 0) {
         if (isnan(fabs(a(j, j))) || bi == 0x7fffffff) bi = j;
+        // The pivot itself goes through shared memory too: the rows are
+        // interchanged below while other warps may be only here.
+        const T v = a(bi, j);
         sh.piv = bi;
+        sh.pivot = v;
         ipiv[j] = bi + 1;
-        if (a(bi, j) == T(0) && *info == 0) *info = col0 + j + 1;
+        if (v == T(0) && *info == 0) *info = col0 + j + 1;
       }
     }
     __syncthreads();
     const int piv = sh.piv;
-    const T pivot = a(piv, j);
+    const T pivot = sh.pivot;
     if (pivot != T(0) && piv != j) {
       for (int c = threadIdx.x; c < w; c += blockDim.x) {
         const T t = a(j, c);
