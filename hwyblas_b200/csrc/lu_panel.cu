@@ -37,18 +37,19 @@ constexpr int kPanelLd = kPanelW + 16 / static_cast<int>(sizeof(T));
 constexpr int kPanelThreads = 512;  // rows of a CTA at most
 constexpr int kPanelLeast = 256;   // threads at least: the solves share all warps
 constexpr int kPanelCtas = 16;
-// Polls of a wait for the other CTAs' candidates: each lasts up to the
-// hardware's suspend time, far above any real wait in total.
-constexpr uint32_t kPanelPolls = 1u << 20;
+// Polls of a wait for the other CTAs' candidates (some 30 ns each): far above
+// any real wait.
+constexpr uint32_t kPanelPolls = 1u << 22;
 
-// A CTA's candidate of one column: the row from that column on, the reciprocal of
-// its pivot, its key, position and place in the panel.
+// A CTA's candidate of one column: its key, its position after and its place
+// before the interchanges, and the row from that column on. The reciprocal of
+// its pivot follows in a message of its own, computed while the first is on its
+// way.
 template <typename T>
 struct __align__(16) PanelSlot {
-  T row[kPanelLeaf];
   unsigned long long key;
   int pos, place;
-  T rinv;
+  T row[kPanelLeaf];
 };
 
 template <typename T>
@@ -66,27 +67,31 @@ struct PanelArgs {
 
 // Order of the pivot search: larger |x|, NaN below everything (0).
 __device__ __forceinline__ unsigned long long PivotKey(double x) {
-  const double v = fabs(x);
-  return isnan(v) ? 0ull : static_cast<unsigned long long>(__double_as_longlong(v)) + 1;
+  const unsigned long long v = __double_as_longlong(x) & 0x7fffffffffffffffull;
+  return v > 0x7ff0000000000000ull ? 0ull : v + 1;
 }
 __device__ __forceinline__ unsigned long long PivotKey(float x) {
-  const float v = fabsf(x);
-  return isnan(v) ? 0ull : static_cast<unsigned long long>(__float_as_uint(v)) + 1;
+  const unsigned v = __float_as_uint(x) & 0x7fffffffu;
+  return v > 0x7f800000u ? 0ull : static_cast<unsigned long long>(v) + 1;
 }
 
-// The warp's largest key and the smallest position holding it.
+// The lane with the warp's largest key, the one with the smallest position if
+// several hold it. The keys' high words nearly always decide.
 template <typename T>
-__device__ __forceinline__ void WarpBest(unsigned long long& key, int& pos) {
+__device__ __forceinline__ int WarpBest(unsigned long long key, int pos) {
   const unsigned lo = static_cast<unsigned>(key), hi = static_cast<unsigned>(key >> 32);
-  unsigned mhi = 0;
-  bool top = true;
-  if constexpr (sizeof(T) == 8) {
-    mhi = __reduce_max_sync(0xffffffffu, hi);
-    top = hi == mhi;
+  const unsigned word = sizeof(T) == 8 ? hi : lo;
+  const unsigned largest = __reduce_max_sync(0xffffffffu, word);
+  unsigned top = __ballot_sync(0xffffffffu, word == largest);
+  if (top & (top - 1)) {
+    const bool in = (top >> (threadIdx.x % 32)) & 1;
+    const unsigned second = sizeof(T) == 8 && in ? lo : 0u;
+    const unsigned most = __reduce_max_sync(0xffffffffu, second);  // by every lane
+    const bool in2 = in && second == most;
+    const int first = __reduce_min_sync(0xffffffffu, in2 ? pos : 0x7fffffff);
+    top = __ballot_sync(0xffffffffu, in2 && pos == first);
   }
-  const unsigned mlo = __reduce_max_sync(0xffffffffu, top ? lo : 0u);
-  pos = __reduce_min_sync(0xffffffffu, top && lo == mlo ? pos : 0x7fffffff);
-  key = (static_cast<unsigned long long>(mhi) << 32) | mlo;
+  return __ffs(top) - 1;
 }
 
 __device__ __forceinline__ uint32_t MapRank(uint32_t addr, int rank) {
@@ -102,6 +107,21 @@ __device__ __forceinline__ void StAsync16(uint32_t dst, ulonglong2 v, uint32_t b
       : "r"(dst), "l"(v.x), "l"(v.y), "r"(bar)
       : "memory");
 }
+// One value to another CTA's shared memory, counted on its mbarrier.
+__device__ __forceinline__ void StAsync(uint32_t dst, double v, uint32_t bar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+      :
+      : "r"(dst), "l"(__double_as_longlong(v)), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void StAsync(uint32_t dst, float v, uint32_t bar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+      :
+      : "r"(dst), "r"(__float_as_int(v)), "r"(bar)
+      : "memory");
+}
 __device__ __forceinline__ double LoadRemote(uint32_t addr, double) {
   double v;
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
@@ -112,6 +132,17 @@ __device__ __forceinline__ float LoadRemote(uint32_t addr, float) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
+__device__ __forceinline__ bool MbarTest(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(SmemAddr(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ void ClusterBarrier() {
   asm volatile(
       "barrier.cluster.arrive.release.aligned;\n\t"
@@ -119,20 +150,28 @@ __device__ __forceinline__ void ClusterBarrier() {
           : "memory");
 }
 
-// Solves with the unit lower triangle, two columns a warp, a lane one row: the
+// One element global -> shared, asynchronously.
+template <typename T>
+__device__ __forceinline__ void CopyElement(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(SmemAddr(dst)), "l"(src),
+               "n"(sizeof(T))
+               : "memory");
+}
+
+// Solves with the unit lower triangle, N columns a warp, a lane one row: the
 // solved values go round by shuffles, so that r rows are r - 1 steps and each
 // element's chain runs over q ascending (src/trsm-inl.h:107-174). lrow: the
 // lane's row of the triangle.
-template <typename T>
-__device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[2]) {
+template <typename T, int N>
+__device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[N]) {
   const int lane = threadIdx.x % 32;
 #pragma unroll 4
   for (int q = 0; q + 1 < r; ++q) {
     const T l = lrow[q];
-    const T y0 = __shfl_sync(0xffffffffu, y[0], q), y1 = __shfl_sync(0xffffffffu, y[1], q);
-    if (lane > q) {
-      y[0] = fma(-y0, l, y[0]);
-      y[1] = fma(-y1, l, y[1]);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const T yq = __shfl_sync(0xffffffffu, y[i], q);
+      if (lane > q) y[i] = fma(-yq, l, y[i]);
     }
   }
 }
@@ -141,15 +180,17 @@ __device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[2]) {
 // lower in their columns [0, n1), U in columns [n1, n1 + n2)).
 template <typename T>
 __device__ __forceinline__ void PanelSolve(T* rows, int n1, int n2) {
+  constexpr int N = 4;
   const int lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
   T* row = rows + min(lane, n1 - 1) * kPanelLd<T>;
-  for (int c = 2 * (threadIdx.x / 32); c < n2; c += 2 * nwarps) {
-    T y[2] = {row[n1 + c], row[n1 + min(c + 1, n2 - 1)]};
-    LaneSolve<T>(row, n1, y);
-    if (lane < n1) {
-      row[n1 + c] = y[0];
-      if (c + 1 < n2) row[n1 + c + 1] = y[1];
-    }
+  for (int c = N * (threadIdx.x / 32); c < n2; c += N * nwarps) {
+    T y[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) y[i] = row[n1 + min(c + i, n2 - 1)];
+    LaneSolve<T, N>(row, n1, y);
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (lane < n1 && c + i < n2) row[n1 + c + i] = y[i];
   }
 }
 
@@ -177,6 +218,7 @@ __device__ __forceinline__ void PanelUpdate(const T* l, T* x, int R, const T* u,
   T acc[2][kPanelLeaf];
 #pragma unroll
   for (int c = 0; c < kPanelLeaf; ++c) acc[0][c] = acc[1][c] = T(0);
+#pragma unroll 2
   for (int q = 0; q < n1; ++q) {
     const T la = l[q * R + ra], lb = l[q * R + rb];
 #pragma unroll
@@ -203,14 +245,16 @@ template <typename T>
 __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p) {
   extern __shared__ __align__(16) unsigned char panel_smem[];
   const int P = gridDim.x, cta = blockIdx.x, R = p.R, w = p.w;
-  PanelSlot<T>* slots = reinterpret_cast<PanelSlot<T>*>(panel_smem);  // [2][kPanelCtas]
-  T* prow = reinterpret_cast<T*>(slots + 2 * kPanelCtas);            // [w][kPanelLd] pivot rows
+  // [2][kPanelCtas] from the CTAs, then this CTA's own.
+  PanelSlot<T>* slots = reinterpret_cast<PanelSlot<T>*>(panel_smem);
+  PanelSlot<T>* own = slots + 2 * kPanelCtas;
+  T* prow = reinterpret_cast<T*>(own + 1);                           // [w][kPanelLd] pivot rows
   T* S = prow + w * kPanelLd<T>;                                     // [w][R] this CTA's rows
-  __shared__ PanelSlot<T> s_mine;
+  __shared__ T s_rinv[2][kPanelCtas];
   __shared__ unsigned long long s_wkey[2][kPanelThreads / 32];
   __shared__ int s_wpos[2][kPanelThreads / 32];
   __shared__ int s_place[kPanelW], s_pos[kPanelThreads], s_op[7][4];
-  __shared__ __align__(8) uint64_t s_bar[2];
+  __shared__ __align__(8) uint64_t s_bar[2], s_rbar[2];
   __shared__ int s_ops;
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, nwarps = blockDim.x / 32;
   const int place = cta * R + tid;
@@ -220,6 +264,8 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
   if (tid == 0) {
     MbarInit(&s_bar[0], 1);
     MbarInit(&s_bar[1], 1);
+    MbarInit(&s_rbar[0], 1);
+    MbarInit(&s_rbar[1], 1);
     FenceBarrierInit();
     // The recursion's steps: leaves (columns c0.., n) and, between the halves
     // of a block (n1 and n2 columns), its solve and update.
@@ -249,17 +295,11 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
   }
   if (valid) {
     const T* src = p.a + place;
-#pragma unroll 1
-    for (int c0 = 0; c0 < w; c0 += 16) {
-      T v[16];
-#pragma unroll
-      for (int c = 0; c < 16; ++c)
-        if (c0 + c < w) v[c] = src[(c0 + c) * p.lda];
-#pragma unroll
-      for (int c = 0; c < 16; ++c)
-        if (c0 + c < w) S[(c0 + c) * R + tid] = v[c];
-    }
+#pragma unroll 4
+    for (int c = 0; c < w; ++c) CopyElement(S + c * R + tid, src + c * p.lda);
   }
+  CpAsyncCommit();
+  CpAsyncWait<0>();
   // Every CTA's mbarriers are ready before any candidate is sent.
   if (P > 1) ClusterBarrier();
   else __syncthreads();
@@ -277,42 +317,35 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
 #pragma unroll 1
       for (int j = 0; j < n1; ++j) {
         const int jc = c0 + j, par = jc & 1;
+        if (P > 1 && tid == 0) {
+          MbarArriveExpectTx(&s_bar[par], P * static_cast<uint32_t>(sizeof(PanelSlot<T>)));
+          MbarArriveExpectTx(&s_rbar[par], P * static_cast<uint32_t>(sizeof(T)));
+        }
         // The warp's candidate among the rows not yet taken (position >= jc). A
         // NaN at position jc wins, as the reference's search starts from it.
-        const bool in = valid && pos >= jc;
-        unsigned long long key = in ? PivotKey(x[0]) : 0ull;
-        if (in && pos == jc && key == 0) key = sizeof(T) == 8 ? ~0ull : 0xffffffffull;
-        int best = pos;
-        WarpBest<T>(key, best);
-        if (lane == 0) {
+        unsigned long long key = valid && pos >= jc ? PivotKey(x[0]) : 0ull;
+        if (valid && pos == jc && key == 0) key = sizeof(T) == 8 ? ~0ull : 0xffffffffull;
+        const int wbest = WarpBest<T>(key, pos);
+        if (lane == wbest) {
           s_wkey[par][warp] = key;
-          s_wpos[par][warp] = best;
+          s_wpos[par][warp] = pos;
         }
-        const T rinv = T(1) / x[0];
-        if (__syncthreads_or(timed_out)) {
-          alive = false;
-          break;
-        }
+        __syncthreads();
         // The block's, found by every warp; the warp that holds the row sends it.
-        key = lane < nwarps ? s_wkey[par][lane] : 0ull;
-        best = lane < nwarps ? s_wpos[par][lane] : 0x7fffffff;
-        WarpBest<T>(key, best);
-        const bool mine = in && key != 0 && pos == best;
-        if (__any_sync(0xffffffffu, mine) || (key == 0 && warp == 0)) {
-          if (mine) {
+        const int cbest = WarpBest<T>(lane < nwarps ? s_wkey[par][lane] : 0ull,
+                                      lane < nwarps ? s_wpos[par][lane] : 0x7fffffff);
+        if (warp == cbest) {
+          if (lane == wbest) {
+            own->key = key;
+            own->pos = pos;
+            own->place = place;
 #pragma unroll
-            for (int k = 0; k < kPanelLeaf; ++k) s_mine.row[k] = x[k];
-            s_mine.rinv = rinv;
-            s_mine.place = place;
-          }
-          if (mine || (key == 0 && lane == 0)) {
-            s_mine.key = key;
-            s_mine.pos = best;
+            for (int k = 0; k < kPanelLeaf; ++k) own->row[k] = x[k];
           }
           __syncwarp();
           if (P > 1) {
             constexpr int kPieces = sizeof(PanelSlot<T>) / 16;
-            const ulonglong2* src = reinterpret_cast<const ulonglong2*>(&s_mine);
+            const ulonglong2* src = reinterpret_cast<const ulonglong2*>(own);
             const uint32_t dst = SmemAddr(&slots[par * kPanelCtas + cta]);
             const uint32_t bar = SmemAddr(&s_bar[par]);
             for (int i = lane; i < P * kPieces; i += 32) {
@@ -320,33 +353,37 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
               StAsync16(MapRank(dst + 16 * e, to), src[e], MapRank(bar, to));
             }
           }
+          const T rinv = T(1) / own->row[0];
+          if (P > 1) {
+            if (lane < P)
+              StAsync(MapRank(SmemAddr(&s_rinv[par][cta]), lane), rinv,
+                      MapRank(SmemAddr(&s_rbar[par]), lane));
+          } else if (lane == 0) {
+            s_rinv[par][0] = rinv;
+          }
         }
-        const PanelSlot<T>* win = &s_mine;
+        int at = 2 * kPanelCtas, from = 0;  // the winner's slot
         if (P > 1) {
-          if (tid == 0)
-            MbarArriveExpectTx(&s_bar[par], P * static_cast<uint32_t>(sizeof(PanelSlot<T>)));
-          uint32_t polls = 0;
-          while (!MbarTryWait(&s_bar[par], (jc >> 1) & 1)) {
+          // After a wait that gave up the columns run on without waiting, to the
+          // leaf's end, where the block leaves together.
+          for (uint32_t polls = 0;
+               !timed_out && !MbarTest(&s_bar[par], (jc >> 1) & 1);) {
             if (++polls >= kPanelPolls) {
               atomicExch(p.timeout_flag, 1);
-              timed_out = true;  // every thread learns of it at the next block barrier
-              break;
+              timed_out = true;
             }
           }
-          key = lane < P ? slots[par * kPanelCtas + lane].key : 0ull;
-          best = lane < P ? slots[par * kPanelCtas + lane].pos : 0x7fffffff;
-          const unsigned long long own_key = key;
-          const int own_pos = best;
-          WarpBest<T>(key, best);
-          const unsigned hit = __ballot_sync(0xffffffffu, own_key == key && own_pos == best);
-          win = &slots[par * kPanelCtas + ((__ffs(hit) - 1) & (kPanelCtas - 1))];
+          const PanelSlot<T>* slot = slots + par * kPanelCtas + lane;
+          from = WarpBest<T>(lane < P ? slot->key : 0ull, lane < P ? slot->pos : 0x7fffffff);
+          at = par * kPanelCtas + (from & (kPanelCtas - 1));
         } else {
           __syncthreads();
         }
+        const PanelSlot<T>* win = slots + at;
         const int piv = win->pos;
         const T pivot = win->row[0];
         if (tid < n1 - j) prow[jc * kPanelLd<T> + jc + tid] = win->row[tid];
-        if (tid == 0) {
+        if (tid == 32) {
           s_place[jc] = win->place;
           if (cta == 0) {
             p.ipiv[jc] = piv + 1 + p.ipiv_add;
@@ -356,17 +393,26 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
         // A zero pivot is at position jc already.
         if (pos == piv) pos = jc;
         else if (pos == jc) pos = piv;
+        for (uint32_t polls = 0; P > 1 && !timed_out && !MbarTest(&s_rbar[par], (jc >> 1) & 1);) {
+          if (++polls >= kPanelPolls) {
+            atomicExch(p.timeout_flag, 1);
+            timed_out = true;
+          }
+        }
         if (valid && pos > jc) {
           // The column below the pivot times its reciprocal (divided if the
           // pivot is below the safe minimum, kept if it is zero), then the
           // rank-1 update of the leaf's later columns, which move up by one.
-          T l = x[0];
-          if (pivot != T(0)) l = !(fabs(pivot) >= Sfmin<T>()) ? l / pivot : l * win->rinv;
+          T l = x[0] * s_rinv[par][from & (kPanelCtas - 1)];
+          if (!(fabs(pivot) >= Sfmin<T>())) l = pivot != T(0) ? x[0] / pivot : x[0];
           S[jc * R + tid] = l;
           const int len = p.m - jc - 1;
           if (len >= p.lanes) {
 #pragma unroll
-            for (int k = 1; k < kPanelLeaf; ++k) x[k - 1] = fma(l, -win->row[k], x[k]);
+            for (int k = 1; k < kPanelLeaf; ++k) {
+              if (k == 9 && n1 - j <= 9) break;  // no such columns
+              x[k - 1] = fma(l, -win->row[k], x[k]);
+            }
           } else {
 #pragma unroll
             for (int k = 1; k < kPanelLeaf; ++k)
@@ -381,13 +427,16 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
         // rows change no more.
         if (__syncthreads_or(timed_out)) alive = false;
         if (P > 1) ClusterBarrier();
-        for (int i = tid; alive && i < n1 * w; i += blockDim.x) {
-          const int s = i / w, col = i - s * w;
-          if (col >= c0 + s && col < c0 + n1) continue;
-          const int from = s_place[c0 + s], owner = from / R;
-          const T* at = S + col * R + (from - owner * R);
-          prow[(c0 + s) * kPanelLd<T> + col] =
-              P > 1 ? LoadRemote(MapRank(SmemAddr(at), owner), T(0)) : *at;
+        for (int r = warp; alive && r < n1; r += nwarps) {
+          const int from = s_place[c0 + r], owner = from / R;
+          const T* row = S + (from - owner * R);
+#pragma unroll
+          for (int d = 0; d < kPanelW / 32; ++d) {
+            const int col = lane + 32 * d;
+            if (col >= w || (col >= c0 + r && col < c0 + n1)) continue;
+            prow[(c0 + r) * kPanelLd<T> + col] =
+                P > 1 ? LoadRemote(MapRank(SmemAddr(row + col * R), owner), T(0)) : row[col * R];
+          }
         }
         __syncthreads();
       }
@@ -415,11 +464,14 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
     }
   }
   if (!__syncthreads_or(timed_out) && alive) {
-    for (int c = cta; c < w; c += P)
-      for (int r = tid; r < w; r += blockDim.x) p.a[r + c * p.lda] = prow[r * kPanelLd<T> + c];
+#pragma unroll 4
+    for (int i = tid; i < (w - cta + P - 1) / P * kPanelW; i += blockDim.x) {
+      const int r = i % kPanelW, c = cta + i / kPanelW * P;
+      if (r < w) p.a[r + c * p.lda] = prow[r * kPanelLd<T> + c];
+    }
     if (valid && pos >= w) {
       T* dst = p.a + pos;
-#pragma unroll 4
+#pragma unroll 8
       for (int c = 0; c < w; ++c) dst[c * p.lda] = S[c * R + tid];
     }
     if (valid && pos != place && p.moves != nullptr) {
@@ -434,7 +486,7 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
 
 template <typename T>
 size_t PanelSmem(int w, int R) {
-  return 2 * kPanelCtas * sizeof(PanelSlot<T>) +
+  return (2 * kPanelCtas + 1) * sizeof(PanelSlot<T>) +
          sizeof(T) * static_cast<size_t>(w) * (kPanelLd<T> + R);
 }
 
@@ -528,7 +580,7 @@ __global__ void __launch_bounds__(kSwapThreads) PanelSwapTrsmKernel(SwapArgs<T> 
   static_assert(kSwapCols == 2 * (kSwapThreads / 32), "two columns a warp");
   const T* l1 = s_l + min(lane, jb - 1) * kLd;
   T y[2] = {s_b[c][lane], s_b[c + 1][lane]};
-  LaneSolve<T>(l1, r1, y);
+  LaneSolve<T, 2>(l1, r1, y);
   T z[2] = {T(0), T(0)};
   if (r2 > 0) {
     const T* l2 = s_l + min(32 + lane, jb - 1) * kLd;
@@ -541,7 +593,7 @@ __global__ void __launch_bounds__(kSwapThreads) PanelSwapTrsmKernel(SwapArgs<T> 
     }
     z[0] = T(-1) * acc[0] + s_b[c][32 + lane];
     z[1] = T(-1) * acc[1] + s_b[c + 1][32 + lane];
-    LaneSolve<T>(l2 + 32, r2, z);
+    LaneSolve<T, 2>(l2 + 32, r2, z);
   }
 #pragma unroll
   for (int d = 0; d < 2; ++d) {
