@@ -204,25 +204,19 @@ __device__ __forceinline__ void StoreX(T* p, T v) {
   else *p = v;
 }
 
-// N rows of X solved by a warp, lane s holding the element of step s: at step q
-// lane q's element is final, goes round by shuffles, and every later lane takes
-// its term, so each element's chain is over q ascending, as above, but the
-// chains of a row run side by side. The loop is rolled: unrolled for one
-// thread a row, a launch fetched a thousand instructions to run each once
-// (10 us; 3 us so), and lanes along a column-major X read it coalesced.
-// xr[i]: row i's first element; rows with i >= n are not touched.
-template <typename T, bool kCg, int N>
-__device__ __forceinline__ void WarpSolve(const T (*st)[33], const T* sinv, int lower, int unit,
-                                          int r, T* const (&xr)[N], int n, long long xs_col) {
+// N rows of X solved by a warp, lane s holding the element of step s (y): at
+// step q lane q's element is final, goes round by shuffles, and every later
+// lane takes its term, so each element's chain is over q ascending, as above,
+// but the chains of a row run side by side. st: the triangle, row stride ld. The
+// loop is rolled: unrolled for one thread a row, a launch fetched a thousand
+// instructions to run each once (32 x 32 base: 10 us; 4 to 6 us so), and lanes
+// along a column-major X read it coalesced.
+template <typename T, int N>
+__device__ __forceinline__ void LaneSolve(const T* st, int ld, T inv, int unit, int r, T (&y)[N]) {
   const int lane = threadIdx.x % 32;
-  const long long at = (lower ? r - 1 - lane : lane) * xs_col;
-  T y[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) y[i] = i < n && lane < r ? LoadX<T, kCg>(xr[i] + at) : T(0);
-  const T inv = sinv[lane];
 #pragma unroll 2
   for (int q = 0; q < r; ++q) {
-    const T l = st[q][lane];
+    const T l = st[q * ld + lane];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const T yq = __shfl_sync(0xffffffffu, unit ? y[i] : y[i] * inv, q);
@@ -230,45 +224,100 @@ __device__ __forceinline__ void WarpSolve(const T (*st)[33], const T* sinv, int 
       else if (lane > q) y[i] = fma(-yq, l, y[i]);
     }
   }
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-    if (i < n && lane < r) StoreX<T, kCg>(xr[i] + at, y[i]);
 }
 
-// A base solve of many rows: a CTA takes kBaseRows of them, two a warp. Rows
-// that are contiguous in memory across each other (right side) go through
-// shared memory, so that both sides read and write whole sectors.
-constexpr int kBaseThreads = 256, kBaseRows = 2 * kBaseThreads / 32;
+// One row of X in global memory against a 32 x 32 triangle (LoadBaseTriangle).
+template <typename T, bool kCg>
+__device__ __forceinline__ void WarpSolve(const T (*st)[33], const T* sinv, int lower, int unit,
+                                          int r, T* xr, long long xs_col) {
+  const int lane = threadIdx.x % 32;
+  T* at = xr + (lower ? r - 1 - lane : lane) * xs_col;
+  T y[1] = {lane < r ? LoadX<T, kCg>(at) : T(0)};
+  LaneSolve<T, 1>(&st[0][0], 33, sinv[lane], unit, r, y);
+  if (lane < r) StoreX<T, kCg>(at, y[0]);
+}
+
+// The recursion's node of at most 64 columns (src/trsm.cc:87-135: a base solve,
+// the product, a base solve) for many rows in one launch: a CTA takes kBaseRows
+// of them, two a warp. Rows that are contiguous in memory across each other
+// (right side) go through shared memory, so that both sides read and write
+// whole sectors.
+constexpr int kBaseThreads = 256, kBaseRows = 2 * kBaseThreads / 32, kBaseW = 64;
 template <typename T>
 __global__ void __launch_bounds__(kBaseThreads)
     TrsmBaseKernel(View<T> tri, int lower, int unit, int r, int rows, T* x,
                    long long xs_row, long long xs_col, const int* guard) {
   if (guard != nullptr && *guard != 0) return;
-  __shared__ T st[32][33];  // st[s][u] = T(col(s), col(u)) in solve order
-  __shared__ T sinv[32];
-  __shared__ T xt[kBaseRows][33];
+  constexpr int ld = kBaseW + 1;
+  __shared__ T st[kBaseW * ld];  // st[s][u] = T(col(s), col(u)) in solve order, s < u
+  __shared__ T sinv[kBaseW];
+  __shared__ T xt[kBaseRows][kBaseW + 1];
+  const int tid = threadIdx.x, lane = tid % 32, i0 = tid / 32 * 2;
   const int row0 = blockIdx.x * kBaseRows, n = min(kBaseRows, rows - row0);
   const bool across = xs_row == 1;
   x += row0 * xs_row;
   if (across) {
-    for (int idx = threadIdx.x; idx < kBaseRows * r; idx += kBaseThreads) {
-      const int i = idx % kBaseRows, s = idx / kBaseRows;
-      if (i < n) xt[i][s] = x[i + s * xs_col];
+    for (int idx = tid; idx < kBaseRows * r; idx += kBaseThreads) {
+      const int i = idx % kBaseRows, c = idx / kBaseRows;
+      if (i < n) xt[i][c] = x[i + c * xs_col];
     }
   }
-  LoadBaseTriangle(tri, lower, unit, r, st, sinv);
-  const int i0 = threadIdx.x / 32 * 2;
-  if (across) {
-    T* const xr[2] = {xt[i0], xt[i0 + 1]};
-    WarpSolve<T, false>(st, sinv, lower, unit, r, xr, n - i0, 1);
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < kBaseRows * r; idx += kBaseThreads) {
-      const int i = idx % kBaseRows, s = idx / kBaseRows;
-      if (i < n) x[i + s * xs_col] = xt[i][s];
+  const int w = r > 32 ? 64 : 32;
+  const bool rows_fast = tri.rs == 1;
+  for (int idx = tid; idx < w * w; idx += kBaseThreads) {
+    const int s = rows_fast ? idx % w : idx / w, u = rows_fast ? idx / w : idx % w;
+    T v = T(0);
+    if (s < r && u < r && (s < u || (s == u && !unit))) {
+      const int q = lower ? r - 1 - s : s, j = lower ? r - 1 - u : u;
+      v = tri.data[q * tri.rs + j * tri.cs];
     }
-  } else {
-    T* const xr[2] = {x + i0 * xs_row, x + (i0 + 1) * xs_row};
-    WarpSolve<T, false>(st, sinv, lower, unit, r, xr, n - i0, xs_col);
+    st[s * ld + u] = v;
+    if (s == u) sinv[s] = s < r && !unit ? T(1) / v : T(1);
+  }
+  __syncthreads();
+  // The half solved first: the leading 32 columns (upper) or the others (lower),
+  // which is 32 columns' solve order from its start.
+  const int f = r <= 32 ? r : (lower ? r - 32 : 32), g = r - f;
+  // Column of step s, in elements from a row's first.
+  const auto col = [&](int s) { return lower ? r - 1 - s : s; };
+  T y[2], z[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const T* xr = across ? xt[i0 + i] : x + (i0 + i) * xs_row;
+    const long long xc = across ? 1 : xs_col;
+    const bool in = i0 + i < n;
+    y[i] = in && lane < f ? xr[col(lane) * xc] : T(0);
+    z[i] = in && lane < g ? xr[col(f + lane) * xc] : T(0);
+  }
+  LaneSolve<T, 2>(st, ld, sinv[lane], unit, f, y);
+  if (g > 0) {
+    // z -= y T: one chain an element, over the columns in memory order.
+    T acc[2] = {T(0), T(0)};
+#pragma unroll 4
+    for (int e = 0; e < f; ++e) {
+      const int q = lower ? f - 1 - e : e;
+      const T t = st[q * ld + f + lane];
+      acc[0] = fma(__shfl_sync(0xffffffffu, y[0], q), t, acc[0]);
+      acc[1] = fma(__shfl_sync(0xffffffffu, y[1], q), t, acc[1]);
+    }
+    z[0] = T(-1) * acc[0] + z[0];
+    z[1] = T(-1) * acc[1] + z[1];
+    LaneSolve<T, 2>(st + f * ld + f, ld, sinv[min(f + lane, kBaseW - 1)], unit, g, z);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    T* xr = across ? xt[i0 + i] : x + (i0 + i) * xs_row;
+    const long long xc = across ? 1 : xs_col;
+    if (i0 + i >= n) continue;
+    if (lane < f) xr[col(lane) * xc] = y[i];
+    if (lane < g) xr[col(f + lane) * xc] = z[i];
+  }
+  if (across) {
+    __syncthreads();
+    for (int idx = tid; idx < kBaseRows * r; idx += kBaseThreads) {
+      const int i = idx % kBaseRows, c = idx / kBaseRows;
+      if (i < n) x[i + c * xs_col] = xt[i][c];
+    }
   }
 }
 
@@ -492,8 +541,7 @@ __global__ void __launch_bounds__(kTcThreads) TrsmCoopKernel(TrsmCoopArgs<T> p) 
       // Rows go to the CTAs in turn, then to their warps.
       for (long long row = blockIdx.x + static_cast<long long>(gridDim.x) * (threadIdx.x / 32);
            row < p.other; row += static_cast<long long>(gridDim.x) * (blockDim.x / 32)) {
-        T* const xr[1] = {xb + row * xs_row};
-        WarpSolve<T, true>(st, sinv, lo, p.unit, rr, xr, 1, xs_col);
+        WarpSolve<T, true>(st, sinv, lo, p.unit, rr, xb + row * xs_row, xs_col);
       }
       --sp;
       if (!GridBarrier(p.barrier, gridDim.x, ++gen, p.timeout_flag)) return;
@@ -693,8 +741,7 @@ __global__ void __launch_bounds__(kTcThreads) TrsmColsKernel(TrsmCoopArgs<double
       const int lo = !p.lower;
       LoadBaseTriangle(t, lo, p.unit, rr, st, sinv);
       for (int j = threadIdx.x / 32; j < w; j += blockDim.x / 32) {
-        double* const xr[1] = {xb + off + j * p.ldb};
-        WarpSolve<double, true>(st, sinv, lo, p.unit, rr, xr, 1, 1);
+        WarpSolve<double, true>(st, sinv, lo, p.unit, rr, xb + off + j * p.ldb, 1);
       }
       --sp;
       __syncthreads();
@@ -759,7 +806,7 @@ void LaunchGemm<float>(int m, int n, int k, float alpha, View<float> a,
 template <typename T>
 void TrsmRec(bool left, View<T> tri, bool lower, bool unit, int r, int other,
              T* b, int ldb) {
-  if (r <= 32) {
+  if (r <= kBaseW) {
     TrsmSolve<T>(left, tri, lower, unit, r, other, b, ldb);
     return;
   }
