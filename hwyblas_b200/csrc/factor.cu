@@ -3,7 +3,7 @@
 //   IAMAX      src/level1.cc:383-402, src/level1-inl.h:343-423
 //   LASWP      src/lapack/getrf.cc:28-81
 //   GetrfLeaf  src/lapack/factor_kernels.cc:79-183
-//   PotrfLeaf  src/lapack/factor_kernels.cc:187-221
+//   Cholesky leaf  src/lapack/factor_kernels.cc:187-221
 // "lanes" is the vector length (in elements) of the reference's SIMD target:
 // AXPY columns shorter than one vector are updated as y + (alpha*x) (two
 // roundings), longer ones as fma(x, alpha, y) (factor_kernels.cc:79-118).
@@ -606,67 +606,131 @@ __global__ void GetrfLeafTrailingKernel(int m, int w, int n, T* a,
 }
 
 // ---------------------------------------------------------------------------
-// Cholesky leaf (n <= 64) in one CTA, the block in shared memory.
+// Cholesky block (n <= 64) in one CTA: the reference's recursion
+// (src/lapack/potrf.cc:48-119: two leaves of at most 32 columns with the
+// triangular solve and the symmetric update between them) on the block in
+// shared memory. An upper block is held transposed: its operations are the
+// lower ones with each product's factors exchanged, except for the length that
+// decides an AXPY's rounding. Bound by the latency of the n dependent square
+// roots and reciprocals; a leaf is one warp, a lane one row, whose remaining
+// columns sit in registers that shift with every step (a rolled loop: its
+// instructions are fetched once). 64 columns: 27 us a leaf, plus solve and update
+// in launches of their own, -> the whole block in one launch.
+constexpr int kCholW = 64, kCholLd = kCholW + 1, kCholLeaf = 32, kCholThreads = 256;
+
+// The leaf at (c0, c0) of s; false after a non-positive (or NaN) diagonal.
 template <typename T>
-__global__ void __launch_bounds__(256)
-    PotrfLeafKernel(int upper, int n, T* a, long long lda, int* info,
-                    int info_base, int lanes, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
-  __shared__ T s[64][65];  // s[i][j] = A(i, j)
-  __shared__ T row[64];
-  __shared__ int stop;
-  for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-    const int i = idx % n, j = idx / n;
-    const bool ref = upper ? (i <= j) : (i >= j);
-    s[i][j] = ref ? a[i + j * lda] : T(0);
-  }
-  if (threadIdx.x == 0) stop = 0;
-  __syncthreads();
+__device__ bool CholLeaf(T* s, T* col, T* sinv, int upper, int c0, int n, int lanes, int* info,
+                         int info_base) {
+  const int lane = threadIdx.x;
+  T* row = s + (c0 + lane) * kCholLd + c0;
+  T x[kCholLeaf];
+#pragma unroll
+  for (int k = 0; k < kCholLeaf; ++k) x[k] = lane < n && k <= lane ? row[k] : T(0);
+#pragma unroll 1
   for (int j = 0; j < n; ++j) {
-    if (threadIdx.x == 0) {
-      const T ajj = s[j][j];
-      if (ajj <= T(0) || isnan(ajj)) {
-        stop = 1;
-        if (*info == 0) *info = info_base + j + 1;
+    const T ajj = __shfl_sync(0xffffffffu, x[0], j);
+    if (ajj <= T(0) || isnan(ajj)) {
+#pragma unroll
+      for (int k = 0; k < kCholLeaf; ++k)
+        if (lane < n && j + k <= lane) row[j + k] = x[k];
+      if (lane == 0 && *info == 0) *info = info_base + c0 + j + 1;
+      return false;
+    }
+    const T r = sqrt(ajj), rinv = T(1) / r;
+    const T l = lane == j ? r : x[0] * rinv;
+    if (lane >= j && lane < n) row[j] = l;
+    if (lane == 0) sinv[c0 + j] = rinv;
+    __syncwarp();
+    col[lane] = l;
+    __syncwarp();
+    // Column j + k from its diagonal on: y += -l(j + k) * l.
+#pragma unroll
+    for (int k = 1; k < kCholLeaf; ++k) {
+      if (k % 8 == 1 && k >= n - j) break;  // no such columns
+      const T u = col[j + k];
+      if ((upper ? lane - j : n - j - k) < lanes) {
+        const T p = -u * l;
+        x[k - 1] = x[k] + p;
       } else {
-        const T r = sqrt(ajj);
-        s[j][j] = r;
-        row[j] = T(1) / r;  // rinv
+        x[k - 1] = fma(l, -u, x[k]);
       }
     }
-    __syncthreads();
-    if (stop) break;
-    const T rinv = row[j];
-    __syncthreads();
-    if (upper) {
-      for (int k = j + 1 + threadIdx.x; k < n; k += blockDim.x) {
-        s[j][k] = s[j][k] * rinv;
-        row[k] = s[j][k];
-      }
-      __syncthreads();
-      // Column k, rows j+1..k: y += (-U(j,k)) * row, length k - j.
-      for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-        const int i = idx % n, k = idx / n;
-        if (k <= j || i <= j || i > k) continue;
-        s[i][k] = Axpy(s[i][k], -s[j][k], row[i], k - j, lanes);
-      }
-    } else {
-      for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) s[i][j] = s[i][j] * rinv;
-      __syncthreads();
-      // Column k, rows k..n-1: y += (-L(k,j)) * L(k:n, j), length n - k.
-      for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-        const int i = idx % n, k = idx / n;
-        if (k <= j || i < k) continue;
-        s[i][k] = Axpy(s[i][k], -s[k][j], s[i][j], n - k, lanes);
-      }
-    }
-    __syncthreads();
+  }
+  return true;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kCholThreads)
+    PotrfBlockKernel(int upper, int n, T* a, long long lda, int* info, int info_base, int lanes,
+                     const int* guard) {
+  if (guard != nullptr && *guard != 0) return;
+  __shared__ T s[kCholW * kCholLd];  // s[i][j], i >= j
+  __shared__ T col[2 * kCholLeaf], sinv[kCholW];
+  __shared__ int alive;
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  for (int idx = tid; idx < n * n; idx += kCholThreads) {
+    const int x = idx % n, y = idx / n;  // x is contiguous in memory
+    const int i = upper ? y : x, j = upper ? x : y;
+    if (i >= j) s[i * kCholLd + j] = a[x + y * lda];
+  }
+  if (tid < 2 * kCholLeaf) col[tid] = T(0);
+  __syncthreads();
+  const int n1 = n <= kCholLeaf ? n : n / 2, n2 = n - n1;
+  if (warp == 0) {
+    const bool ok = CholLeaf(s, col, sinv, upper, 0, n1, lanes, info, info_base);
+    if (lane == 0) alive = ok;
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-    const int i = idx % n, j = idx / n;
-    const bool ref = upper ? (i <= j) : (i >= j);
-    if (ref) a[i + j * lda] = s[i][j];
+  if (n2 > 0 && alive) {
+    // Rows n1.. : X L^T = B, a lane one column, four rows a warp.
+    T y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = warp * 4 + i;
+      y[i] = r < n2 && lane < n1 ? s[(n1 + r) * kCholLd + lane] : T(0);
+    }
+    const T inv = lane < n1 ? sinv[lane] : T(0);
+#pragma unroll 2
+    for (int q = 0; q < n1; ++q) {
+      const T l = s[min(lane, n1 - 1) * kCholLd + q];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const T yq = __shfl_sync(0xffffffffu, y[i] * inv, q);
+        if (lane == q) y[i] = yq;
+        else if (lane > q) y[i] = fma(-yq, l, y[i]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = warp * 4 + i;
+      if (r < n2 && lane < n1) s[(n1 + r) * kCholLd + lane] = y[i];
+    }
+    __syncthreads();
+    // The trailing block's lower part: -sum + c, each sum one chain.
+    T acc[4] = {T(0), T(0), T(0), T(0)};
+    const T* ri = s + (n1 + min(lane, n2 - 1)) * kCholLd;
+#pragma unroll 4
+    for (int q = 0; q < n1; ++q) {
+      const T l = ri[q];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        acc[e] = fma(l, s[(n1 + min(warp + 8 * e, n2 - 1)) * kCholLd + q], acc[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int k = warp + 8 * e;
+      T* c = s + (n1 + lane) * kCholLd + n1 + k;
+      if (lane < n2 && k <= lane) *c = T(-1) * acc[e] + *c;
+    }
+    __syncthreads();
+    if (warp == 0) CholLeaf(s, col, sinv, upper, n1, n2, lanes, info, info_base);
+    __syncthreads();
+  }
+  for (int idx = tid; idx < n * n; idx += kCholThreads) {
+    const int x = idx % n, y = idx / n;
+    const int i = upper ? y : x, j = upper ? x : y;
+    if (i >= j) a[x + y * lda] = s[i * kCholLd + j];
   }
 }
 
@@ -859,15 +923,15 @@ unsigned int SetLeafWaitLimit(unsigned int polls) {
 }
 
 template <typename T>
-void PotrfLeaf(bool upper, int n, T* a, int lda, int* info, int info_base) {
+void PotrfBlock(bool upper, int n, T* a, int lda, int* info, int info_base) {
   const int lanes = sizeof(T) == 8 ? RefLanesDouble() : 2 * RefLanesDouble();
-  PotrfLeafKernel<T><<<1, 256, 0, Ctx().stream>>>(upper ? 1 : 0, n, a, lda, info, info_base,
-                                                  lanes, Ctx().guard);
+  PotrfBlockKernel<T><<<1, kCholThreads, 0, Ctx().stream>>>(upper ? 1 : 0, n, a, lda, info,
+                                                            info_base, lanes, Ctx().guard);
   CountLaunch();
-  LaunchFailed("potrf leaf");
+  LaunchFailed("potrf block");
 }
-template void PotrfLeaf<double>(bool, int, double*, int, int*, int);
-template void PotrfLeaf<float>(bool, int, float*, int, int*, int);
+template void PotrfBlock<double>(bool, int, double*, int, int*, int);
+template void PotrfBlock<float>(bool, int, float*, int, int*, int);
 
 // ---------------------------------------------------------------------------
 // IDAMAX that allocates nothing (hwyblas_idamax_noalloc).

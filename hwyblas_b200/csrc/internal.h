@@ -240,13 +240,19 @@ bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info,
 // panel's unit lower triangle on the latter.
 template <typename T>
 void PanelSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const int* moves);
+// The same for the complex LU (interleaved elements, aligned to their size).
+template <typename R>
+bool ZGetrfPanel(int m, int n, R* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,
+                 int* moves);
+template <typename R>
+void ZPanelSwapTrsm(int j, int jb, int left, int c0, int nc, R* a, int lda, const int* moves);
 // Sets the poll limit of the cooperative leaf's exchange on the current
 // device (0: the default); returns the previous one.
 unsigned int SetLeafWaitLimit(unsigned int polls);
-// PotrfLeaf on device: n <= 64; sets *info to info_base + j + 1 and stops at
-// the first non-positive (or NaN) diagonal, if *info is still 0.
+// Potrf2 of a block of n <= 64 columns on device: sets *info to info_base + j + 1
+// and stops at the first non-positive (or NaN) diagonal, if *info is still 0.
 template <typename T>
-void PotrfLeaf(bool upper, int n, T* a, int lda, int* info, int info_base);
+void PotrfBlock(bool upper, int n, T* a, int lda, int* info, int info_base);
 
 // LAPACK drivers on device data (ipiv, info: device pointers).
 template <typename T>

@@ -5,7 +5,7 @@
 //           src/lapack/factor_kernels.h:27)
 //   Getrf   src/lapack/getrf.cc:216-280 (nb = 64, src/lapack/environment.cc:86-88)
 //   Getrs   src/lapack/getrf.cc:287-339
-//   Potrf2  src/lapack/potrf.cc:48-119 (leaf at n <= 32)
+//   Potrf2  src/lapack/potrf.cc:48-119 (leaf at n <= 32, inside PotrfBlock)
 //   Potrf   src/lapack/potrf.cc:128-199 (nb = 64, environment.cc:110-111)
 //   Potrs   src/lapack/posv.cc:31-76
 // Every step is a kernel launch on the context's stream; pivots and INFO stay
@@ -166,8 +166,8 @@ namespace {
 template <typename T>
 void Potrf2Rec(bool upper, int n, T* a, int lda, int* info, int col0) {
   if (n == 0) return;
-  if (n <= 32) {
-    PotrfLeaf<T>(upper, n, a, lda, info, col0);
+  if (n <= 64) {  // down to the leaves of 32
+    PotrfBlock<T>(upper, n, a, lda, info, col0);
     return;
   }
   const int n1 = n / 2, n2 = n - n1;
