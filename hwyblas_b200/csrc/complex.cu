@@ -27,31 +27,11 @@
 
 #include "device.cuh"
 #include "internal.h"
+#include "complex.cuh"
 #include "ref_order.cuh"
 
 namespace hb {
 namespace {
-
-template <typename R>
-__device__ __forceinline__ R Mul(R x, R y) {
-  if constexpr (sizeof(R) == 8) return __dmul_rn(x, y);
-  else return __fmul_rn(x, y);
-}
-template <typename R>
-__device__ __forceinline__ R Add(R x, R y) {
-  if constexpr (sizeof(R) == 8) return __dadd_rn(x, y);
-  else return __fadd_rn(x, y);
-}
-template <typename R>
-__device__ __forceinline__ R Sub(R x, R y) {
-  if constexpr (sizeof(R) == 8) return __dsub_rn(x, y);
-  else return __fsub_rn(x, y);
-}
-template <typename R>
-__device__ __forceinline__ R Fma(R x, R y, R z) {
-  if constexpr (sizeof(R) == 8) return fma(x, y, z);
-  else return fmaf(x, y, z);
-}
 
 constexpr int kZM = 64, kZN = 64, kZK = 16, kZChunk = 256;
 
@@ -534,92 +514,12 @@ __global__ void ZScaleKernel(int m, int n, R beta_re, R beta_im, R* c, long long
   }
 }
 
-// (a + i b) / (c + i d) as the C++ runtime's complex quotient: for double,
-// Smith's method with its scalings for very large and very small magnitudes
-// and its alternative when the ratio is subnormal; for float, the textbook
-// quotient (a c + b d, b c - a d) / (c^2 + d^2) in double precision, rounded.
-// (Checked against the host compiler's complex division on random quotients
-// spanning 2^-60..2^60, zero parts included; non-finite inputs are not
-// reproduced.)
+// The triangle in solve order (conjugated for 'C') and the reciprocals of its
+// diagonal, in shared memory.
 template <typename R>
-__device__ __forceinline__ void ZDiv(R ar, R ai, R cr, R ci, R* xr, R* xi) {
-  if constexpr (sizeof(R) == 8) {
-    double a = ar, b = ai, c = cr, d = ci;
-    const double kBig = DBL_MAX / 2, kMin = DBL_MIN, kEps = DBL_EPSILON;
-    const double kScale = 1.0 / kEps, kMax2 = kBig * kEps;
-    double x, y;
-    if (fabs(c) < fabs(d)) {
-      if (fabs(d) >= kBig) {
-        a = a / 2; b = b / 2; c = c / 2; d = d / 2;
-      }
-      if (fabs(d) < kEps) {
-        a = a * kScale; b = b * kScale; c = c * kScale; d = d * kScale;
-      } else if ((fabs(a) < kMin && fabs(b) < kMax2 && fabs(d) < kMax2) ||
-                 (fabs(b) < kMin && fabs(a) < kMax2 && fabs(d) < kMax2)) {
-        a = a * kScale; b = b * kScale; c = c * kScale; d = d * kScale;
-      }
-      const double ratio = c / d;
-      const double denom = __dadd_rn(__dmul_rn(c, ratio), d);
-      if (fabs(ratio) > kMin) {
-        x = __dadd_rn(__dmul_rn(a, ratio), b) / denom;
-        y = __dsub_rn(__dmul_rn(b, ratio), a) / denom;
-      } else {
-        x = __dadd_rn(__dmul_rn(c, a / d), b) / denom;
-        y = __dsub_rn(__dmul_rn(c, b / d), a) / denom;
-      }
-    } else {
-      if (fabs(c) >= kBig) {
-        a = a / 2; b = b / 2; c = c / 2; d = d / 2;
-      }
-      if (fabs(c) < kEps) {
-        a = a * kScale; b = b * kScale; c = c * kScale; d = d * kScale;
-      } else if ((fabs(a) < kMin && fabs(b) < kMax2 && fabs(c) < kMax2) ||
-                 (fabs(b) < kMin && fabs(a) < kMax2 && fabs(c) < kMax2)) {
-        a = a * kScale; b = b * kScale; c = c * kScale; d = d * kScale;
-      }
-      const double ratio = d / c;
-      const double denom = __dadd_rn(__dmul_rn(d, ratio), c);
-      if (fabs(ratio) > kMin) {
-        x = __dadd_rn(__dmul_rn(b, ratio), a) / denom;
-        y = __dsub_rn(b, __dmul_rn(a, ratio)) / denom;
-      } else {
-        x = __dadd_rn(a, __dmul_rn(d, b / c)) / denom;
-        y = __dsub_rn(b, __dmul_rn(d, a / c)) / denom;
-      }
-    }
-    *xr = x;
-    *xi = y;
-  } else {
-    const double a = ar, b = ai, c = cr, d = ci;
-    const double den = __dadd_rn(__dmul_rn(c, c), __dmul_rn(d, d));
-    const double re = __dadd_rn(__dmul_rn(a, c), __dmul_rn(b, d));
-    const double im = __dsub_rn(__dmul_rn(b, c), __dmul_rn(a, d));
-    *xr = static_cast<float>(re / den);
-    *xi = static_cast<float>(im / den);
-  }
-}
-
-// 1 / (c + i d): the quotient above with numerator (1, 0).
-template <typename R>
-__device__ __forceinline__ void ZRecip(R cr, R ci, R* xr, R* xi) {
-  ZDiv<R>(R(1), R(0), cr, ci, xr, xi);
-}
-
-// Complex TRSM base: X T = B for independent rows of X (src/trsm-inl.h:
-// 175-214), T r x r (r <= 32) read through a view. Column j (solve order) is
-// b_j - sum of x_q t(q, j) over the solved q in increasing q, kept as four
-// fma chains (xr tr, xi tr, xr ti, xi ti) combined as (rr - ii, ir + ri),
-// then times inv_j = 1 / t(j, j). One thread owns one row; the row sits in
-// registers indexed in solve order (static indices), T in shared memory.
-// Element (row, j) of X is at x + 2 * (row * xs_row + j * xs_col).
-template <typename R>
-__global__ void __launch_bounds__(128)
-    ZTrsmBaseKernel(ZView<R> tri, int lower, int unit, int r, int rows, R* x,
-                    long long xs_row, long long xs_col, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
-  // st[s][u] = T(q(s), j(u)) in solve order (conjugated for 'C').
-  __shared__ R st_re[32][33], st_im[32][33];
-  __shared__ R inv_re[32], inv_im[32];
+__device__ __forceinline__ void ZLoadTriangle(const ZView<R>& tri, int lower, int unit, int r,
+                                              R (*st_re)[33], R (*st_im)[33], R* inv_re,
+                                              R* inv_im) {
   for (int idx = threadIdx.x; idx < 32 * 32; idx += blockDim.x) {
     const int s = idx / 32, u = idx % 32;
     R vr = R(0), vi = R(0);
@@ -641,6 +541,24 @@ __global__ void __launch_bounds__(128)
     inv_im[s] = b;
   }
   __syncthreads();
+}
+
+// Complex TRSM base: X T = B for independent rows of X (src/trsm-inl.h:
+// 175-214), T r x r (r <= 32) read through a view. Column j (solve order) is
+// b_j - sum of x_q t(q, j) over the solved q in increasing q, kept as four
+// fma chains (xr tr, xi tr, xr ti, xi ti) combined as (rr - ii, ir + ri),
+// then times inv_j = 1 / t(j, j). One thread owns one row; the row sits in
+// registers indexed in solve order (static indices), T in shared memory.
+// Element (row, j) of X is at x + 2 * (row * xs_row + j * xs_col).
+template <typename R>
+__global__ void __launch_bounds__(128)
+    ZTrsmBaseKernel(ZView<R> tri, int lower, int unit, int r, int rows, R* x,
+                    long long xs_row, long long xs_col, const int* guard) {
+  if (guard != nullptr && *guard != 0) return;
+  // st[s][u] = T(q(s), j(u)) in solve order (conjugated for 'C').
+  __shared__ R st_re[32][33], st_im[32][33];
+  __shared__ R inv_re[32], inv_im[32];
+  ZLoadTriangle<R>(tri, lower, unit, r, st_re, st_im, inv_re, inv_im);
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= rows) return;
   R* xr = x + 2 * (row * xs_row);
@@ -701,6 +619,68 @@ __global__ void __launch_bounds__(128)
   }
 }
 
+// The same for an upper T, whose columns are solved in increasing order: two
+// rows a warp, lane s holding the element of step s and its four chains, which
+// take x_q's term as soon as step q has made it and sent it round by shuffles.
+// (A lower T is solved from its last column while the chains run over
+// increasing columns: there each column waits for the one solved just before
+// it, and ZTrsmBaseKernel's order is all there is.) One row a thread unrolled,
+// a launch took 15 us, most of it fetching its instructions.
+constexpr int kZLaneThreads = 256, kZLaneRows = 2 * kZLaneThreads / 32;
+template <typename R>
+__global__ void __launch_bounds__(kZLaneThreads)
+    ZTrsmLaneKernel(ZView<R> tri, int unit, int r, int rows, R* x, long long xs_row,
+                    long long xs_col, const int* guard) {
+  if (guard != nullptr && *guard != 0) return;
+  __shared__ R st_re[32][33], st_im[32][33];
+  __shared__ R inv_re[32], inv_im[32];
+  ZLoadTriangle<R>(tri, 0, unit, r, st_re, st_im, inv_re, inv_im);
+  const int lane = threadIdx.x % 32, row0 = blockIdx.x * kZLaneRows + threadIdx.x / 32 * 2;
+  R y[2][2], acc[2][4];  // re, im; rr, ir, ri, ii
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const R* e = x + 2 * ((row0 + i) * xs_row + lane * xs_col);
+    const bool in = row0 + i < rows && lane < r;
+    y[i][0] = in ? e[0] : R(0);
+    y[i][1] = in ? e[1] : R(0);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[i][c] = R(0);
+  }
+  const R vr = inv_re[lane], vi = inv_im[lane];
+#pragma unroll 1
+  for (int q = 0; q < r; ++q) {
+    const R tr = st_re[q][lane], ti = st_im[q][lane];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      R re = Sub(y[i][0], Sub(acc[i][0], acc[i][3]));
+      R im = Sub(y[i][1], Add(acc[i][1], acc[i][2]));
+      if (!unit) {
+        const R a0 = Mul(re, vr), a1 = Mul(im, vi), a2 = Mul(im, vr), a3 = Mul(re, vi);
+        re = Sub(a0, a1);
+        im = Add(a2, a3);
+      }
+      re = __shfl_sync(0xffffffffu, re, q);
+      im = __shfl_sync(0xffffffffu, im, q);
+      if (lane == q) {
+        y[i][0] = re;
+        y[i][1] = im;
+      } else if (lane > q) {
+        acc[i][0] = Fma(re, tr, acc[i][0]);
+        acc[i][1] = Fma(im, tr, acc[i][1]);
+        acc[i][2] = Fma(re, ti, acc[i][2]);
+        acc[i][3] = Fma(im, ti, acc[i][3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (row0 + i >= rows || lane >= r) continue;
+    R* e = x + 2 * ((row0 + i) * xs_row + lane * xs_col);
+    e[0] = y[i][0];
+    e[1] = y[i][1];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Complex LU leaf (src/lapack/factor_kernels.cc:107-139 for complex T).
 //
@@ -737,50 +717,6 @@ struct ZLeafArgs {
   unsigned int* tags;    // [2][P], zeroed before a cooperative launch
   int* timeout_flag;
 };
-
-template <typename R>
-__device__ __forceinline__ R ZMag(R re, R im) {
-  return Add(fabs(re), fabs(im));
-}
-
-template <typename R>
-__device__ __forceinline__ bool ZBetter(R v, int i, R bv, int bi) {
-  return v > bv || (v == bv && v >= R(0) && i < bi);
-}
-
-// std::abs(z) >= s for the safe minimum s. |z| is at least the larger part,
-// so only two parts below s need the magnitude itself: they are scaled by an
-// exact power of two (double) or widened (float) and the square root of the
-// sum of squares is compared in double precision. (std::abs is hypot: an
-// infinite part gives infinity, otherwise a NaN part gives NaN.)
-template <typename R>
-__device__ __forceinline__ bool ZAbsAtLeast(R re, R im, R s) {
-  const R ar = fabs(re), ai = fabs(im);
-  if (isinf(ar) || isinf(ai)) return true;
-  if (isnan(ar) || isnan(ai)) return false;
-  if ((ar > ai ? ar : ai) >= s) return true;
-  const double k = sizeof(R) == 8 ? 0x1p600 : 1.0;
-  const double sr = __dmul_rn(static_cast<double>(ar), k);
-  const double si = __dmul_rn(static_cast<double>(ai), k);
-  const double mag = sqrt(__dadd_rn(__dmul_rn(sr, sr), __dmul_rn(si, si)));
-  return mag >= __dmul_rn(static_cast<double>(s), k);
-}
-
-// y += alpha x for one element of a column of len complex elements.
-template <typename R>
-__device__ __forceinline__ void ZAxpyRef(R& yr, R& yi, R ar, R ai, R xr, R xi, int len,
-                                         int lanes) {
-  if (2 * len < lanes) {
-    const R pr = Sub(Mul(ar, xr), Mul(ai, xi));
-    const R pi = Add(Mul(ar, xi), Mul(ai, xr));
-    yr = Add(yr, pr);
-    yi = Add(yi, pi);
-  } else {
-    const R tr = Fma(xr, ar, yr), ti = Fma(xi, ar, yi);
-    yr = Fma(xi, -ai, tr);
-    yi = Fma(xr, ai, ti);
-  }
-}
 
 // kCluster: the P CTAs form one thread-block cluster and exchange their
 // candidates through distributed shared memory (each publishes into its own
@@ -1270,8 +1206,14 @@ static void ZTrsmRec(bool left, ZView<R> tri, bool lower, bool unit, int r, int 
       xs_row = 1;
       xs_col = ldb;
     }
-    ZTrsmBaseKernel<R><<<(other + 127) / 128, 128, 0, Ctx().stream>>>(
-        t, lo ? 1 : 0, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
+    if (!lo) {
+      ZTrsmLaneKernel<R>
+          <<<(other + kZLaneRows - 1) / kZLaneRows, kZLaneThreads, 0, Ctx().stream>>>(
+              t, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
+    } else {
+      ZTrsmBaseKernel<R><<<(other + 127) / 128, 128, 0, Ctx().stream>>>(
+          t, 1, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
+    }
     CountLaunch();
     LaunchFailed("complex trsm base");
     return;
@@ -1533,6 +1475,7 @@ void ZGetrfLeaf(int m, int n, R* a, int lda, int* ipiv, int* info, int info_base
 template <typename R>
 void ZGetrfRec(int m, int n, R* a, int lda, int* ipiv, int* info, int col0) {
   if (m == 0 || n == 0) return;
+  if (ZGetrfPanel<R>(m, n, a, lda, ipiv, 0, info, col0, nullptr)) return;
   if (std::min(m, n) <= 16) {
     ZGetrfLeaf<R>(m, n, a, lda, ipiv, info, col0);
     return;
@@ -1550,6 +1493,10 @@ void ZGetrfRec(int m, int n, R* a, int lda, int* ipiv, int* info, int col0) {
 }
 }  // namespace
 
+// The blocked LU with the real one's look-ahead (Getrf): on the side stream panel
+// j's interchanges, solve and update reach panel j + 1's columns first, which is
+// then factored there, while the context's stream updates the others. The columns
+// are independent, so every element's operations are the reference's.
 template <typename R>
 void ZGetrf(bool recursive, int m, int n, R* a, int lda, int* ipiv, int* info) {
   if (m == 0 || n == 0) return;
@@ -1559,30 +1506,71 @@ void ZGetrf(bool recursive, int m, int n, R* a, int lda, int* ipiv, int* info) {
     ZGetrfRec<R>(m, n, a, lda, ipiv, info, 0);
     return;
   }
+  // Both streams' split buffers, and the panels' lists of moved rows.
   size_t split_bytes = 0;
   for (int j = 0; j < mn; j += nb) {
     const int jb = std::min(mn - j, nb);
     split_bytes = std::max({split_bytes, ZGetrfSplitMax<R>(m - j, jb),
                             ZTrsmSplitMax<R>(jb, n - j - jb),
-                            ZSplitBytes<R>(m - j - jb, n - j - jb, jb)});
+                            ZSplitBytes<R>(m - j - jb, n - j - jb, jb),
+                            ZSplitBytes<R>(m - j - jb, std::min(nb, n - j - jb), jb)});
   }
-  if (!ZReserveSplit<R>(split_bytes)) return;
+  bool reserved = ZReserveSplit<R>(split_bytes);
+  OnSide([&] { reserved = ZReserveSplit<R>(split_bytes) && reserved; });
+  if (!reserved) return;
+  constexpr int kList = 2 + kPanelMoves;
+  const size_t list_bytes = sizeof(int) * kList * static_cast<size_t>((mn + nb - 1) / nb);
+  int* lists = static_cast<int*>(Workspace(kWsLuMoves, list_bytes));
+  if (lists == nullptr) return;
+  SideStream& side = Side();
+  const cudaStream_t main = Ctx().stream;
+  const cudaStream_t look = side.ok ? side.stream : main;
+  cudaMemsetAsync(lists, 0, list_bytes, main);
   const R one[2] = {R(1), R(0)}, m1[2] = {R(-1), R(0)};
-  for (int j = 0; j < mn; j += nb) {
-    const int jb = std::min(mn - j, nb);
-    ZGetrfRec<R>(m - j, jb, ZAt(a, lda, j, j), lda, ipiv + j, info, j);
-    AdjustPivots(ipiv, j, std::min(m, j + jb), j);
-    ZLaswp<R>(j, a, lda, j + 1, j + jb, ipiv, 1);
-    if (j + jb < n) {
-      ZLaswp<R>(n - j - jb, ZAt(a, lda, 0, j + jb), lda, j + 1, j + jb, ipiv, 1);
-      ZtrsmFull<R>(true, true, 0, true, jb, n - j - jb, one, ZAt(a, lda, j, j), lda,
-                   ZAt(a, lda, j, j + jb), lda);
-      if (j + jb < m) {
-        ZgemmFull<R>(0, 0, m - j - jb, n - j - jb, jb, m1, ZAt(a, lda, j + jb, j), lda,
-                     ZAt(a, lda, j, j + jb), lda, one, ZAt(a, lda, j + jb, j + jb), lda);
+  bool listed = false;
+  const auto panel = [&](int j, int jb) {
+    R* at = ZAt(a, lda, j, j);
+    listed = ZGetrfPanel<R>(m - j, jb, at, lda, ipiv + j, j, info, j, lists + j / nb * kList);
+    if (!listed) {
+      ZGetrfRec<R>(m - j, jb, at, lda, ipiv + j, info, j);
+      AdjustPivots(ipiv, j, j + jb, j);
+    }
+  };
+  const auto update = [&](int j, int jb, int left, int c0, int nc, bool list) {
+    if (list) {
+      ZPanelSwapTrsm<R>(j, jb, left, c0, nc, a, lda, lists + j / nb * kList);
+    } else {
+      ZLaswp<R>(left, a, lda, j + 1, j + jb, ipiv, 1);
+      if (nc > 0) {
+        ZLaswp<R>(nc, ZAt(a, lda, 0, c0), lda, j + 1, j + jb, ipiv, 1);
+        ZtrsmFull<R>(true, true, 0, true, jb, nc, one, ZAt(a, lda, j, j), lda,
+                     ZAt(a, lda, j, c0), lda);
       }
     }
+    if (nc > 0 && j + jb < m) {
+      ZgemmFull<R>(0, 0, m - j - jb, nc, jb, m1, ZAt(a, lda, j + jb, j), lda,
+                   ZAt(a, lda, j, c0), lda, one, ZAt(a, lda, j + jb, c0), lda);
+    }
+  };
+  StreamAfter(side.to_side, main, look);
+  OnSide([&] { panel(0, nb); });
+  for (int j = 0; j < mn; j += nb) {
+    const int jb = std::min(mn - j, nb);
+    const int right = n - j - jb;               // columns right of the panel
+    const int next = std::min(nb, right);       // the next panel's columns
+    const int jb2 = std::min(mn - j - jb, nb);  // the next panel's width
+    const bool list = listed;
+    StreamAfter(side.to_side, main, look);
+    StreamAfter(side.to_main, look, main);
+    if (next > 0) {
+      OnSide([&] {
+        update(j, jb, 0, j + jb, next, list);
+        if (jb2 > 0) panel(j + jb, jb2);
+      });
+    }
+    update(j, jb, j, j + jb + next, std::max(0, right - next), list);
   }
+  StreamAfter(side.to_main, look, main);
 }
 template void ZGetrf<double>(bool, int, int, double*, int, int*, int*);
 template void ZGetrf<float>(bool, int, int, float*, int, int*, int*);

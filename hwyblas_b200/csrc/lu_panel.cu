@@ -18,10 +18,13 @@
 // to every CTA of the cluster by st.async (one one-way trip; the receiving
 // mbarrier counts the bytes), and every warp picks the winner by itself.
 // After a leaf, every CTA collects its pivot rows' other columns and solves
-// the small triangles for itself.
+// the small triangles for itself. T is float, double or a complex element
+// (Cx<float>, Cx<double>): the complex LU has the same recursion and leaves, on
+// |re| + |im| and the complex AXPY, product and quotient of complex.cuh.
 #include <algorithm>
 #include <cstdio>
 
+#include "complex.cuh"
 #include "device.cuh"
 #include "internal.h"
 #include "ref_order.cuh"
@@ -34,12 +37,123 @@ constexpr int kPanelLeaf = 16;     // src/lapack/factor_kernels.h:27
 // Row stride of the pivot rows: 16-byte aligned, few bank conflicts by column.
 template <typename T>
 constexpr int kPanelLd = kPanelW + 16 / static_cast<int>(sizeof(T));
-constexpr int kPanelThreads = 512;  // rows of a CTA at most
+// Rows of a CTA at most: its registers hold 16 elements a row.
+template <typename T>
+constexpr int kPanelThreads = sizeof(T) == 16 ? 256 : 512;
 constexpr int kPanelLeast = 256;   // threads at least: the solves share all warps
 constexpr int kPanelCtas = 16;
 // Polls of a wait for the other CTAs' candidates (some 30 ns each): far above
 // any real wait.
 constexpr uint32_t kPanelPolls = 1u << 22;
+
+template <typename R>
+struct __align__(2 * sizeof(R)) Cx {
+  R re, im;
+};
+template <typename T>
+struct ElemOf {
+  using Real = T;
+  static constexpr bool kComplex = false;
+};
+template <typename R>
+struct ElemOf<Cx<R>> {
+  using Real = R;
+  static constexpr bool kComplex = true;
+};
+template <typename T>
+using RealOf = typename ElemOf<T>::Real;
+
+// The leaf's element operations (src/lapack/factor_kernels.cc:33-183).
+template <typename T>
+__device__ __forceinline__ T Zero() {
+  if constexpr (ElemOf<T>::kComplex) return T{0, 0};
+  else return T(0);
+}
+__device__ __forceinline__ bool IsZero(double x) { return x == 0.0; }
+__device__ __forceinline__ bool IsZero(float x) { return x == 0.f; }
+template <typename R>
+__device__ __forceinline__ bool IsZero(Cx<R> x) {
+  return x.re == R(0) && x.im == R(0);
+}
+template <typename T>
+__device__ __forceinline__ bool IsTiny(T x) {
+  if constexpr (ElemOf<T>::kComplex)
+    return !ZAbsAtLeast(x.re, x.im, Sfmin<RealOf<T>>());
+  else
+    return !(fabs(x) >= Sfmin<T>());
+}
+template <typename T>
+__device__ __forceinline__ T Recip(T x) {
+  if constexpr (ElemOf<T>::kComplex) {
+    T r;
+    ZRecip(x.re, x.im, &r.re, &r.im);
+    return r;
+  } else {
+    return T(1) / x;
+  }
+}
+template <typename T>
+__device__ __forceinline__ T Times(T x, T v) {
+  if constexpr (ElemOf<T>::kComplex)
+    return T{Sub(Mul(x.re, v.re), Mul(x.im, v.im)), Add(Mul(x.im, v.re), Mul(x.re, v.im))};
+  else
+    return x * v;
+}
+template <typename T>
+__device__ __forceinline__ T Over(T x, T p) {
+  if constexpr (ElemOf<T>::kComplex) {
+    T q;
+    ZDiv(x.re, x.im, p.re, p.im, &q.re, &q.im);
+    return q;
+  } else {
+    return x / p;
+  }
+}
+// y - u l in the AXPY rounding of a column of len elements.
+template <typename T>
+__device__ __forceinline__ T AxpyMinus(T y, T u, T l, int len, int lanes) {
+  if constexpr (ElemOf<T>::kComplex) {
+    ZAxpyRef(y.re, y.im, -u.re, -u.im, l.re, l.im, len, lanes);
+    return y;
+  } else {
+    return Axpy(y, -u, l, len, lanes);
+  }
+}
+// The same for a column of at least one vector.
+template <typename T>
+__device__ __forceinline__ T AxpyMinusLong(T y, T u, T l) {
+  if constexpr (ElemOf<T>::kComplex)
+    return AxpyMinus(y, u, l, 1, 0);
+  else
+    return fma(l, -u, y);
+}
+template <typename T>
+__device__ __forceinline__ T Shfl(T x, int from) {
+  if constexpr (ElemOf<T>::kComplex)
+    return T{__shfl_sync(0xffffffffu, x.re, from), __shfl_sync(0xffffffffu, x.im, from)};
+  else
+    return __shfl_sync(0xffffffffu, x, from);
+}
+// Global elements are aligned as their real parts.
+template <typename T>
+__device__ __forceinline__ T LoadGlobal(const T* p) {
+  if constexpr (ElemOf<T>::kComplex) {
+    const RealOf<T>* r = reinterpret_cast<const RealOf<T>*>(p);
+    return T{r[0], r[1]};
+  } else {
+    return *p;
+  }
+}
+template <typename T>
+__device__ __forceinline__ void StoreGlobal(T* p, T v) {
+  if constexpr (ElemOf<T>::kComplex) {
+    RealOf<T>* r = reinterpret_cast<RealOf<T>*>(p);
+    r[0] = v.re;
+    r[1] = v.im;
+  } else {
+    *p = v;
+  }
+}
 
 // A CTA's candidate of one column: its key, its position after and its place
 // before the interchanges, and the row from that column on. The reciprocal of
@@ -75,17 +189,23 @@ __device__ __forceinline__ unsigned long long PivotKey(float x) {
   return v > 0x7f800000u ? 0ull : static_cast<unsigned long long>(v) + 1;
 }
 
+template <typename R>
+__device__ __forceinline__ unsigned long long PivotKey(Cx<R> x) {
+  return PivotKey(ZMag(x.re, x.im));
+}
+
 // The lane with the warp's largest key, the one with the smallest position if
 // several hold it. The keys' high words nearly always decide.
 template <typename T>
 __device__ __forceinline__ int WarpBest(unsigned long long key, int pos) {
   const unsigned lo = static_cast<unsigned>(key), hi = static_cast<unsigned>(key >> 32);
-  const unsigned word = sizeof(T) == 8 ? hi : lo;
+  constexpr bool kWide = sizeof(RealOf<T>) == 8;
+  const unsigned word = kWide ? hi : lo;
   const unsigned largest = __reduce_max_sync(0xffffffffu, word);
   unsigned top = __ballot_sync(0xffffffffu, word == largest);
   if (top & (top - 1)) {
     const bool in = (top >> (threadIdx.x % 32)) & 1;
-    const unsigned second = sizeof(T) == 8 && in ? lo : 0u;
+    const unsigned second = kWide && in ? lo : 0u;
     const unsigned most = __reduce_max_sync(0xffffffffu, second);  // by every lane
     const bool in2 = in && second == most;
     const int first = __reduce_min_sync(0xffffffffu, in2 ? pos : 0x7fffffff);
@@ -122,6 +242,13 @@ __device__ __forceinline__ void StAsync(uint32_t dst, float v, uint32_t bar) {
       : "r"(dst), "r"(__float_as_int(v)), "r"(bar)
       : "memory");
 }
+__device__ __forceinline__ void StAsync(uint32_t dst, Cx<float> v, uint32_t bar) {
+  StAsync(dst, __hiloint2double(__float_as_int(v.im), __float_as_int(v.re)), bar);
+}
+__device__ __forceinline__ void StAsync(uint32_t dst, Cx<double> v, uint32_t bar) {
+  StAsync16(dst,
+            make_ulonglong2(__double_as_longlong(v.re), __double_as_longlong(v.im)), bar);
+}
 __device__ __forceinline__ double LoadRemote(uint32_t addr, double) {
   double v;
   asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
@@ -131,6 +258,10 @@ __device__ __forceinline__ float LoadRemote(uint32_t addr, float) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
+}
+template <typename R>
+__device__ __forceinline__ Cx<R> LoadRemote(uint32_t addr, Cx<R>) {
+  return Cx<R>{LoadRemote(addr, R(0)), LoadRemote(addr + sizeof(R), R(0))};
 }
 __device__ __forceinline__ bool MbarTest(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -153,8 +284,14 @@ __device__ __forceinline__ void ClusterBarrier() {
 // One element global -> shared, asynchronously.
 template <typename T>
 __device__ __forceinline__ void CopyElement(T* dst, const T* src) {
+  if constexpr (ElemOf<T>::kComplex) {
+    using R = RealOf<T>;
+    CopyElement(reinterpret_cast<R*>(dst), reinterpret_cast<const R*>(src));
+    CopyElement(reinterpret_cast<R*>(dst) + 1, reinterpret_cast<const R*>(src) + 1);
+    return;
+  }
   asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(SmemAddr(dst)), "l"(src),
-               "n"(sizeof(T))
+               "n"(ElemOf<T>::kComplex ? 4 : sizeof(T))
                : "memory");
 }
 
@@ -165,13 +302,39 @@ __device__ __forceinline__ void CopyElement(T* dst, const T* src) {
 template <typename T, int N>
 __device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[N]) {
   const int lane = threadIdx.x % 32;
-#pragma unroll 4
-  for (int q = 0; q + 1 < r; ++q) {
-    const T l = lrow[q];
+  if constexpr (ElemOf<T>::kComplex) {
+    // Four chains an element from zero (src/trsm-inl.h:175-214), combined when
+    // its step comes.
+    using R = RealOf<T>;
+    R rr[N], ir[N], ri[N], ii[N];
 #pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const T yq = __shfl_sync(0xffffffffu, y[i], q);
-      if (lane > q) y[i] = fma(-yq, l, y[i]);
+    for (int i = 0; i < N; ++i) rr[i] = ir[i] = ri[i] = ii[i] = R(0);
+#pragma unroll 1
+    for (int q = 0; q < r; ++q) {
+      const T l = lrow[q];
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const T v = T{Sub(y[i].re, Sub(rr[i], ii[i])), Sub(y[i].im, Add(ir[i], ri[i]))};
+        const T yq = Shfl(v, q);
+        if (lane == q) {
+          y[i] = yq;
+        } else if (lane > q) {
+          rr[i] = Fma(yq.re, l.re, rr[i]);
+          ir[i] = Fma(yq.im, l.re, ir[i]);
+          ri[i] = Fma(yq.re, l.im, ri[i]);
+          ii[i] = Fma(yq.im, l.im, ii[i]);
+        }
+      }
+    }
+  } else {
+#pragma unroll 4
+    for (int q = 0; q + 1 < r; ++q) {
+      const T l = lrow[q];
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const T yq = __shfl_sync(0xffffffffu, y[i], q);
+        if (lane > q) y[i] = fma(-yq, l, y[i]);
+      }
     }
   }
 }
@@ -180,7 +343,7 @@ __device__ __forceinline__ void LaneSolve(const T* lrow, int r, T (&y)[N]) {
 // lower in their columns [0, n1), U in columns [n1, n1 + n2)).
 template <typename T>
 __device__ __forceinline__ void PanelSolve(T* rows, int n1, int n2) {
-  constexpr int N = 4;
+  constexpr int N = ElemOf<T>::kComplex ? 2 : 4;
   const int lane = threadIdx.x % 32, nwarps = blockDim.x / 32;
   T* row = rows + min(lane, n1 - 1) * kPanelLd<T>;
   for (int c = N * (threadIdx.x / 32); c < n2; c += N * nwarps) {
@@ -241,8 +404,55 @@ __device__ __forceinline__ void PanelUpdate(const T* l, T* x, int R, const T* u,
   }
 }
 
+// c + (-1) ab for ab = (rr - ii, ir + ri): the GEMM merge with alpha -1, beta 1.
+template <typename R>
+__device__ __forceinline__ Cx<R> MinusProduct(Cx<R> c, R rr, R ir, R ri, R ii) {
+  const R re = Sub(rr, ii), im = Add(ir, ri);
+  return Cx<R>{Add(Sub(Mul(re, R(-1)), Mul(im, R(0))), c.re),
+               Add(Add(Mul(im, R(-1)), Mul(re, R(0))), c.im)};
+}
+
+// The complex update: four chains an element, combined as the product with
+// alpha -1 and added (src/gemm_kernel-inl.h:226-428), four columns at a time.
+template <typename R>
+__device__ __forceinline__ void PanelUpdateComplex(const Cx<R>* l, Cx<R>* x, int S,
+                                                   const Cx<R>* u, int n1, int nc, int ra,
+                                                   int rb, bool ina, bool inb) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < nc; c0 += 4) {
+    R acc[2][4][4];  // rr, ir, ri, ii
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i / 16][i / 4 % 4][i % 4] = R(0);
+#pragma unroll 2
+    for (int q = 0; q < n1; ++q) {
+      const Cx<R> lv[2] = {l[q * S + ra], l[q * S + rb]};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const Cx<R> uv = u[q * kPanelLd<Cx<R>> + c0 + c];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          acc[i][c][0] = Fma(lv[i].re, uv.re, acc[i][c][0]);
+          acc[i][c][1] = Fma(lv[i].im, uv.re, acc[i][c][1]);
+          acc[i][c][2] = Fma(lv[i].re, uv.im, acc[i][c][2]);
+          acc[i][c][3] = Fma(lv[i].im, uv.im, acc[i][c][3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (c0 + c >= nc) continue;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (!(i == 0 ? ina : inb)) continue;
+        Cx<R>& e = x[(c0 + c) * S + (i == 0 ? ra : rb)];
+        e = MinusProduct(e, acc[i][c][0], acc[i][c][1], acc[i][c][2], acc[i][c][3]);
+      }
+    }
+  }
+}
+
 template <typename T>
-__global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p) {
+__global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T> p) {
   extern __shared__ __align__(16) unsigned char panel_smem[];
   const int P = gridDim.x, cta = blockIdx.x, R = p.R, w = p.w;
   // [2][kPanelCtas] from the CTAs, then this CTA's own.
@@ -251,9 +461,9 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
   T* prow = reinterpret_cast<T*>(own + 1);                           // [w][kPanelLd] pivot rows
   T* S = prow + w * kPanelLd<T>;                                     // [w][R] this CTA's rows
   __shared__ T s_rinv[2][kPanelCtas];
-  __shared__ unsigned long long s_wkey[2][kPanelThreads / 32];
-  __shared__ int s_wpos[2][kPanelThreads / 32];
-  __shared__ int s_place[kPanelW], s_pos[kPanelThreads], s_op[7][4];
+  __shared__ unsigned long long s_wkey[2][kPanelThreads<T> / 32];
+  __shared__ int s_wpos[2][kPanelThreads<T> / 32];
+  __shared__ int s_place[kPanelW], s_pos[kPanelThreads<T>], s_op[7][4];
   __shared__ __align__(8) uint64_t s_bar[2], s_rbar[2];
   __shared__ int s_ops;
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, nwarps = blockDim.x / 32;
@@ -313,7 +523,7 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
       T x[kPanelLeaf];
 #pragma unroll
       for (int k = 0; k < kPanelLeaf; ++k)
-        x[k] = valid && k < n1 ? S[(c0 + k) * R + tid] : T(0);
+        x[k] = valid && k < n1 ? S[(c0 + k) * R + tid] : Zero<T>();
 #pragma unroll 1
       for (int j = 0; j < n1; ++j) {
         const int jc = c0 + j, par = jc & 1;
@@ -324,7 +534,8 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
         // The warp's candidate among the rows not yet taken (position >= jc). A
         // NaN at position jc wins, as the reference's search starts from it.
         unsigned long long key = valid && pos >= jc ? PivotKey(x[0]) : 0ull;
-        if (valid && pos == jc && key == 0) key = sizeof(T) == 8 ? ~0ull : 0xffffffffull;
+        if (valid && pos == jc && key == 0)
+          key = sizeof(RealOf<T>) == 8 ? ~0ull : 0xffffffffull;
         const int wbest = WarpBest<T>(key, pos);
         if (lane == wbest) {
           s_wkey[par][warp] = key;
@@ -353,7 +564,7 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
               StAsync16(MapRank(dst + 16 * e, to), src[e], MapRank(bar, to));
             }
           }
-          const T rinv = T(1) / own->row[0];
+          const T rinv = Recip(own->row[0]);
           if (P > 1) {
             if (lane < P)
               StAsync(MapRank(SmemAddr(&s_rinv[par][cta]), lane), rinv,
@@ -387,7 +598,7 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
           s_place[jc] = win->place;
           if (cta == 0) {
             p.ipiv[jc] = piv + 1 + p.ipiv_add;
-            if (pivot == T(0) && *p.info == 0) *p.info = p.info_base + jc + 1;
+            if (IsZero(pivot) && *p.info == 0) *p.info = p.info_base + jc + 1;
           }
         }
         // A zero pivot is at position jc already.
@@ -403,20 +614,20 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
           // The column below the pivot times its reciprocal (divided if the
           // pivot is below the safe minimum, kept if it is zero), then the
           // rank-1 update of the leaf's later columns, which move up by one.
-          T l = x[0] * s_rinv[par][from & (kPanelCtas - 1)];
-          if (!(fabs(pivot) >= Sfmin<T>())) l = pivot != T(0) ? x[0] / pivot : x[0];
+          T l = Times(x[0], s_rinv[par][from & (kPanelCtas - 1)]);
+          if (IsTiny(pivot)) l = IsZero(pivot) ? x[0] : Over(x[0], pivot);
           S[jc * R + tid] = l;
           const int len = p.m - jc - 1;
           if (len >= p.lanes) {
 #pragma unroll
             for (int k = 1; k < kPanelLeaf; ++k) {
               if (k == 9 && n1 - j <= 9) break;  // no such columns
-              x[k - 1] = fma(l, -win->row[k], x[k]);
+              x[k - 1] = AxpyMinusLong(x[k], win->row[k], l);
             }
           } else {
 #pragma unroll
             for (int k = 1; k < kPanelLeaf; ++k)
-              x[k - 1] = Axpy(x[k], -win->row[k], l, len, p.lanes);
+              x[k - 1] = AxpyMinus(x[k], win->row[k], l, len, p.lanes);
           }
         }
       }
@@ -435,7 +646,8 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
             const int col = lane + 32 * d;
             if (col >= w || (col >= c0 + r && col < c0 + n1)) continue;
             prow[(c0 + r) * kPanelLd<T> + col] =
-                P > 1 ? LoadRemote(MapRank(SmemAddr(row + col * R), owner), T(0)) : row[col * R];
+                P > 1 ? LoadRemote(MapRank(SmemAddr(row + col * R), owner), Zero<T>())
+                      : row[col * R];
           }
         }
         __syncthreads();
@@ -453,7 +665,10 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
         const int cb = n1 + blk * cw;
         const bool ina = s_pos[ra] >= c0 + n1;
         const bool inb = ra + half < R && s_pos[rb] >= c0 + n1;
-        if ((c0 + cb) % (16 / static_cast<int>(sizeof(T))) == 0)
+        if constexpr (ElemOf<T>::kComplex)
+          PanelUpdateComplex(S + c0 * R, S + (c0 + cb) * R, R, rows + cb, n1, nc, ra, rb, ina,
+                             inb);
+        else if ((c0 + cb) % (16 / static_cast<int>(sizeof(T))) == 0)
           PanelUpdate<T, true>(S + c0 * R, S + (c0 + cb) * R, R, rows + cb, n1, nc, cw, ra, rb,
                                ina, inb);
         else
@@ -467,12 +682,12 @@ __global__ void __launch_bounds__(kPanelThreads) GetrfPanelKernel(PanelArgs<T> p
 #pragma unroll 4
     for (int i = tid; i < (w - cta + P - 1) / P * kPanelW; i += blockDim.x) {
       const int r = i % kPanelW, c = cta + i / kPanelW * P;
-      if (r < w) p.a[r + c * p.lda] = prow[r * kPanelLd<T> + c];
+      if (r < w) StoreGlobal(p.a + r + c * p.lda, prow[r * kPanelLd<T> + c]);
     }
     if (valid && pos >= w) {
       T* dst = p.a + pos;
 #pragma unroll 8
-      for (int c = 0; c < w; ++c) dst[c * p.lda] = S[c * R + tid];
+      for (int c = 0; c < w; ++c) StoreGlobal(dst + c * p.lda, S[c * R + tid]);
     }
     if (valid && pos != place && p.moves != nullptr) {
       const int e = atomicAdd(p.moves, 1);
@@ -490,14 +705,14 @@ size_t PanelSmem(int w, int R) {
          sizeof(T) * static_cast<size_t>(w) * (kPanelLd<T> + R);
 }
 
-constexpr size_t kPanelSmemMax = 227 * 1024 - 8 * 1024;  // beside the static arrays
+constexpr size_t kPanelSmemMax = 227 * 1024 - 4 * 1024;  // beside the static arrays
 
 // CTAs and rows a CTA for an m x w panel; false if it does not fit a cluster
 // of at most `most` CTAs.
 template <typename T>
 bool PanelShape(int m, int w, int most, int* ctas, int* rows) {
-  int fit = kPanelThreads;
-  while (fit > 0 && PanelSmem<T>(w, fit) > kPanelSmemMax) fit -= 32;
+  int fit = kPanelThreads<T>;
+  while (fit > 0 && PanelSmem<T>(w, fit) > kPanelSmemMax) fit -= 8;
   if (fit <= 0) return false;
   const int least = (m + fit - 1) / fit;
   if (least > most) return false;
@@ -528,11 +743,17 @@ struct SwapArgs {
 };
 
 template <typename T>
+constexpr int SwapSmem() {
+  return static_cast<int>(sizeof(T)) * (kPanelW + kSwapCols) * (kPanelW + 1);
+}
+
+template <typename T>
 __global__ void __launch_bounds__(kSwapThreads) PanelSwapTrsmKernel(SwapArgs<T> p) {
   constexpr int kLd = kPanelW + 1;
   __shared__ int s_dst[kMovesMax], s_src[kMovesMax], s_top[kPanelW];
-  __shared__ T s_l[kPanelW * kLd];
-  __shared__ T s_b[kSwapCols][kLd];
+  extern __shared__ __align__(16) unsigned char swap_smem[];
+  T* s_l = reinterpret_cast<T*>(swap_smem);  // [kPanelW][kLd] the triangle
+  T* s_b = s_l + kPanelW * kLd;              // [kSwapCols][kLd] the columns
   const int tid = threadIdx.x, jb = p.jb;
   const int cnt = min(p.moves[0], kMovesMax);
   const int left_blocks = (p.left + kSwapCols - 1) / kSwapCols;
@@ -546,9 +767,9 @@ __global__ void __launch_bounds__(kSwapThreads) PanelSwapTrsmKernel(SwapArgs<T> 
   }
   if (tid < kPanelW) s_top[tid] = tid;
   if (solve) {
-    for (int i = tid; i < jb * jb; i += kSwapThreads) {
-      const int r = i % jb, c = i / jb;
-      s_l[r * kLd + c] = p.l[r + c * p.lda];
+    for (int i = tid; i < kPanelW * jb; i += kSwapThreads) {
+      const int r = i % kPanelW, c = i / kPanelW;
+      if (r < jb) CopyElement(s_l + r * kLd + c, p.l + r + c * p.lda);
     }
   }
   __syncthreads();
@@ -560,55 +781,85 @@ __global__ void __launch_bounds__(kSwapThreads) PanelSwapTrsmKernel(SwapArgs<T> 
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     const int e = (tid + i * kSwapThreads) % kMovesMax, c = (tid + i * kSwapThreads) / kMovesMax;
-    if (e < cnt && c < cols && !(solve && s_dst[e] < jb)) v[i] = b[s_src[e] + c * p.lda];
+    if (e < cnt && c < cols && !(solve && s_dst[e] < jb))
+      v[i] = LoadGlobal(b + s_src[e] + c * p.lda);
   }
   if (solve) {
     for (int i = tid; i < kPanelW * kSwapCols; i += kSwapThreads) {
       const int r = i % kPanelW, c = i / kPanelW;
-      s_b[c][r] = r < jb && c < cols ? b[s_top[r] + c * p.lda] : T(0);
+      if (r < jb && c < cols) CopyElement(s_b + c * kLd + r, b + s_top[r] + c * p.lda);
+      else s_b[c * kLd + r] = Zero<T>();
     }
   }
+  CpAsyncCommit();
+  CpAsyncWait<0>();
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
     const int e = (tid + i * kSwapThreads) % kMovesMax, c = (tid + i * kSwapThreads) / kMovesMax;
-    if (e < cnt && c < cols && !(solve && s_dst[e] < jb)) b[s_dst[e] + c * p.lda] = v[i];
+    if (e < cnt && c < cols && !(solve && s_dst[e] < jb))
+      StoreGlobal(b + s_dst[e] + c * p.lda, v[i]);
   }
   if (!solve) return;
   // The recursion's split (src/trsm.cc:87-135): 32 rows, the product, the rest.
   const int r1 = min(jb, 32), r2 = jb - r1, lane = tid % 32, c = tid / 32 * 2;
   static_assert(kSwapCols == 2 * (kSwapThreads / 32), "two columns a warp");
   const T* l1 = s_l + min(lane, jb - 1) * kLd;
-  T y[2] = {s_b[c][lane], s_b[c + 1][lane]};
+  const T* b0 = s_b + c * kLd;
+  const T* b1 = b0 + kLd;
+  T y[2] = {b0[lane], b1[lane]};
   LaneSolve<T, 2>(l1, r1, y);
-  T z[2] = {T(0), T(0)};
+  T z[2] = {Zero<T>(), Zero<T>()};
   if (r2 > 0) {
     const T* l2 = s_l + min(32 + lane, jb - 1) * kLd;
-    T acc[2] = {T(0), T(0)};
+    z[0] = b0[32 + lane];
+    z[1] = b1[32 + lane];
+    if constexpr (ElemOf<T>::kComplex) {
+      using R = RealOf<T>;
+      R acc[2][4] = {};
+#pragma unroll 2
+      for (int q = 0; q < 32; ++q) {
+        const T l = l2[q];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const T yq = Shfl(y[i], q);
+          acc[i][0] = Fma(l.re, yq.re, acc[i][0]);
+          acc[i][1] = Fma(l.im, yq.re, acc[i][1]);
+          acc[i][2] = Fma(l.re, yq.im, acc[i][2]);
+          acc[i][3] = Fma(l.im, yq.im, acc[i][3]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        z[i] = MinusProduct(z[i], acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    } else {
+      T acc[2] = {T(0), T(0)};
 #pragma unroll 4
-    for (int q = 0; q < 32; ++q) {
-      const T l = l2[q];
-      acc[0] = fma(l, __shfl_sync(0xffffffffu, y[0], q), acc[0]);
-      acc[1] = fma(l, __shfl_sync(0xffffffffu, y[1], q), acc[1]);
+      for (int q = 0; q < 32; ++q) {
+        const T l = l2[q];
+        acc[0] = fma(l, __shfl_sync(0xffffffffu, y[0], q), acc[0]);
+        acc[1] = fma(l, __shfl_sync(0xffffffffu, y[1], q), acc[1]);
+      }
+      z[0] = T(-1) * acc[0] + z[0];
+      z[1] = T(-1) * acc[1] + z[1];
     }
-    z[0] = T(-1) * acc[0] + s_b[c][32 + lane];
-    z[1] = T(-1) * acc[1] + s_b[c + 1][32 + lane];
     LaneSolve<T, 2>(l2 + 32, r2, z);
   }
 #pragma unroll
   for (int d = 0; d < 2; ++d) {
     if (c + d >= cols) continue;
     T* col = b + (c + d) * p.lda;
-    if (lane < r1) col[lane] = y[d];
-    if (lane < r2) col[32 + lane] = z[d];
+    if (lane < r1) StoreGlobal(col + lane, y[d]);
+    if (lane < r2) StoreGlobal(col + 32 + lane, z[d]);
   }
 }
 
 }  // namespace
 
+namespace {
 template <typename T>
-bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,
-                int* moves) {
+bool LaunchPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,
+                 int* moves) {
   Context& ctx = Ctx();
   PanelArgs<T> args;
   int ctas = 0;
@@ -624,7 +875,7 @@ bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info,
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kPanelCtas);
-    cfg.blockDim = dim3(kPanelThreads);
+    cfg.blockDim = dim3(kPanelThreads<T>);
     cfg.dynamicSmemBytes = kPanelSmemMax;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -647,7 +898,7 @@ bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info,
     return false;
   args.m = m;
   args.w = n;
-  args.lanes = sizeof(T) == 8 ? RefLanesDouble() : 2 * RefLanesDouble();
+  args.lanes = sizeof(RealOf<T>) == 8 ? RefLanesDouble() : 2 * RefLanesDouble();
   args.a = a;
   args.lda = lda;
   args.ipiv = ipiv;
@@ -675,13 +926,13 @@ bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info,
   LaunchFailed("getrf panel");
   return true;
 }
-template bool GetrfPanel<double>(int, int, double*, int, int*, int, int*, int, int*);
-template bool GetrfPanel<float>(int, int, float*, int, int*, int, int*, int, int*);
-
 template <typename T>
-void PanelSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const int* moves) {
+void LaunchSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const int* moves) {
   const int blocks = (left + kSwapCols - 1) / kSwapCols + (nc + kSwapCols - 1) / kSwapCols;
   if (blocks == 0) return;
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      PanelSwapTrsmKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SwapSmem<T>());
+  if (Failed(attr, "panel interchanges attributes")) return;
   SwapArgs<T> args;
   args.jb = jb;
   args.left = left;
@@ -691,11 +942,38 @@ void PanelSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const
   args.c0 = c0;
   args.l = a + j + static_cast<long long>(j) * lda;
   args.moves = moves;
-  PanelSwapTrsmKernel<T><<<blocks, kSwapThreads, 0, Ctx().stream>>>(args);
+  PanelSwapTrsmKernel<T><<<blocks, kSwapThreads, SwapSmem<T>(), Ctx().stream>>>(args);
   CountLaunch();
   LaunchFailed("panel interchanges");
 }
+}  // namespace
+
+template <typename T>
+bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,
+                int* moves) {
+  return LaunchPanel<T>(m, n, a, lda, ipiv, ipiv_add, info, info_base, moves);
+}
+template <typename R>
+bool ZGetrfPanel(int m, int n, R* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,
+                 int* moves) {
+  return LaunchPanel<Cx<R>>(m, n, reinterpret_cast<Cx<R>*>(a), lda, ipiv, ipiv_add, info,
+                            info_base, moves);
+}
+template <typename T>
+void PanelSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const int* moves) {
+  LaunchSwapTrsm<T>(j, jb, left, c0, nc, a, lda, moves);
+}
+template <typename R>
+void ZPanelSwapTrsm(int j, int jb, int left, int c0, int nc, R* a, int lda, const int* moves) {
+  LaunchSwapTrsm<Cx<R>>(j, jb, left, c0, nc, reinterpret_cast<Cx<R>*>(a), lda, moves);
+}
+template bool GetrfPanel<double>(int, int, double*, int, int*, int, int*, int, int*);
+template bool GetrfPanel<float>(int, int, float*, int, int*, int, int*, int, int*);
+template bool ZGetrfPanel<double>(int, int, double*, int, int*, int, int*, int, int*);
+template bool ZGetrfPanel<float>(int, int, float*, int, int*, int, int*, int, int*);
 template void PanelSwapTrsm<double>(int, int, int, int, int, double*, int, const int*);
 template void PanelSwapTrsm<float>(int, int, int, int, int, float*, int, const int*);
+template void ZPanelSwapTrsm<double>(int, int, int, int, int, double*, int, const int*);
+template void ZPanelSwapTrsm<float>(int, int, int, int, int, float*, int, const int*);
 
 }  // namespace hb

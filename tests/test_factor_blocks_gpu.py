@@ -1,0 +1,91 @@
+"""Cholesky blocks, triangular base solves and the complex LU panel against the
+oracle, bit for bit, at the edges of their tiles."""
+import numpy as np
+import pytest
+
+from tests.oracle_lib import rand, same_bits, first_diff
+
+pytestmark = pytest.mark.gpu
+REAL = {"d": np.float64, "s": np.float32}
+
+
+@pytest.mark.parametrize("p", ["d", "s"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("n", [1, 2, 7, 31, 32, 33, 40, 63, 64, 65, 150])
+@pytest.mark.parametrize("bad", [None, 0, "half", "last"])
+def test_potrf_blocks(hb, orc, p, uplo, n, bad):
+    rng = np.random.default_rng(n)
+    g = rand(rng, n, n)
+    a = (g @ g.T / n + np.eye(n)).astype(REAL[p])
+    if bad is not None:
+        i = {"half": n // 2, "last": n - 1}.get(bad, bad)
+        a[i, i] = np.nan if n % 2 else -1.0
+    a1, a2 = np.asfortranarray(a), np.asfortranarray(a.copy())
+    i1 = getattr(hb, f"{p}potrf")(uplo, n, a1, n)
+    i2 = getattr(orc, f"{p}potrf")(uplo, n, a2, n)
+    assert i1 == i2
+    assert same_bits(a1, a2), first_diff(a1, a2)
+
+
+@pytest.mark.parametrize("p", ["d", "s"])
+@pytest.mark.parametrize("side", ["L", "R"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("diag", ["N", "U"])
+@pytest.mark.parametrize("r", [31, 32, 33, 47, 63, 64, 65, 97])
+def test_trsm_bases(hb, orc, p, side, uplo, trans, diag, r):
+    rng = np.random.default_rng(r)
+    for other in (1, 16, 35):
+        m, n = (r, other) if side == "L" else (other, r)
+        a = rand(rng, r + 1, r, REAL[p]) / REAL[p](np.sqrt(r))
+        a[:r] += np.diag(np.full(r, 1.5)).astype(REAL[p])
+        a = np.asfortranarray(a)
+        b = rand(rng, m + 2, n, REAL[p])
+        x1, x2 = b.copy(order="F"), b.copy(order="F")
+        getattr(hb, f"{p}trsm")(side, uplo, trans, diag, m, n, 1.0, a, r + 1, x1, m + 2)
+        getattr(orc, f"{p}trsm")(side, uplo, trans, diag, m, n, REAL[p](1.0), a, r + 1, x2, m + 2)
+        assert same_bits(x1, x2), (other, first_diff(x1, x2))
+
+
+def check_zgetrf(hb, orc, p, a, recursive):
+    m, n = a.shape
+    a1, a2 = a.copy(order="F"), a.copy(order="F")
+    p1, p2 = np.zeros(min(m, n), np.int32), np.zeros(min(m, n), np.int32)
+    i1 = hb.zgetrf(p, m, n, a1, m, p1, recursive=recursive)
+    i2 = orc.zgetrf(m, n, a2, m, p2, recursive=recursive)
+    assert i1 == i2
+    assert np.array_equal(p1, p2), np.flatnonzero(p1 != p2)[:4]
+    r = REAL["d" if p == "z" else "s"]
+    b1, b2 = a1.T.view(r), a2.T.view(r)  # row by row: column by column of a
+    assert same_bits(b1, b2), first_diff(b1, b2)
+
+
+def crand(rng, p, m, n):
+    t = np.complex128 if p == "z" else np.complex64
+    return np.asfortranarray((rng.uniform(-1, 1, (m, n)) + 1j * rng.uniform(-1, 1, (m, n))).astype(t))
+
+
+@pytest.mark.parametrize("p", ["z", "c"])
+@pytest.mark.parametrize("m", [64, 130, 300, 1000])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 33, 50, 63, 64])
+def test_complex_panel_widths(hb, orc, p, m, n):
+    check_zgetrf(hb, orc, p, crand(np.random.default_rng(m + n), p, m, n), True)
+
+
+@pytest.mark.parametrize("p,m", [("z", 1152), ("z", 1153), ("z", 2304), ("z", 2320), ("c", 2700),
+                                 ("c", 5300)])
+def test_complex_panel_heights(hb, orc, p, m):
+    check_zgetrf(hb, orc, p, crand(np.random.default_rng(m), p, m, 64), False)
+
+
+@pytest.mark.parametrize("p", ["z", "c"])
+@pytest.mark.parametrize("m,n", [(200, 200), (65, 64), (300, 130), (130, 300), (600, 600)])
+@pytest.mark.parametrize("ties", [False, True])
+def test_complex_blocked(hb, orc, p, m, n, ties):
+    rng = np.random.default_rng(m + 2 * n)
+    a = crand(rng, p, m, n)
+    if ties:  # magnitudes from a few values, columns that become zero
+        a = np.asfortranarray((rng.integers(-1, 2, (m, n)) + 1j * rng.integers(-1, 2, (m, n)))
+                              .astype(a.dtype))
+        a[:, 5] = a[:, 3]
+    check_zgetrf(hb, orc, p, a, False)
