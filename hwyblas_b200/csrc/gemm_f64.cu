@@ -1094,12 +1094,13 @@ size_t DgemmSplitBytes(int m, int n, int k) {
 namespace {
 // Products for DgemmSmallKernel: those of at most a few million multiply-adds
 // or with a side below 32, and larger ones whose (tile, chunk) pairs still fit
-// the SMs about twice.
-bool SmallTakes(int m, int n, int k, bool small) {
+// the SMs about twice, but for k <= 64 where DgemmShortKKernel can take them
+// (512 x 512 x 64: 27 us a call there, 32 here).
+bool SmallTakes(int m, int n, int k, bool small, bool short_k) {
   const int nchunks = (k + 255) / 256, S = std::min(nchunks, kSmCluster);
   const long long ctas = static_cast<long long>((m + kSmT - 1) / kSmT) * ((n + kSmT - 1) / kSmT) * S;
   if ((nchunks + S - 1) / S > kSmMaxParts || ctas > (1LL << 30)) return false;
-  return small || ctas <= 2LL * Ctx().num_sms;
+  return small || (!short_k && ctas <= 2LL * Ctx().num_sms);
 }
 
 void DgemmSmall(int m, int n, int k, double alpha, View<double> a, View<double> b, double beta,
@@ -1145,7 +1146,9 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
            double beta, double* c, int ldc, Part part, Tri tri) {
   Context& ctx = Ctx();
   const bool small = static_cast<long long>(m) * n * k <= (1LL << 22) || m < 32 || n < 32;
-  if (tri == kTriNone && SmallTakes(m, n, k, small)) {
+  const bool short_k = k <= kSkK && tri == kTriNone && TmaReady(a.data, a.ld(), 8) &&
+                       TmaReady(b.data, b.ld(), 8) && TmaReady(c, ldc, 8);
+  if (tri == kTriNone && SmallTakes(m, n, k, small, short_k)) {
     DgemmSmall(m, n, k, alpha, a, b, beta, c, ldc, part);
     return;
   }
@@ -1182,8 +1185,7 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
       return;
     }
   }
-  if (k <= kSkK && tri == kTriNone && TmaReady(a.data, a.ld(), 8) &&
-      TmaReady(b.data, b.ld(), 8) && TmaReady(c, ldc, 8)) {
+  if (short_k) {
     static bool sk_configured = false;
     if (!sk_configured) {
       const auto set = [](const void* f) {
