@@ -126,9 +126,8 @@ enum WorkspaceSlot : int {
   kWsZFactorB = 31,    // aligned copy of the right-hand sides of its solve
   kWsResidual = 32,    // hwyblas_dresidual_dd partial sums
   kWsMixedInv = 33,    // mixed Cholesky: the inverse of a diagonal block
-  kWsTrsmBarrier = 34, // cooperative TRSM: its grid barrier counter
-  kWsLuMoves = 35,     // LU panels' lists of moved rows
-  kNumWorkspaceSlots = 36
+  kWsLuMoves = 34,     // LU panels' lists of moved rows
+  kNumWorkspaceSlots = 35
 };
 
 // Makes `to` wait for the work enqueued on `from` so far.

@@ -4,9 +4,11 @@
 // (argument-independent quick returns and alpha scaling).
 #include <algorithm>
 #include <cstdio>
+#include <utility>
 
 #include "device.cuh"
 #include "internal.h"
+#include "lane_solve.cuh"
 
 namespace hb {
 namespace {
@@ -167,76 +169,6 @@ __global__ void __launch_bounds__(256)
 // b_j -= x_q t(q, j) as fma(-x_q, t, b) for every solved q in that order, then
 // x_j = b_j * (1/t(j, j)). Element (row, col q) of X is
 // x[row * xs_row + q * xs_col].
-// The triangle of a base solve in shared memory, in solve order, and the
-// reciprocals of its diagonal (the CTA's threads share the loads).
-template <typename T>
-__device__ void LoadBaseTriangle(View<T> tri, int lower, int unit, int r, T (*st)[33],
-                                 T* sinv) {
-  for (int idx = threadIdx.x; idx < 32 * 32; idx += blockDim.x) {
-    const int s = idx / 32, u = idx % 32;
-    T v = T(0);
-    if (s < r && u < r) {
-      const int q = lower ? r - 1 - s : s, j = lower ? r - 1 - u : u;
-      // Only the triangle's solved-before part (s < u) and the diagonal are
-      // referenced.
-      if (s < u || (s == u && !unit)) v = tri.data[q * tri.rs + j * tri.cs];
-    }
-    st[s][u] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int s = threadIdx.x;
-    sinv[s] = (s < r && !unit) ? T(1) / st[s][s] : T(1);
-  }
-  __syncthreads();
-}
-
-// One row of X: loads through L2 only when kCg (rows written by other CTAs
-// in an earlier step of a cooperative launch).
-template <typename T, bool kCg>
-__device__ __forceinline__ T LoadX(const T* p) {
-  if constexpr (kCg) return __ldcg(p);
-  return *p;
-}
-template <typename T, bool kCg>
-__device__ __forceinline__ void StoreX(T* p, T v) {
-  if constexpr (kCg) __stcg(p, v);
-  else *p = v;
-}
-
-// N rows of X solved by a warp, lane s holding the element of step s (y): at
-// step q lane q's element is final, goes round by shuffles, and every later
-// lane takes its term, so each element's chain is over q ascending, as above,
-// but the chains of a row run side by side. st: the triangle, row stride ld. The
-// loop is rolled: unrolled for one thread a row, a launch fetched a thousand
-// instructions to run each once (32 x 32 base: 10 us; 4 to 6 us so), and lanes
-// along a column-major X read it coalesced.
-template <typename T, int N>
-__device__ __forceinline__ void LaneSolve(const T* st, int ld, T inv, int unit, int r, T (&y)[N]) {
-  const int lane = threadIdx.x % 32;
-#pragma unroll 2
-  for (int q = 0; q < r; ++q) {
-    const T l = st[q * ld + lane];
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const T yq = __shfl_sync(0xffffffffu, unit ? y[i] : y[i] * inv, q);
-      if (lane == q) y[i] = yq;
-      else if (lane > q) y[i] = fma(-yq, l, y[i]);
-    }
-  }
-}
-
-// One row of X in global memory against a 32 x 32 triangle (LoadBaseTriangle).
-template <typename T, bool kCg>
-__device__ __forceinline__ void WarpSolve(const T (*st)[33], const T* sinv, int lower, int unit,
-                                          int r, T* xr, long long xs_col) {
-  const int lane = threadIdx.x % 32;
-  T* at = xr + (lower ? r - 1 - lane : lane) * xs_col;
-  T y[1] = {lane < r ? LoadX<T, kCg>(at) : T(0)};
-  LaneSolve<T, 1>(&st[0][0], 33, sinv[lane], unit, r, y);
-  if (lane < r) StoreX<T, kCg>(at, y[0]);
-}
-
 // The recursion's node of at most 64 columns (src/trsm.cc:87-135: a base solve,
 // the product, a base solve) for many rows in one launch: a CTA takes kBaseRows
 // of them, two a warp. Rows that are contiguous in memory across each other
@@ -321,430 +253,196 @@ __global__ void __launch_bounds__(kBaseThreads)
   }
 }
 
-// Cooperative TRSM of a subtree of the recursion (at most kTcRows rows of
-// the triangle, at most TcOther right-hand sides): all of its base solves
-// and updates in one launch, in TrsmRec's order, with a bounded grid barrier
-// after each step; below that size the recursion is a chain of small
-// dependent launches. (n = 16384, one right-hand side: 22 -> 12 ms a
-// triangle; 64: 21 -> 12 ms.) A base step solves the `other` rows of X, one a
-// thread, with the 32 x 32 triangle in every CTA's shared memory; an update
-// step gives each thread C elements, each the reference's FMA chain over k
-// restarted every KC and merged in order (alpha -1, beta 1), as the GEMM
-// kernels compute it. X is read and written through L2 only: its rows
-// change owner between steps.
-constexpr int kTcRows = 512, kTcThreads = 256;
-// Right-hand sides of the cooperative path: up to 64 on the staged FMA
-// chains; in FP64 up to 1024, with the updates on the tensor pipe from 32.
-template <typename T>
-constexpr int TcOther() { return sizeof(T) == 8 ? 1024 : 64; }
+// A subtree of the TRSM recursion (65 to kTcRows rows of the triangle) in one
+// launch. Bound by latency: up to 16 dependent base solves with an update after
+// each, so all that does not depend on X is on the chip beforehand. A cluster of
+// kTcCtas CTAs takes kTcRhs right-hand sides (their columns are independent): its
+// CTAs hold the triangle's 16-row strips in turn (at most 155 KB each) in shared
+// memory, copied once while the first base is solved, and the next base triangle
+// is copied while one is solved. A base solve gives each warp a right-hand side,
+// an update each warp 16 x 8 tiles of the strips its CTA holds; every element's
+// chains, restarted every KC, and merges are the GEMM kernels'. Steps end with a cluster barrier, which is some 1.5 us less than a
+// grid barrier; X goes through L2. The right side is the left side of the
+// transposed system (each product's factors change places).
+// 512 rows: one right-hand side 168 us as a cooperative launch over the grid, 512
+// right-hand sides 140 us with 8 columns a CTA.
+constexpr int kTcRows = 512, kTcThreads = 256, kTcCtas = 8, kTcRhs = 64;
+constexpr int kTcStrip = 16, kTcStrips = kTcRows / kTcStrip / kTcCtas;  // a CTA's strips
+constexpr int kTcLd = kTcStrip + 4;  // conflict-free fragments
+constexpr int kTcMaxOther = 1024;    // wider systems fill the GPU as separate launches
 
 template <typename T>
-struct KcOf {
-  static constexpr int value = sizeof(T) == 8 ? 256 : 384;
-};
+constexpr int kTcKc = sizeof(T) == 8 ? 256 : 384;
 
 template <typename T>
-__device__ __forceinline__ View<T> SubView(View<T> v, long long i, long long j) {
-  v.data += i * v.rs + j * v.cs;
-  return v;
+constexpr int TcSmem() {
+  // The strips' columns of the CTA that has the most: 32-row blocks below a
+  // strip's own, for the strips 7, 15, 23, 31.
+  constexpr int cols = 32 * (3 + 7 + 11 + 15);
+  return static_cast<int>(sizeof(T)) * (cols * kTcLd + 2 * 32 * 33);
 }
 
 template <typename T>
-struct TrsmCoopArgs {
-  View<T> tri;
-  int left, lower, unit, r, other;
-  T* b;
-  long long ldb;
-  unsigned int* barrier;
-  int* timeout_flag;
+struct TrsmClusterArgs {
+  View<T> tri;  // T of T X = B
+  int lower, unit, r, other;
+  T* x;         // element (row, right-hand side) at row * xs + rhs * xr
+  long long xs, xr;
   const int* guard;
 };
 
-// C (mm x nn) -= A (mm x kk) B (kk x nn), kk <= 2 KC (all strided views;
-// element (i, j) of a view at data[i rs + j cs]). Each element's chain is
-// sequential, so its operands are staged first: a CTA takes blocks of
-// kTcRowsCta rows by kTcColsCta columns of C, copies those rows of A and
-// columns of B (all kk) into shared memory, then each thread runs its
-// elements' chains from there. The staging is wide and independent of the
-// chains, which then wait on no memory.
-constexpr int kTcRowsCta = 32, kTcColsCta = 16;
-constexpr int kTcKMax = 512;  // update depth within a subtree of kTcRows rows
-template <typename T>
-__device__ void CoopUpdate(int mm, int nn, int kk, View<T> a, View<T> bv, View<T> cv_,
-                           T* sa, T* sb) {
-  constexpr int KC = KcOf<T>::value;
-  const int rgroups = (mm + kTcRowsCta - 1) / kTcRowsCta;
-  const int items = rgroups * ((nn + kTcColsCta - 1) / kTcColsCta);
-  for (int item = blockIdx.x; item < items; item += gridDim.x) {
-    const int i0 = (item % rgroups) * kTcRowsCta, rows = min(kTcRowsCta, mm - i0);
-    const int j0 = (item / rgroups) * kTcColsCta, cols = min(kTcColsCta, nn - j0);
-    __syncthreads();  // the previous block's reads are done
-    // sa[q * 32 + il] = A(i0 + il, q); sb[q * 16 + jl] = B(q, j0 + jl)
-    for (int idx = threadIdx.x; idx < kk * kTcRowsCta; idx += blockDim.x) {
-      const int il = idx % kTcRowsCta, q = idx / kTcRowsCta;
-      sa[idx] = il < rows ? __ldcg(a.data + (i0 + il) * a.rs + q * a.cs) : T(0);
-    }
-    for (int idx = threadIdx.x; idx < kk * kTcColsCta; idx += blockDim.x) {
-      const int jl = idx % kTcColsCta, q = idx / kTcColsCta;
-      sb[idx] = jl < cols ? __ldcg(bv.data + q * bv.rs + (j0 + jl) * bv.cs) : T(0);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < rows * cols; e += blockDim.x) {
-      const int il = e % rows, jl = e / rows;
-      T* cij = const_cast<T*>(cv_.data) + (i0 + il) * cv_.rs + (j0 + jl) * cv_.cs;
-      T cv = __ldcg(cij);
-      for (int pc = 0; pc < kk; pc += KC) {
-        const int pe = min(kk, pc + KC);
-        T acc = T(0);
-        for (int q = pc; q < pe; ++q)
-          acc = fma(sa[q * kTcRowsCta + il], sb[q * kTcColsCta + jl], acc);
-        const T r = T(-1) * acc;
-        cv = r + cv;
-      }
-      __stcg(cij, cv);
-    }
-  }
+__device__ __forceinline__ void TcBarrier() {
+  asm volatile(
+      "barrier.cluster.arrive.release.aligned;\n\t"
+      "barrier.cluster.wait.acquire.aligned;" ::
+          : "memory");
 }
 
-// The same update on the FP64 tensor pipe for many right-hand sides: blocks
-// of 32 x 32 of C, the CTA's 8 warps one 16 x 8 tile each, k staged in
-// 64-deep chunks (A and B padded to 36 doubles a row, conflict-free
-// fragments) and each tile's m16n8k8 chain restarted every KC = 256 and
-// merged in order: every element's chain and merges are CoopUpdate's.
-constexpr int kTcDmmaB = 32, kTcDmmaKb = 64, kTcDmmaLd = kTcDmmaB + 4;
-__device__ void CoopUpdateDmma(int mm, int nn, int kk, View<double> a, View<double> bv,
-                               View<double> cv_, double* sa, double* sb) {
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int g = lane >> 2, t = lane & 3;
-  const int wr = warp % 2, wc = warp / 2;  // tile rows 16 wr, columns 8 wc
-  const int rgroups = (mm + kTcDmmaB - 1) / kTcDmmaB;
-  const int items = rgroups * ((nn + kTcDmmaB - 1) / kTcDmmaB);
-  for (int item = blockIdx.x; item < items; item += gridDim.x) {
-    const int i0 = (item % rgroups) * kTcDmmaB, j0 = (item / rgroups) * kTcDmmaB;
-    // This thread's four elements (the m16n8 accumulator layout) and their C.
-    double cv[4], acc[4] = {0.0, 0.0, 0.0, 0.0};
-    bool in[4];
-    double* cp[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = i0 + wr * 16 + g + (e >> 1) * 8, j = j0 + wc * 8 + 2 * t + (e & 1);
-      in[e] = i < mm && j < nn;
-      cp[e] = const_cast<double*>(cv_.data) + i * cv_.rs + j * cv_.cs;
-      cv[e] = in[e] ? __ldcg(cp[e]) : 0.0;
-    }
-    for (int k0 = 0; k0 < kk; k0 += kTcDmmaKb) {
-      __syncthreads();  // the previous chunk's fragments are read
-      // sa[q * 36 + il] = A(i0 + il, k0 + q); sb[q * 36 + jl] = B(k0 + q, j0 + jl)
-      for (int idx = threadIdx.x; idx < kTcDmmaKb * kTcDmmaB; idx += blockDim.x) {
-        const int l = idx % kTcDmmaB, q = idx / kTcDmmaB;
-        const bool kq = k0 + q < kk;
-        sa[q * kTcDmmaLd + l] = (kq && i0 + l < mm)
-                                    ? __ldcg(a.data + (i0 + l) * a.rs + (k0 + q) * a.cs)
-                                    : 0.0;
-        sb[q * kTcDmmaLd + l] = (kq && j0 + l < nn)
-                                    ? __ldcg(bv.data + (k0 + q) * bv.rs + (j0 + l) * bv.cs)
-                                    : 0.0;
-      }
-      __syncthreads();
-      const int steps = (min(kTcDmmaKb, kk - k0) + 7) / 8;
-      for (int ks = 0; ks < steps; ++ks) {
-        const double* pa = sa + (ks * 8 + t) * kTcDmmaLd + wr * 16 + g;
-        const double* pb = sb + (ks * 8 + t) * kTcDmmaLd + wc * 8 + g;
-        asm volatile(
-            "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
-            "{%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-            : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
-            : "d"(pa[0]), "d"(pa[8]), "d"(pa[4 * kTcDmmaLd]), "d"(pa[4 * kTcDmmaLd + 8]),
-              "d"(pb[0]), "d"(pb[4 * kTcDmmaLd]));
-      }
-      // End of a KC chunk (or of k): merge alpha * acc = -acc, restart.
-      if ((k0 + kTcDmmaKb) % 256 == 0 || k0 + kTcDmmaKb >= kk) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const double r = -1.0 * acc[e];
-          cv[e] = r + cv[e];
-          acc[e] = 0.0;
-        }
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (in[e]) __stcg(cp[e], cv[e]);
-  }
+template <typename T>
+__device__ __forceinline__ void TcCopy(T* dst, const T* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(SmemAddr(dst)), "l"(src),
+               "n"(sizeof(T))
+               : "memory");
 }
 
-// The update of a cooperative step: the tensor-pipe tiles in FP64 when the
-// right-hand sides fill them, else the staged FMA chains.
+// A 16 x 8 tile of C -= A X: a(row, q) at a[q * kTcLd + row] in shared memory, x and c
+// in global memory, kk terms; rows < mr and columns < nc exist.
 template <typename T>
-__device__ __forceinline__ void CoopStep(int mm, int nn, int kk, View<T> a, View<T> bv,
-                                         View<T> c, T* sa, T* sb) {
+__device__ __forceinline__ void TcTile(const T* a, const T* x, T* c, long long xs, long long xr,
+                                       int kk, int mr, int nc) {
+  const int lane = threadIdx.x % 32, g = lane >> 2, t = lane & 3;
+  T cv[4], acc[4] = {T(0), T(0), T(0), T(0)};
+  bool in[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = g + (e >> 1) * 8, j = 2 * t + (e & 1);
+    in[e] = i < mr && j < nc;
+    cv[e] = in[e] ? __ldcg(c + i * xs + j * xr) : T(0);
+  }
   if constexpr (sizeof(T) == 8) {
-    if (nn >= kTcDmmaB) {
-      CoopUpdateDmma(mm, nn, kk, a, bv, c, sa, sb);
-      return;
-    }
-  }
-  CoopUpdate(mm, nn, kk, a, bv, c, sa, sb);
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kTcThreads) TrsmCoopKernel(TrsmCoopArgs<T> p) {
-  if (p.guard != nullptr && *p.guard != 0) return;
-  __shared__ T st[32][33];
-  __shared__ T sinv[32];
-  extern __shared__ __align__(16) unsigned char tc_smem[];
-  T* sa = reinterpret_cast<T*>(tc_smem);   // kTcKMax x kTcRowsCta
-  T* sb = sa + kTcKMax * kTcRowsCta;       // kTcKMax x kTcColsCta
-  const auto col = [&](T* x, long long ld) {  // column-major, element (i, j) at x[i + j ld]
-    View<T> v;
-    v.data = x;
-    v.rs = 1;
-    v.cs = ld;
-    return v;
-  };
-  const auto row = [&](T* x, long long ld) {  // its transpose, element (i, j) at x[j + i ld]
-    View<T> v;
-    v.data = x;
-    v.rs = ld;
-    v.cs = 1;
-    return v;
-  };
-  // Which half TrsmRec solves first: t11 for left-lower and right-upper.
-  const bool first11 = (p.left != 0) == (p.lower != 0);
-  int s_off[8], s_r[8], s_ph[8];
-  int sp = 0;
-  s_off[0] = 0;
-  s_r[0] = p.r;
-  s_ph[0] = 0;
-  unsigned int gen = 0;
-  while (sp >= 0) {
-    const int off = s_off[sp], rr = s_r[sp];
-    if (rr <= 32) {
-      View<T> t = SubView(p.tri, off, off);
-      int lo = p.lower;
-      long long xs_row, xs_col;
-      T* xb;
-      if (p.left) {  // T X = B as X^T T^T = B^T: rows of X^T are B's columns
-        const long long rs = t.rs;
-        t.rs = t.cs;
-        t.cs = rs;
-        lo = !lo;
-        xs_row = p.ldb;
-        xs_col = 1;
-        xb = p.b + off;
-      } else {
-        xs_row = 1;
-        xs_col = p.ldb;
-        xb = p.b + static_cast<long long>(off) * p.ldb;
-      }
-      LoadBaseTriangle(t, lo, p.unit, rr, st, sinv);
-      // Rows go to the CTAs in turn, then to their warps.
-      for (long long row = blockIdx.x + static_cast<long long>(gridDim.x) * (threadIdx.x / 32);
-           row < p.other; row += static_cast<long long>(gridDim.x) * (blockDim.x / 32)) {
-        WarpSolve<T, true>(st, sinv, lo, p.unit, rr, xb + row * xs_row, xs_col);
-      }
-      --sp;
-      if (!GridBarrier(p.barrier, gridDim.x, ++gen, p.timeout_flag)) return;
-      continue;
-    }
-    const int r1 = max(32, (rr / 2) / 32 * 32), r2 = rr - r1;
-    const int ph = s_ph[sp]++;
-    if (ph == 2) {
-      --sp;
-      continue;
-    }
-    if (ph == 1) {
-      const View<T> toff =
-          p.lower ? SubView(p.tri, off + r1, off) : SubView(p.tri, off, off + r1);
-      if (p.left) {
-        T* b1 = p.b + off;
-        T* b2 = p.b + off + r1;
-        if (p.lower)
-          CoopStep(r2, p.other, r1, toff, col(b1, p.ldb), col(b2, p.ldb), sa, sb);
-        else
-          CoopStep(r1, p.other, r2, toff, col(b2, p.ldb), col(b1, p.ldb), sa, sb);
-      } else {
-        // X op(T) = B: the update C -= X_k toff, computed transposed,
-        // C^T -= toff^T X_k^T (each product's factors swap, which leaves
-        // every FMA's value unchanged), so that the few right-hand sides are
-        // the columns.
-        T* b1 = p.b + static_cast<long long>(off) * p.ldb;
-        T* b2 = p.b + static_cast<long long>(off + r1) * p.ldb;
-        View<T> tt = toff;
-        tt.rs = toff.cs;
-        tt.cs = toff.rs;
-        if (p.lower)
-          CoopStep(r1, p.other, r2, tt, row(b2, p.ldb), row(b1, p.ldb), sa, sb);
-        else
-          CoopStep(r2, p.other, r1, tt, row(b1, p.ldb), row(b2, p.ldb), sa, sb);
-      }
-      if (!GridBarrier(p.barrier, gridDim.x, ++gen, p.timeout_flag)) return;
-    }
-    // ph 0: the first half; ph 1: the second.
-    const bool take11 = (ph == 0) == first11;
-    ++sp;
-    s_off[sp] = take11 ? off : off + r1;
-    s_r[sp] = take11 ? r1 : r2;
-    s_ph[sp] = 0;
-  }
-}
-
-template <typename T>
-bool TrsmCoop(bool left, View<T> tri, bool lower, bool unit, int r, int other, T* b,
-              int ldb) {
-  Context& ctx = Ctx();
-  static int per_sm[2] = {-1, -1};
-  int& occ = per_sm[sizeof(T) == 8 ? 0 : 1];
-  constexpr int kSmem = static_cast<int>(sizeof(T)) * kTcKMax * (kTcRowsCta + kTcColsCta);
-  if (occ < 0) {
-    int v = 0;
-    if (cudaFuncSetAttribute(reinterpret_cast<const void*>(TrsmCoopKernel<T>),
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, TrsmCoopKernel<T>, kTcThreads,
-                                                      kSmem) != cudaSuccess) {
-      cudaGetLastError();
-      v = 0;
-    }
-    occ = v;
-  }
-  if (occ <= 0) return false;
-  // One CTA per block of the largest update, at most one an SM (fewer CTAs
-  // make cheaper barriers).
-  const int blocks =
-      (sizeof(T) == 8 && other >= kTcDmmaB)
-          ? ((r - 32 + kTcDmmaB - 1) / kTcDmmaB) * ((other + kTcDmmaB - 1) / kTcDmmaB)
-          : ((r - 32 + kTcRowsCta - 1) / kTcRowsCta) * ((other + kTcColsCta - 1) / kTcColsCta);
-  const int grid = std::max(1, std::min(blocks, std::min(ctx.num_sms, ctx.num_sms * occ)));
-  unsigned int* bar = static_cast<unsigned int*>(Workspace(kWsTrsmBarrier, 256));
-  if (bar == nullptr) return false;
-  cudaMemsetAsync(bar, 0, sizeof(unsigned int), ctx.stream);
-  TrsmCoopArgs<T> a;
-  a.tri = tri;
-  a.left = left ? 1 : 0;
-  a.lower = lower ? 1 : 0;
-  a.unit = unit ? 1 : 0;
-  a.r = r;
-  a.other = other;
-  a.b = b;
-  a.ldb = ldb;
-  a.barrier = bar;
-  a.timeout_flag = ctx.wait_flag;
-  a.guard = ctx.guard;
-  void* args[] = {&a};
-  if (cudaLaunchCooperativeKernel(reinterpret_cast<void*>(TrsmCoopKernel<T>), grid,
-                                  kTcThreads, args, kSmem, ctx.stream) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  CountLaunch();
-  LaunchFailed("trsm cooperative");
-  return true;
-}
-
-// Left-side FP64 TRSM subtree (at most kTcRows rows) with many right-hand
-// sides: the columns of X are independent, so each CTA owns kTsCols of them
-// and walks the whole recursion for those columns alone, with block
-// barriers only (no grid barrier, no cooperative launch). Base solves are
-// the base kernel's code (one thread a column); an update C -= A X of the
-// CTA's columns gives each warp 16-row strips of C and runs the element's
-// m16n8k8 chain over k, restarted every KC = 256 and merged in order (alpha
-// -1, beta 1): every element's FMA chain and merges are those of the
-// cooperative kernel's updates, so X comes out the same.
-constexpr int kTsCols = 8;       // right-hand sides a CTA owns: one n8 fragment
-constexpr int kTsMinOther = 256;  // the column-owned path from this many
-// ... and from this many rows: a shallower subtree is a short chain of
-// launches already, and the LU's 64-row panel solves over thousands of
-// columns measured slower column-owned (dgesv n = 16384 251 -> 278 ms).
-constexpr int kTsMinRows = 256;
-
-// C (mm x w) -= A (mm x kk) X (kk x w); X and C column-major with leading
-// dimension ld, A a strided view. Fragments come from L2 four k8 steps at a
-// time (zero past kk, mm and w: fma(0, 0, acc) = acc for a chain started at
-// +0).
-__device__ void ColsUpdate(int mm, int kk, View<double> a, const double* x, double* c,
-                           long long ld, int w) {
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int g = lane >> 2, t = lane & 3;
-  const int warps = blockDim.x / 32;
-  for (int i0 = warp * 16; i0 < mm; i0 += warps * 16) {
-    double acc[4] = {0.0, 0.0, 0.0, 0.0}, cv[4];
-    bool in[4];
+    constexpr int kSteps = 8;  // k8 steps whose X is in flight together
+    for (int k0 = 0; k0 < kk; k0 += 8 * kSteps) {
+      T fb[kSteps][2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = i0 + g + (e >> 1) * 8, j = 2 * t + (e & 1);
-      in[e] = i < mm && j < w;
-      cv[e] = in[e] ? __ldcg(c + i + j * ld) : 0.0;
-    }
-    const int ra = i0 + g, rb = i0 + g + 8;
-    for (int k0 = 0; k0 < kk; k0 += 32) {
-      double fa[4][4], fb[4][2];
+      for (int s = 0; s < kSteps; ++s)
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const int q0 = k0 + 8 * s + t, q1 = q0 + 4;
-        fa[s][0] = (ra < mm && q0 < kk) ? __ldcg(a.data + ra * a.rs + q0 * a.cs) : 0.0;
-        fa[s][1] = (rb < mm && q0 < kk) ? __ldcg(a.data + rb * a.rs + q0 * a.cs) : 0.0;
-        fa[s][2] = (ra < mm && q1 < kk) ? __ldcg(a.data + ra * a.rs + q1 * a.cs) : 0.0;
-        fa[s][3] = (rb < mm && q1 < kk) ? __ldcg(a.data + rb * a.rs + q1 * a.cs) : 0.0;
-        fb[s][0] = (g < w && q0 < kk) ? __ldcg(x + q0 + g * ld) : 0.0;
-        fb[s][1] = (g < w && q1 < kk) ? __ldcg(x + q1 + g * ld) : 0.0;
-      }
+        for (int h = 0; h < 2; ++h) {
+          const int q = k0 + 8 * s + 4 * h + t;
+          fb[s][h] = q < kk && g < nc ? __ldcg(x + q * xs + g * xr) : 0.0;
+        }
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
+      for (int s = 0; s < kSteps; ++s) {
+        if (k0 + 8 * s >= kk) break;
+        const int q = k0 + 8 * s + t;
+        const T* fa = a + q * kTcLd + g;
+        // Past kk: -0 times +0, which leaves every sum as it is.
+        const bool i0 = q < kk, i1 = q + 4 < kk;
+        const T a0 = i0 ? fa[0] : -0.0, a1 = i0 ? fa[8] : -0.0;
+        const T a2 = i1 ? fa[4 * kTcLd] : -0.0, a3 = i1 ? fa[4 * kTcLd + 8] : -0.0;
         asm volatile(
             "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
             "{%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
             : "+d"(acc[0]), "+d"(acc[1]), "+d"(acc[2]), "+d"(acc[3])
-            : "d"(fa[s][0]), "d"(fa[s][1]), "d"(fa[s][2]), "d"(fa[s][3]), "d"(fb[s][0]),
-              "d"(fb[s][1]));
-      }
-      // End of a KC chunk (or of k): merge alpha * acc = -acc, restart.
-      if ((k0 + 32) % 256 == 0 || k0 + 32 >= kk) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const double r = -1.0 * acc[e];
-          cv[e] = r + cv[e];
-          acc[e] = 0.0;
-        }
+            : "d"(a0), "d"(a1), "d"(a2), "d"(a3), "d"(fb[s][0]), "d"(fb[s][1]));
       }
     }
+  } else {
+    constexpr int kSteps = 16;
+    for (int k0 = 0; k0 < kk; k0 += kSteps) {
+      T fb[kSteps][2];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = i0 + g + (e >> 1) * 8, j = 2 * t + (e & 1);
-      if (in[e]) __stcg(c + i + j * ld, cv[e]);
+      for (int s = 0; s < kSteps; ++s)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          fb[s][h] = k0 + s < kk && 2 * t + h < nc ? __ldcg(x + (k0 + s) * xs + (2 * t + h) * xr)
+                                                   : T(0);
+#pragma unroll
+      for (int s = 0; s < kSteps; ++s) {
+        if (k0 + s >= kk) break;
+        const T a0 = a[(k0 + s) * kTcLd + g], a1 = a[(k0 + s) * kTcLd + g + 8];
+        acc[0] = fma(a0, fb[s][0], acc[0]);
+        acc[1] = fma(a0, fb[s][1], acc[1]);
+        acc[2] = fma(a1, fb[s][0], acc[2]);
+        acc[3] = fma(a1, fb[s][1], acc[3]);
+      }
     }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int i = g + (e >> 1) * 8, j = 2 * t + (e & 1);
+    if (in[e]) __stcg(c + i * xs + j * xr, T(-1) * acc[e] + cv[e]);
   }
 }
 
-__global__ void __launch_bounds__(kTcThreads) TrsmColsKernel(TrsmCoopArgs<double> p) {
+template <typename T>
+__global__ void __launch_bounds__(kTcThreads) TrsmClusterKernel(TrsmClusterArgs<T> p) {
   if (p.guard != nullptr && *p.guard != 0) return;
-  __shared__ double st[32][33];
-  __shared__ double sinv[32];
-  const int j0 = blockIdx.x * kTsCols;
-  const int w = min(kTsCols, p.other - j0);
-  if (w <= 0) return;
-  double* xb = p.b + static_cast<long long>(j0) * p.ldb;  // this CTA's columns
-  // Which half TrsmRec solves first: t11 for left-lower.
-  const bool first11 = p.lower != 0;
+  extern __shared__ __align__(16) unsigned char tc_smem[];
+  T* tri[2] = {reinterpret_cast<T*>(tc_smem), reinterpret_cast<T*>(tc_smem) + 32 * 33};
+  T* strips = tri[1] + 32 * 33;
+  const int rank = blockIdx.x % kTcCtas, j0 = blockIdx.x / kTcCtas * kTcRhs;
+  const int nrhs = min(kTcRhs, p.other - j0);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  T* x = p.x + j0 * p.xr;
+  const bool rows_fast = p.tri.rs == 1;
+  const int blocks = (p.r + 31) / 32;
+  // Base triangle number t (in the order they are solved), in solve order:
+  // st[s][u] = T(row u, column s), s <= u.
+  const auto load_base = [&](int t) {
+    if (t >= blocks || rank >= nrhs) return;
+    const int off = 32 * (p.lower ? t : blocks - 1 - t), n = min(32, p.r - off);
+    T* st = tri[t & 1];
+    for (int idx = threadIdx.x; idx < 32 * 32; idx += kTcThreads) {
+      const int s = rows_fast ? idx / 32 : idx % 32, u = rows_fast ? idx % 32 : idx / 32;
+      if (s > u || u >= n || (s == u && p.unit)) continue;
+      const int row = off + (p.lower ? u : n - 1 - u), q = off + (p.lower ? s : n - 1 - s);
+      TcCopy(st + s * 33 + u, p.tri.data + row * p.tri.rs + q * p.tri.cs);
+    }
+  };
+  load_base(0);
+  CpAsyncCommit();
+  // This CTA's strips: number rank + kTcCtas i, its columns solved before its block.
+  int at[kTcStrips], first[kTcStrips];
+  int used = 0;
+#pragma unroll
+  for (int i = 0; i < kTcStrips; ++i) {
+    const int row0 = (rank + kTcCtas * i) * kTcStrip, blk = row0 / 32;
+    const int q0 = p.lower ? 0 : 32 * (blk + 1);
+    const int n = row0 < p.r ? max(0, (p.lower ? 32 * blk : p.r) - q0) : 0;
+    at[i] = used;
+    first[i] = q0;
+    T* dst = strips + used;
+    used += n * kTcLd;
+    for (int idx = threadIdx.x; idx < n * kTcStrip; idx += kTcThreads) {
+      const int il = rows_fast ? idx % kTcStrip : idx / n, q = rows_fast ? idx / kTcStrip : idx % n;
+      if (row0 + il < p.r)
+        TcCopy(dst + q * kTcLd + il, p.tri.data + (row0 + il) * p.tri.rs + (q0 + q) * p.tri.cs);
+    }
+  }
+  CpAsyncCommit();
   int s_off[8], s_r[8], s_ph[8];
-  int sp = 0;
+  int sp = 0, base = 0;
   s_off[0] = 0;
   s_r[0] = p.r;
   s_ph[0] = 0;
   while (sp >= 0) {
     const int off = s_off[sp], rr = s_r[sp];
     if (rr <= 32) {
-      // T X = B as X^T T^T = B^T: rows of X^T are B's columns.
-      View<double> t = SubView(p.tri, off, off);
-      const long long rs = t.rs;
-      t.rs = t.cs;
-      t.cs = rs;
-      const int lo = !p.lower;
-      LoadBaseTriangle(t, lo, p.unit, rr, st, sinv);
-      for (int j = threadIdx.x / 32; j < w; j += blockDim.x / 32) {
-        WarpSolve<double, true>(st, sinv, lo, p.unit, rr, xb + off + j * p.ldb, 1);
-      }
-      --sp;
+      if (base == 0) CpAsyncWait<1>();
+      else CpAsyncWait<0>();
       __syncthreads();
+      const T* st = tri[base & 1];
+      load_base(++base);
+      CpAsyncCommit();
+      for (int j = rank + kTcCtas * warp; j < nrhs; j += kTcCtas * (kTcThreads / 32)) {
+        T* e = x + (off + (p.lower ? lane : rr - 1 - lane)) * p.xs + j * p.xr;
+        T y[1] = {lane < rr ? __ldcg(e) : T(0)};
+        const T inv = lane < rr && !p.unit ? T(1) / st[lane * 33 + lane] : T(1);
+        LaneSolve<T, 1>(st, 33, inv, p.unit, rr, y);
+        if (lane < rr) __stcg(e, y[0]);
+      }
+      TcBarrier();
+      --sp;
       continue;
     }
     const int r1 = max(32, (rr / 2) / 32 * 32), r2 = rr - r1;
@@ -754,38 +452,77 @@ __global__ void __launch_bounds__(kTcThreads) TrsmColsKernel(TrsmCoopArgs<double
       continue;
     }
     if (ph == 1) {
-      if (p.lower)
-        ColsUpdate(r2, r1, SubView(p.tri, off + r1, off), xb + off, xb + off + r1, p.ldb, w);
-      else
-        ColsUpdate(r1, r2, SubView(p.tri, off, off + r1), xb + off + r1, xb + off, p.ldb, w);
-      __syncthreads();
+      if (base == 1) {  // the strips have arrived
+        CpAsyncWait<0>();
+        __syncthreads();
+      }
+      // The half just solved, columns [q0, q0 + kk), on the rows of the other.
+      const int c0 = p.lower ? off + r1 : off, c1 = p.lower ? off + rr : off + r1;
+      const int q0 = p.lower ? off : off + r1, kk = p.lower ? r1 : r2;
+      const int tiles = (nrhs + 7) / 8;
+      int unit = 0;
+#pragma unroll
+      for (int i = 0; i < kTcStrips; ++i) {
+        const int row0 = (rank + kTcCtas * i) * kTcStrip;
+        if (row0 < c0 || row0 >= c1) continue;
+        for (int ct = 0; ct < tiles; ++ct, ++unit) {
+          if (unit % (kTcThreads / 32) != warp) continue;
+          T* xc = x + 8 * ct * p.xr;
+          for (int k0 = 0; k0 < kk; k0 += kTcKc<T>)
+            TcTile<T>(strips + at[i] + (q0 + k0 - first[i]) * kTcLd, xc + (q0 + k0) * p.xs,
+                      xc + row0 * p.xs, p.xs, p.xr, min(kTcKc<T>, kk - k0), c1 - row0,
+                      nrhs - 8 * ct);
+        }
+      }
+      TcBarrier();
     }
-    // ph 0: the first half; ph 1: the second.
-    const bool take11 = (ph == 0) == first11;
+    // ph 0: the half solved first (the leading one of a lower triangle).
+    const bool leading = (ph == 0) == (p.lower != 0);
     ++sp;
-    s_off[sp] = take11 ? off : off + r1;
-    s_r[sp] = take11 ? r1 : r2;
+    s_off[sp] = leading ? off : off + r1;
+    s_r[sp] = leading ? r1 : r2;
     s_ph[sp] = 0;
   }
 }
 
-bool TrsmCols(View<double> tri, bool lower, bool unit, int r, int other, double* b, int ldb) {
+template <typename T>
+bool TrsmCluster(bool left, View<T> tri, bool lower, bool unit, int r, int other, T* b, int ldb) {
   Context& ctx = Ctx();
-  TrsmCoopArgs<double> a;
+  static const bool ready = [] {
+    const bool ok =
+        cudaFuncSetAttribute(reinterpret_cast<const void*>(TrsmClusterKernel<T>),
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             TcSmem<T>()) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+  }();
+  if (!ready) return false;
+  TrsmClusterArgs<T> a;
   a.tri = tri;
-  a.left = 1;
-  a.lower = lower ? 1 : 0;
+  if (!left) std::swap(a.tri.rs, a.tri.cs);
+  a.lower = left == lower ? 1 : 0;
   a.unit = unit ? 1 : 0;
   a.r = r;
   a.other = other;
-  a.b = b;
-  a.ldb = ldb;
-  a.barrier = nullptr;
-  a.timeout_flag = ctx.wait_flag;
+  a.x = b;
+  a.xs = left ? 1 : ldb;
+  a.xr = left ? ldb : 1;
   a.guard = ctx.guard;
-  TrsmColsKernel<<<(other + kTsCols - 1) / kTsCols, kTcThreads, 0, ctx.stream>>>(a);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((other + kTcRhs - 1) / kTcRhs * kTcCtas);
+  cfg.blockDim = dim3(kTcThreads);
+  cfg.dynamicSmemBytes = TcSmem<T>();
+  cfg.stream = ctx.stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = kTcCtas;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  Failed(cudaLaunchKernelEx(&cfg, TrsmClusterKernel<T>, a), "trsm subtree");
   CountLaunch();
-  return !LaunchFailed("trsm column-owned");
+  return !LaunchFailed("trsm subtree");
 }
 
 template <typename T>
@@ -810,14 +547,8 @@ void TrsmRec(bool left, View<T> tri, bool lower, bool unit, int r, int other,
     TrsmSolve<T>(left, tri, lower, unit, r, other, b, ldb);
     return;
   }
-  if constexpr (sizeof(T) == 8) {
-    if (left && r <= kTcRows && r >= kTsMinRows && other >= kTsMinOther) {
-      TrsmCols(tri, lower, unit, r, other, b, ldb);
-      return;
-    }
-  }
-  if (r <= kTcRows && other <= TcOther<T>() &&
-      TrsmCoop<T>(left, tri, lower, unit, r, other, b, ldb))
+  if (r <= kTcRows && other <= kTcMaxOther &&
+      TrsmCluster<T>(left, tri, lower, unit, r, other, b, ldb))
     return;
   const int r1 = std::max(32, (r / 2) / 32 * 32);
   const int r2 = r - r1;

@@ -62,6 +62,8 @@ struct ElemOf<Cx<R>> {
 };
 template <typename T>
 using RealOf = typename ElemOf<T>::Real;
+template <typename T>
+constexpr bool kWideKey = sizeof(RealOf<T>) == 8;
 
 // The leaf's element operations (src/lapack/factor_kernels.cc:33-183).
 template <typename T>
@@ -179,39 +181,9 @@ struct PanelArgs {
   int* timeout_flag;
 };
 
-// Order of the pivot search: larger |x|, NaN below everything (0).
-__device__ __forceinline__ unsigned long long PivotKey(double x) {
-  const unsigned long long v = __double_as_longlong(x) & 0x7fffffffffffffffull;
-  return v > 0x7ff0000000000000ull ? 0ull : v + 1;
-}
-__device__ __forceinline__ unsigned long long PivotKey(float x) {
-  const unsigned v = __float_as_uint(x) & 0x7fffffffu;
-  return v > 0x7f800000u ? 0ull : static_cast<unsigned long long>(v) + 1;
-}
-
 template <typename R>
 __device__ __forceinline__ unsigned long long PivotKey(Cx<R> x) {
   return PivotKey(ZMag(x.re, x.im));
-}
-
-// The lane with the warp's largest key, the one with the smallest position if
-// several hold it. The keys' high words nearly always decide.
-template <typename T>
-__device__ __forceinline__ int WarpBest(unsigned long long key, int pos) {
-  const unsigned lo = static_cast<unsigned>(key), hi = static_cast<unsigned>(key >> 32);
-  constexpr bool kWide = sizeof(RealOf<T>) == 8;
-  const unsigned word = kWide ? hi : lo;
-  const unsigned largest = __reduce_max_sync(0xffffffffu, word);
-  unsigned top = __ballot_sync(0xffffffffu, word == largest);
-  if (top & (top - 1)) {
-    const bool in = (top >> (threadIdx.x % 32)) & 1;
-    const unsigned second = kWide && in ? lo : 0u;
-    const unsigned most = __reduce_max_sync(0xffffffffu, second);  // by every lane
-    const bool in2 = in && second == most;
-    const int first = __reduce_min_sync(0xffffffffu, in2 ? pos : 0x7fffffff);
-    top = __ballot_sync(0xffffffffu, in2 && pos == first);
-  }
-  return __ffs(top) - 1;
 }
 
 __device__ __forceinline__ uint32_t MapRank(uint32_t addr, int rank) {
@@ -536,14 +508,14 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
         unsigned long long key = valid && pos >= jc ? PivotKey(x[0]) : 0ull;
         if (valid && pos == jc && key == 0)
           key = sizeof(RealOf<T>) == 8 ? ~0ull : 0xffffffffull;
-        const int wbest = WarpBest<T>(key, pos);
+        const int wbest = WarpBest<kWideKey<T>>(key, pos);
         if (lane == wbest) {
           s_wkey[par][warp] = key;
           s_wpos[par][warp] = pos;
         }
         __syncthreads();
         // The block's, found by every warp; the warp that holds the row sends it.
-        const int cbest = WarpBest<T>(lane < nwarps ? s_wkey[par][lane] : 0ull,
+        const int cbest = WarpBest<kWideKey<T>>(lane < nwarps ? s_wkey[par][lane] : 0ull,
                                       lane < nwarps ? s_wpos[par][lane] : 0x7fffffff);
         if (warp == cbest) {
           if (lane == wbest) {
@@ -585,7 +557,7 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
             }
           }
           const PanelSlot<T>* slot = slots + par * kPanelCtas + lane;
-          from = WarpBest<T>(lane < P ? slot->key : 0ull, lane < P ? slot->pos : 0x7fffffff);
+          from = WarpBest<kWideKey<T>>(lane < P ? slot->key : 0ull, lane < P ? slot->pos : 0x7fffffff);
           at = par * kPanelCtas + (from & (kPanelCtas - 1));
         } else {
           __syncthreads();

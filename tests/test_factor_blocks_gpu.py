@@ -89,3 +89,24 @@ def test_complex_blocked(hb, orc, p, m, n, ties):
                               .astype(a.dtype))
         a[:, 5] = a[:, 3]
     check_zgetrf(hb, orc, p, a, False)
+
+
+@pytest.mark.parametrize("p", ["d", "s"])
+@pytest.mark.parametrize("side", ["L", "R"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("r,other", [(65, 1), (96, 9), (288, 64), (450, 3), (500, 70), (511, 8),
+                                     (512, 130), (700, 17)])
+def test_trsm_subtrees(hb, orc, p, side, uplo, trans, r, other):
+    """Subtrees in one launch: partial blocks, more right-hand sides than a
+    cluster takes, updates deeper than a KC chunk (upper, r = 500 and 511)."""
+    rng = np.random.default_rng(r + other)
+    m, n = (r, other) if side == "L" else (other, r)
+    a = rand(rng, r, r, REAL[p]) / REAL[p](np.sqrt(r))
+    a = np.asfortranarray(a + np.diag(np.full(r, 1.5)).astype(REAL[p]))
+    b = rand(rng, m + 1, n, REAL[p])
+    for diag in "NU":
+        x1, x2 = b.copy(order="F"), b.copy(order="F")
+        getattr(hb, f"{p}trsm")(side, uplo, trans, diag, m, n, 1.0, a, r, x1, m + 1)
+        getattr(orc, f"{p}trsm")(side, uplo, trans, diag, m, n, REAL[p](1.0), a, r, x2, m + 1)
+        assert same_bits(x1, x2), (diag, first_diff(x1, x2))
