@@ -27,6 +27,7 @@
 #include "../../include/hwyblas_b200.h"
 #include "device.cuh"
 #include "internal.h"
+#include "lane_solve.cuh"
 #include "ref_order.cuh"
 
 namespace hb {
@@ -94,11 +95,12 @@ __device__ void CtaGemm(int m, int n, int k, T alpha, Mat<T> a, Mat<T> b, T beta
 // mma.sync.m16n8k8.f64 per k8 step. The MMA accumulates its 8 products in
 // ascending k as a chain of correctly rounded FMAs starting from the
 // accumulator, so chaining the MMAs over k and restarting every KC = 256
-// gives every element the reference's chain; zero padding past k adds +0.
-// Each 256-deep chunk is merged into C exactly as CtaGemm merges it. Operand k-blocks of 32 are staged in shared memory with
-// rows padded to a stride of 8 (mod 32) words, which makes every fragment
-// load conflict free; the next block is fetched into registers while the
-// current one is multiplied.
+// gives every element the reference's chain; the padding past k (-0 times +0)
+// leaves every sum as it is. Each 256-deep chunk is merged into C exactly as
+// CtaGemm merges it. Operand k-blocks of 32 are staged in shared memory with
+// rows padded to a stride of 8 (mod 32) words, which makes every fragment load
+// conflict free; the next block is fetched into registers while the current one
+// is multiplied.
 constexpr int kDmmaKb = 32;
 
 __device__ __forceinline__ void BatchDmma(double (&d)[4], double a0, double a1, double a2,
@@ -127,6 +129,8 @@ __device__ void CtaGemmDmma(int m, int n, int k, double alpha, Mat<double> a, Ma
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int wm = warp % WM, wn = warp / WM;
   const int g = lane >> 2, t = lane & 3;
+  // A warp issues only the MMAs whose 16 x 8 block holds elements of C: at the
+  // ragged edge the other warps have the tensor pipe to themselves.
   // Operand loads: along the contiguous index of each operand.
   const bool a_rows = a.rs == 1;  // A(i, q) contiguous in i
   const bool b_rows = b.rs == 1;  // B(q, j) contiguous in q
@@ -140,7 +144,7 @@ __device__ void CtaGemmDmma(int m, int n, int k, double alpha, Mat<double> a, Ma
           const int idx = threadIdx.x + l * Cfg::kThreads;
           const int i = a_rows ? idx % TM : idx / kDmmaKb;
           const int q = a_rows ? idx / TM : idx % kDmmaKb;
-          ra[l] = (m0 + i < m && kb0 + q < k) ? a(m0 + i, kb0 + q) : 0.0;
+          ra[l] = (m0 + i < m && kb0 + q < k) ? a(m0 + i, kb0 + q) : -0.0;
         }
 #pragma unroll
         for (int l = 0; l < Cfg::kLoadB; ++l) {
@@ -178,12 +182,14 @@ __device__ void CtaGemmDmma(int m, int n, int k, double alpha, Mat<double> a, Ma
           stash();
           __syncthreads();
           if (kb0 + kDmmaKb < k) fetch(kb0 + kDmmaKb);
-          const int steps = (min(pe, kb0 + kDmmaKb) - kb0 + 7) / 8;
+          const int steps =
+              m0 + wm * 16 < m ? (min(pe, kb0 + kDmmaKb) - kb0 + 7) / 8 : 0;
           for (int ks = 0; ks < steps; ++ks) {
             const double* pa = sA + (ks * 8 + t) * SA + wm * 16 + g;
             const double a0 = pa[0], a1 = pa[8], a2 = pa[4 * SA], a3 = pa[4 * SA + 8];
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb) {
+              if (n0 + (wn * NB + nb) * 8 >= n) break;
               const double* pb = sB + (ks * 8 + t) * SB + wn * 8 * NB + nb * 8 + g;
               BatchDmma(acc[nb], a0, a1, a2, a3, pb[0], pb[4 * SB]);
             }
@@ -348,7 +354,7 @@ struct RegGemm {
   T* sB;
   __device__ void operator()(int m, int n, int k, T alpha, Mat<T> a, Mat<T> b, T beta,
                              Mat<T> c) const {
-    if (m < 16 || n < 16)
+    if (m < 16 || n < 4)
       CtaGemm<T>(m, n, k, alpha, a, b, beta, c);
     else
       CtaGemmReg<T, Threads>(m, n, k, alpha, a, b, beta, c, sA, sB);
@@ -361,7 +367,7 @@ struct TileGemm {
   double* sB;
   __device__ void operator()(int m, int n, int k, double alpha, Mat<double> a,
                              Mat<double> b, double beta, Mat<double> c) const {
-    if (m < 16 || n < 16)
+    if (m < 16 || n < 4)
       CtaGemm<double>(m, n, k, alpha, a, b, beta, c);
     else
       CtaGemmDmma<WM, WN, NB>(m, n, k, alpha, a, b, beta, c, sA, sB);
@@ -422,6 +428,21 @@ __device__ void CtaTrsmBase(Mat<T> t, bool lower, bool unit, int r, int other, T
     sinv[s] = (s < r && !unit) ? T(1) / st[s][s] : T(1);
   }
   __syncthreads();
+  if (2 * other <= static_cast<int>(blockDim.x)) {
+    // Few rows: two a warp, a lane an element, instead of a thread a row.
+    const int lane = threadIdx.x % 32;
+    const long long at = (lower ? r - 1 - lane : lane) * xs_col;
+    for (int row = threadIdx.x / 32 * 2; row < other; row += blockDim.x / 16) {
+      T* xr = x + row * xs_row + at;
+      const bool in0 = lane < r, in1 = in0 && row + 1 < other;
+      T y[2] = {in0 ? xr[0] : T(0), in1 ? xr[xs_row] : T(0)};
+      LaneSolve<T, 2>(&st[0][0], 33, sinv[lane], unit, r, y);
+      if (in0) xr[0] = y[0];
+      if (in1) xr[xs_row] = y[1];
+    }
+    __syncthreads();
+    return;
+  }
   for (int row = threadIdx.x; row < other; row += blockDim.x) {
     T* xr = x + row * xs_row;
     T y[32];
@@ -566,7 +587,8 @@ __device__ void CtaTrsmRight(Mat<T> tri, bool lower, bool unit, int r, int other
   }
 }
 
-// Shared scratch of the per-CTA LU.
+// Shared scratch of the per-CTA LU and solves.
+constexpr int kLeafW = 16, kMovesMax = 2 * kLeafW, kPermMax = 1024;
 template <typename T>
 struct LuShared {
   T st[32][33];
@@ -575,16 +597,24 @@ struct LuShared {
   int wi[32];
   int piv;
   T pivot;
+  // The register leaf: each warp's candidate by step parity, the pivot row from
+  // its column on and the reciprocal of its pivot.
+  unsigned long long wkey[2][8];
+  int wpos[2][8];
+  T row[kLeafW];
+  T rinv;
+  // The rows that a leaf's interchanges moved: new and old position.
+  int moves, dst[kMovesMax], src[kMovesMax];
+  int perm[kPermMax];  // a solve's row order
 };
 
-// LU leaf (min(m, n) <= 16) on an m x n block: partial pivoting with the
+// LU leaf of an m x w block (w <= 16, m >= w): partial pivoting with the
 // reference's pivot choice, reciprocal scaling (or division below sfmin) and
-// AXPY rounding; trailing columns (n > m) take all interchanges, then the
-// updates with the final L.
+// AXPY rounding, in memory, for blocks too tall for CtaLeafReg. Leaves the
+// moved rows in the list.
 template <typename T>
-__device__ void CtaLeaf(int m, int n, Mat<T> a, int* ipiv, int* info, int col0, int lanes,
+__device__ void CtaLeaf(int m, int w, Mat<T> a, int* ipiv, int* info, int col0, int lanes,
                         LuShared<T>& sh) {
-  const int w = min(m, n);
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int nwarps = blockDim.x / 32;
   for (int j = 0; j < w; ++j) {
@@ -645,30 +675,162 @@ __device__ void CtaLeaf(int m, int n, Mat<T> a, int* ipiv, int* info, int col0, 
     }
     __syncthreads();
   }
-  for (int k = w + threadIdx.x; k < n; k += blockDim.x) {
+  // The rows moved, by replaying the interchanges on the rows they touch.
+  if (threadIdx.x == 0) {
+    int cnt = w;
+    for (int i = 0; i < w; ++i) sh.dst[i] = sh.src[i] = i;
     for (int j = 0; j < w; ++j) {
       const int p = ipiv[j] - 1;
-      if (p != j) {
-        const T t = a(j, k);
-        a(j, k) = a(p, k);
-        a(p, k) = t;
+      int e = 0;
+      while (e < cnt && sh.dst[e] != p) ++e;
+      if (e == cnt) sh.dst[e] = sh.src[e] = p, ++cnt;
+      const int t = sh.src[j];
+      sh.src[j] = sh.src[e];
+      sh.src[e] = t;
+    }
+    sh.moves = cnt;
+  }
+  __syncthreads();
+}
+
+// The same leaf (m >= w, at most 2 rows a thread) with the rows in registers:
+// bound by the latency of its w dependent pivot searches, two block barriers
+// each. Rows are not interchanged: each keeps its place and carries its
+// position; multipliers and finished rows are written at their place, and the
+// moved rows go into the list, for every column of the matrix (the leaf's too).
+// The update shifts a row's registers, so that the current column is the first
+// (the loop is rolled). Searching and updating in memory, a column took several
+// round trips to L2.
+template <typename T>
+__device__ void CtaLeafReg(int m, int w, Mat<T> a, int* ipiv, int* info, int col0, int lanes,
+                           LuShared<T>& sh) {
+  constexpr bool kWide = sizeof(T) == 8;
+  const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, nwarps = blockDim.x / 32;
+  T x[2][kLeafW];
+  int pos[2];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int i = tid + r * blockDim.x;
+    pos[r] = i < m ? i : -1;
+#pragma unroll
+    for (int k = 0; k < kLeafW; ++k) x[r][k] = i < m && k < w ? a(i, k) : T(0);
+  }
+  if (tid == 0) sh.moves = 0;
+#pragma unroll 1
+  for (int j = 0; j < w; ++j) {
+    const int par = j & 1;
+    unsigned long long key[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      key[r] = pos[r] >= j ? PivotKey(x[r][0]) : 0ull;
+      // A NaN at position j wins, as the reference's search starts from it.
+      if (pos[r] == j && key[r] == 0) key[r] = kWide ? ~0ull : 0xffffffffull;
+    }
+    const bool second = key[1] > key[0] || (key[1] == key[0] && key[1] != 0 && pos[1] < pos[0]);
+    const unsigned long long mine = second ? key[1] : key[0];
+    const int my_pos = second ? pos[1] : pos[0];
+    const int wbest = WarpBest<kWide>(mine, my_pos);
+    if (lane == wbest) {
+      sh.wkey[par][warp] = mine;
+      sh.wpos[par][warp] = my_pos;
+    }
+    __syncthreads();
+    const int cbest = WarpBest<kWide>(lane < nwarps ? sh.wkey[par][lane] : 0ull,
+                                      lane < nwarps ? sh.wpos[par][lane] : 0x7fffffff);
+    if (warp == cbest && lane == wbest) {
+#pragma unroll
+      for (int k = 0; k < kLeafW; ++k) sh.row[k] = second ? x[1][k] : x[0][k];
+      sh.rinv = T(1) / (second ? x[1][0] : x[0][0]);
+      sh.piv = my_pos;
+    }
+    __syncthreads();
+    const int piv = sh.piv, len = m - j - 1;
+    const T pivot = sh.row[0], rinv = sh.rinv;
+    const bool tiny = !(fabs(pivot) >= Sfmin<T>());
+    if (tid == 0) {
+      ipiv[j] = piv + 1;
+      if (pivot == T(0) && *info == 0) *info = col0 + j + 1;
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int i = tid + r * blockDim.x;
+      if (pos[r] == piv) {  // the pivot row's part from column j on
+        pos[r] = j;
+        for (int k = 0; k < w - j; ++k) a(i, j + k) = sh.row[k];
+      } else if (pos[r] == j) {
+        pos[r] = piv;
+      }
+      if (pos[r] <= j) continue;
+      T l = x[r][0] * rinv;
+      if (tiny) l = pivot != T(0) ? x[r][0] / pivot : x[r][0];
+      a(i, j) = l;
+      if (len >= lanes) {
+#pragma unroll
+        for (int k = 1; k < kLeafW; ++k) {
+          if (k == 9 && w - j <= 9) break;  // no such columns
+          x[r][k - 1] = fma(l, -sh.row[k], x[r][k]);
+        }
+      } else {
+#pragma unroll
+        for (int k = 1; k < kLeafW; ++k)
+          x[r][k - 1] = Axpy(x[r][k], -sh.row[k], l, len, lanes);
       }
     }
-    for (int j = 0; j < w; ++j) {
-      const T alpha = -a(j, k);
-      const int len = m - j - 1;
-      for (int i = j + 1; i < m; ++i) a(i, k) = Axpy(a(i, k), alpha, a(i, j), len, lanes);
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int i = tid + r * blockDim.x;
+    if (i < m && pos[r] != i) {
+      const int e = atomicAdd(&sh.moves, 1);
+      sh.dst[e] = pos[r];
+      sh.src[e] = i;
     }
   }
   __syncthreads();
 }
 
-// The reference's recursive LU (Getrf2) of an m x n block at a, with the
-// block's pivots in ipiv (block-relative, 1-based) and col0 its first global
-// column (for INFO). Recursion emulated with an explicit stack; frames sit
-// on the block's diagonal at offset off.
+// Moves rows (cnt of them, dst[e] from src[e], a permutation of one set) of
+// columns [0, n) but [skip, skip_end): a batch of whole columns is read before it
+// is written.
+template <typename T>
+__device__ void CtaMoveRows(int n, int skip, int skip_end, Mat<T> a, int cnt, const int* dst,
+                            const int* src) {
+  constexpr int kPer = 4;
+  if (cnt == 0) return;
+  const int per = kPer * blockDim.x / cnt;  // columns of a batch
+  const int total = n - (skip_end - skip);
+  for (int c0 = 0; c0 < total; c0 += per) {
+    const int items = min(per, total - c0) * cnt;
+    T v[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int idx = threadIdx.x + i * blockDim.x;
+      if (idx >= items) continue;
+      int c = c0 + idx / cnt;
+      if (c >= skip) c += skip_end - skip;
+      v[i] = a(src[idx % cnt], c);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int idx = threadIdx.x + i * blockDim.x;
+      if (idx >= items) continue;
+      int c = c0 + idx / cnt;
+      if (c >= skip) c += skip_end - skip;
+      a(dst[idx % cnt], c) = v[i];
+    }
+  }
+  __syncthreads();
+}
+
+// The reference's recursive LU (Getrf2) of the m x n block (m >= n) at (j, j) of the
+// matrix a of cols columns, with the block's pivots in ipiv (block-relative,
+// 1-based) and j its first column (for INFO). Each leaf's interchanges are applied
+// to all of the matrix's columns at once: nothing else reads a column between
+// them and the point where the reference applies them. Recursion emulated with
+// an explicit stack; frames sit on the block's diagonal at offset off.
 template <typename T, typename G>
-__device__ void CtaGetrfRec(int m, int n, Mat<T> a, int* ipiv, int* info, int col0,
+__device__ void CtaGetrfRec(int m, int n, Mat<T> a, int cols, int j, int* ipiv, int* info,
                             int lanes, LuShared<T>& sh, const G& gemm) {
   int s_m[12], s_n[12], s_off[12], s_ph[12];
   int sp = 0;
@@ -678,19 +840,27 @@ __device__ void CtaGetrfRec(int m, int n, Mat<T> a, int* ipiv, int* info, int co
   s_ph[0] = 0;
   while (sp >= 0) {
     const int fm = s_m[sp], fn = s_n[sp], off = s_off[sp];
-    const Mat<T> fa = a.sub(off, off);
+    const Mat<T> fa = a.sub(j + off, j + off);
     int* fp = ipiv + off;
     if (fm == 0 || fn == 0) {
       --sp;
       continue;
     }
-    const int mn = min(fm, fn);
-    if (mn <= 16) {
-      CtaLeaf(fm, fn, fa, fp, info, col0 + off, lanes, sh);
+    if (fn <= kLeafW) {
+      const int c0 = j + off;
+      int skip = 0, skip_end = 0;
+      if (fm <= 2 * static_cast<int>(blockDim.x)) {
+        CtaLeafReg(fm, fn, fa, fp, info, c0, lanes, sh);
+      } else {
+        CtaLeaf(fm, fn, fa, fp, info, c0, lanes, sh);
+        skip = c0;
+        skip_end = c0 + fn;
+      }
+      CtaMoveRows(cols, skip, skip_end, a.sub(c0, 0), sh.moves, sh.dst, sh.src);
       --sp;
       continue;
     }
-    const int n1 = mn / 2, n2 = fn - n1;
+    const int n1 = fn / 2, n2 = fn - n1;
     const int ph = s_ph[sp]++;
     if (ph == 0) {
       ++sp;
@@ -699,7 +869,6 @@ __device__ void CtaGetrfRec(int m, int n, Mat<T> a, int* ipiv, int* info, int co
       s_off[sp] = off;
       s_ph[sp] = 0;
     } else if (ph == 1) {
-      CtaLaswp(n2, fa.sub(0, n1), 1, n1, fp);
       CtaTrsmLeft(fa, true, true, n1, n2, &fa(0, n1), fa.cs, sh.st, sh.sinv, gemm);
       gemm(fm - n1, n2, n1, T(-1), fa.sub(n1, 0), fa.sub(0, n1), T(1), fa.sub(n1, n1));
       ++sp;
@@ -708,9 +877,8 @@ __device__ void CtaGetrfRec(int m, int n, Mat<T> a, int* ipiv, int* info, int co
       s_off[sp] = off + n1;
       s_ph[sp] = 0;
     } else {
-      for (int i = n1 + threadIdx.x; i < mn; i += blockDim.x) fp[i] += n1;
+      for (int i = n1 + threadIdx.x; i < fn; i += blockDim.x) fp[i] += n1;
       __syncthreads();
-      CtaLaswp(n1, fa, n1 + 1, mn, fp);
       --sp;
     }
   }
@@ -721,25 +889,63 @@ template <typename T, typename G>
 __device__ void CtaGetrf(int n, Mat<T> a, int* ipiv, int* info, int lanes,
                          LuShared<T>& sh, const G& gemm) {
   constexpr int nb = 64;
-  if (n == 0) return;
-  if (nb >= n) {
-    CtaGetrfRec(n, n, a, ipiv, info, 0, lanes, sh, gemm);
-    return;
-  }
   for (int j = 0; j < n; j += nb) {
     const int jb = min(n - j, nb);
-    CtaGetrfRec(n - j, jb, a.sub(j, j), ipiv + j, info, j, lanes, sh, gemm);
-    for (int i = j + threadIdx.x; i < j + jb; i += blockDim.x) ipiv[i] += j;
+    CtaGetrfRec(n - j, jb, a, n, j, ipiv + j, info, lanes, sh, gemm);
+    for (int i = j + threadIdx.x; j > 0 && i < j + jb; i += blockDim.x) ipiv[i] += j;
     __syncthreads();
-    CtaLaswp(j, a, j + 1, j + jb, ipiv);
     if (j + jb < n) {
-      CtaLaswp(n - j - jb, a.sub(0, j + jb), j + 1, j + jb, ipiv);
       CtaTrsmLeft(a.sub(j, j), true, true, jb, n - j - jb, &a(j, j + jb), a.cs, sh.st,
                   sh.sinv, gemm);
       gemm(n - j - jb, n - j - jb, jb, T(-1), a.sub(j + jb, j), a.sub(j, j + jb), T(1),
            a.sub(j + jb, j + jb));
     }
   }
+}
+
+// All n interchanges of a solve on B's columns (backward: from the last): replayed
+// on the row order in shared memory, then each column is one gather.
+template <typename T>
+__device__ void CtaSolveSwaps(bool backward, int n, int nrhs, Mat<T> b, const int* ipiv,
+                              LuShared<T>& sh) {
+  constexpr int kPer = 4;
+  if (n > kPermMax || n > kPer * static_cast<int>(blockDim.x)) {
+    if (backward) CtaLaswpBack(nrhs, b, 1, n, ipiv);
+    else CtaLaswp(nrhs, b, 1, n, ipiv);
+    return;
+  }
+  static_assert(sizeof(sh.st) >= sizeof(sh.perm), "the pivots fit the triangle's place");
+  int* piv = reinterpret_cast<int*>(sh.st);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    sh.perm[i] = i;
+    piv[i] = ipiv[i];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < n; ++s) {
+      const int i = backward ? n - 1 - s : s, p = piv[i] - 1;
+      if (p == i) continue;
+      const int t = sh.perm[i];
+      sh.perm[i] = sh.perm[p];
+      sh.perm[p] = t;
+    }
+  }
+  __syncthreads();
+  for (int c = 0; c < nrhs; ++c) {
+    T v[kPer];
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      if (i < n) v[k] = b(sh.perm[i], c);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      if (i < n && sh.perm[i] != i) b(i, c) = v[k];
+    }
+  }
+  __syncthreads();
 }
 
 // The reference's Getrs: solve op(A) X = B with the LU factors.
@@ -749,7 +955,7 @@ __device__ void CtaGetrs(bool trans, int n, int nrhs, Mat<T> a, const int* ipiv,
   if (n == 0 || nrhs == 0) return;
   const Mat<T> bm = Col(b, ldb);
   if (!trans) {
-    CtaLaswp(nrhs, bm, 1, n, ipiv);
+    CtaSolveSwaps(false, n, nrhs, bm, ipiv, sh);
     CtaTrsmLeft(a, true, true, n, nrhs, b, ldb, sh.st, sh.sinv, gemm);
     CtaTrsmLeft(a, false, false, n, nrhs, b, ldb, sh.st, sh.sinv, gemm);
   } else {
@@ -757,7 +963,7 @@ __device__ void CtaGetrs(bool trans, int n, int nrhs, Mat<T> a, const int* ipiv,
     const Mat<T> at = {a.p, a.cs, a.rs};
     CtaTrsmLeft(at, true, false, n, nrhs, b, ldb, sh.st, sh.sinv, gemm);
     CtaTrsmLeft(at, false, true, n, nrhs, b, ldb, sh.st, sh.sinv, gemm);
-    CtaLaswpBack(nrhs, bm, 1, n, ipiv);
+    CtaSolveSwaps(true, n, nrhs, bm, ipiv, sh);
   }
 }
 
@@ -1054,12 +1260,12 @@ template <int Kind, typename T>
 void* LuKernelOf(int config) {
   if constexpr (sizeof(T) == 8) {
     if (config == kDmma32) return reinterpret_cast<void*>(BatchedLuDmmaKernel<Kind, 2, 2, 2, 4>);
-    if (config == kDmma64) return reinterpret_cast<void*>(BatchedLuDmmaKernel<Kind, 4, 2, 4, 3>);
+    if (config == kDmma64) return reinterpret_cast<void*>(BatchedLuDmmaKernel<Kind, 4, 2, 4, 2>);
   }
   if (config == 64) return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 64, 8>);
   if (config == 128) return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 128, 4>);
   if (config == kDense128) return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 128, 6>);
-  return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 256, 3>);
+  return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 256, 2>);
 }
 
 template <typename T>
