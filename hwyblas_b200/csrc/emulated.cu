@@ -69,6 +69,18 @@ __global__ void FillIntKernel(int* p, int n, int v) {
   if (i < n) p[i] = v;
 }
 
+// |x| as its bits, which order as the values do; infinities and NaNs are at least
+// kInfBits.
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ull;
+__device__ __forceinline__ unsigned long long AbsBits(double x) {
+  return __double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+__device__ __forceinline__ int ExpOfBits(unsigned long long bits) {
+  int e;
+  frexp(__longlong_as_double(bits), &e);
+  return e;
+}
+
 // x(o, k) = data[o * os + k * is]; reduction over k for every o.
 __global__ void ExpOuterContigKernel(View<double> x, int outer, int inner,
                                      int* exps, int* nonfinite) {
@@ -76,19 +88,11 @@ __global__ void ExpOuterContigKernel(View<double> x, int outer, int inner,
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= outer) return;
   const int k0 = blockIdx.y * 256, k1 = min(inner, k0 + 256);
-  double mx = 0.0;
-  bool bad = false;
-  for (int k = k0; k < k1; ++k) {
-    const double v = x.data[o * x.rs + k * x.cs];
-    bad |= !isfinite(v);
-    mx = fmax(mx, fabs(v));
-  }
-  if (bad) atomicOr(nonfinite, 1);
-  if (mx > 0.0) {
-    int e;
-    frexp(mx, &e);
-    atomicMax(&exps[o], e);
-  }
+  unsigned long long mx = 0;
+#pragma unroll 8
+  for (int k = k0; k < k1; ++k) mx = max(mx, AbsBits(x.data[o * x.rs + k * x.cs]));
+  if (mx >= kInfBits) atomicOr(nonfinite, 1);
+  if (mx > 0) atomicMax(&exps[o], ExpOfBits(mx));
 }
 
 __global__ void ExpInnerContigKernel(View<double> x, int outer, int inner,
@@ -98,50 +102,70 @@ __global__ void ExpInnerContigKernel(View<double> x, int outer, int inner,
   const int lane = threadIdx.x % 32;
   if (warp >= outer) return;
   const double* row = x.data + static_cast<long long>(warp) * x.rs;
-  double mx = 0.0;
-  bool bad = false;
-  for (int k = lane; k < inner; k += 32) {
-    const double v = row[k];
-    bad |= !isfinite(v);
-    mx = fmax(mx, fabs(v));
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    bad |= __shfl_xor_sync(0xffffffffu, bad ? 1 : 0, off) != 0;
-  }
+  unsigned long long mx = 0;
+#pragma unroll 8
+  for (int k = lane; k < inner; k += 32) mx = max(mx, AbsBits(row[k]));
+  for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
   if (lane == 0) {
-    if (bad) atomicOr(nonfinite, 1);
-    if (mx > 0.0) {
-      int e;
-      frexp(mx, &e);
-      exps[warp] = e;
-    }
+    if (mx >= kInfBits) atomicOr(nonfinite, 1);
+    if (mx > 0) exps[warp] = ExpOfBits(mx);
   }
 }
 
-// Splits a value into S balanced base-256 digits (see the file comment).
+// a 2^n: the product with the power where that is a normal number (the same
+// single rounding as ldexp's).
+__device__ __forceinline__ double Scale(double a, int n) {
+  if (n >= -1022 && n <= 1023)
+    return a * __longlong_as_double(static_cast<long long>(1023 + n) << 52);
+  return ldexp(a, n);
+}
+
+// The S balanced base-256 digits (each in [-128, 127], the last one rounded half
+// up) of a 2^-(e + 2), |.| < 1/4: those of the whole number
+// N = floor(a 2^(8 S - e - 2) + 1/2), |N| <= 2^62. Such digits are unique, and
+// adding 128 to each digit's place and flipping the sign bits of the bytes gives
+// them all at once; byte i is digit S - 1 - i. (One floor and one conversion a value;
+// digit by digit, eight of each made the splits twice as slow as their reads and
+// writes.)
 template <int S>
-__device__ __forceinline__ void SplitValue(double a, int e, int8_t (&d)[S]) {
-  double x = (e == kZeroExp) ? 0.0 : ldexp(a, -(e + 2));
-  int di[S];
+__device__ __forceinline__ unsigned long long SplitValue(double a, int e) {
+  const double x = e == kZeroExp ? 0.0 : Scale(a, 8 * S - (e + 2));
+  double t = floor(x);
+  if (x - t >= 0.5) t = t + 1.0;
+  const long long n = fabs(t) < 9e18 ? static_cast<long long>(t) : 0;
+  constexpr unsigned long long kBias = 0x8080808080808080ull;
+  return (static_cast<unsigned long long>(n) + kBias) ^ kBias;
+}
+
+// Transposes the 4 x 4 bytes of w: word i of the result holds byte i of each.
+__device__ __forceinline__ void Transpose4(unsigned (&w)[4]) {
+  const unsigned a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+  const unsigned c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+  w[0] = __byte_perm(a, b, 0x5410);
+  w[1] = __byte_perm(a, b, 0x7632);
+  w[2] = __byte_perm(c, d, 0x5410);
+  w[3] = __byte_perm(c, d, 0x7632);
+}
+
+// packed[s] = slice s of eight values' digits, the first value in the low byte.
+template <int S>
+__device__ __forceinline__ void PackSlices(const unsigned long long (&v)[8],
+                                           unsigned long long (&packed)[S]) {
 #pragma unroll
-  for (int s = 0; s < S; ++s) {
-    const double y = x * 256.0;
-    double t = floor(y);
-    if (y - t >= 0.5) t = t + 1.0;
-    di[s] = static_cast<int>(t);
-    x = y - t;
-  }
-  // 128 = -128 + 256: carry into the more significant digit.
+  for (int half = 0; half < (S + 3) / 4; ++half) {
+    unsigned lo[4], hi[4];
 #pragma unroll
-  for (int s = S - 1; s > 0; --s) {
-    if (di[s] == 128) {
-      di[s] = -128;
-      di[s - 1] += 1;
+    for (int j = 0; j < 4; ++j) {
+      lo[j] = static_cast<unsigned>(v[j] >> (32 * half));
+      hi[j] = static_cast<unsigned>(v[j + 4] >> (32 * half));
     }
-  }
+    Transpose4(lo);
+    Transpose4(hi);
 #pragma unroll
-  for (int s = 0; s < S; ++s) d[s] = static_cast<int8_t>(di[s]);
+    for (int i = 0; i < 4; ++i)
+      if (4 * half + i < S)
+        packed[S - 1 - 4 * half - i] = lo[i] | static_cast<unsigned long long>(hi[i]) << 32;
+  }
 }
 
 // Slices of x (outer x inner) into out[s][o][kp] (K-major int8). is == 1:
@@ -156,20 +180,11 @@ __global__ void SplitInnerContigKernel(View<double> x, int outer, int inner,
   const int k0 = static_cast<int>(tid % groups) * 8;
   if (o >= outer) return;
   const int e = exps[o];
-  uint64_t packed[S];
-#pragma unroll
-  for (int s = 0; s < S; ++s) packed[s] = 0;
   const double* row = x.data + o * x.rs;
+  unsigned long long v[8], packed[S];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int k = k0 + j;
-    const double a = (k < inner) ? row[k] : 0.0;
-    int8_t d[S];
-    SplitValue<S>(a, e, d);
-#pragma unroll
-    for (int s = 0; s < S; ++s)
-      packed[s] |= static_cast<uint64_t>(static_cast<uint8_t>(d[s])) << (8 * j);
-  }
+  for (int j = 0; j < 8; ++j) v[j] = SplitValue<S>(k0 + j < inner ? row[k0 + j] : 0.0, e);
+  PackSlices<S>(v, packed);
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     *reinterpret_cast<uint64_t*>(out + (static_cast<long long>(s) * outer + o) * kp + k0) =
@@ -177,41 +192,42 @@ __global__ void SplitInnerContigKernel(View<double> x, int outer, int inner,
   }
 }
 
-// os == 1: a 64 (o) x 64 (k) tile through shared memory (read along o, write
-// along k).
+// os == 1: a 64 (o) x 64 (k) tile through shared memory, read along o; the
+// slices go through it too and out along k, 64 bytes a row.
 template <int S>
 __global__ void __launch_bounds__(512)
     SplitOuterContigKernel(View<double> x, int outer, int inner,
                            const int* exps, int8_t* out, long long kp) {
-  __shared__ double tile[64][65];  // [k][o]
+  constexpr int kRow = 80;  // bytes: 16-byte aligned, few bank conflicts
+  constexpr int kBytes = S * 64 * kRow > 64 * 65 * 8 ? S * 64 * kRow : 64 * 65 * 8;
+  __shared__ __align__(16) unsigned char smem[kBytes];
+  double* tile = reinterpret_cast<double*>(smem);  // [k][65]
   const int o0 = blockIdx.x * 64, k0 = blockIdx.y * 64;
-  for (int idx = threadIdx.x; idx < 64 * 64; idx += blockDim.x) {
-    const int ol = idx % 64, kl = idx / 64;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int ol = threadIdx.x % 64, kl = threadIdx.x / 64 + 8 * i;
     const int o = o0 + ol, k = k0 + kl;
-    tile[kl][ol] = (o < outer && k < inner) ? x.data[o * x.rs + k * x.cs] : 0.0;
+    tile[kl * 65 + ol] = (o < outer && k < inner) ? x.data[o * x.rs + k * x.cs] : 0.0;
   }
   __syncthreads();
   const int ol = threadIdx.x % 64, kq = threadIdx.x / 64;  // 8 groups of 8 k
-  const int o = o0 + ol;
-  if (o >= outer) return;
-  const int e = exps[o];
-  uint64_t packed[S];
+  const int e = o0 + ol < outer ? exps[o0 + ol] : kZeroExp;
+  unsigned long long v[8], packed[S];
 #pragma unroll
-  for (int s = 0; s < S; ++s) packed[s] = 0;
+  for (int j = 0; j < 8; ++j) v[j] = SplitValue<S>(tile[(kq * 8 + j) * 65 + ol], e);
+  PackSlices<S>(v, packed);
+  __syncthreads();  // the tile is read
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    int8_t d[S];
-    SplitValue<S>(tile[kq * 8 + j][ol], e, d);
+  for (int s = 0; s < S; ++s)
+    *reinterpret_cast<unsigned long long*>(smem + (s * 64 + ol) * kRow + kq * 8) = packed[s];
+  __syncthreads();
 #pragma unroll
-    for (int s = 0; s < S; ++s)
-      packed[s] |= static_cast<uint64_t>(static_cast<uint8_t>(d[s])) << (8 * j);
-  }
-  const int k = k0 + kq * 8;
-  if (k >= inner) return;
-#pragma unroll
-  for (int s = 0; s < S; ++s) {
-    *reinterpret_cast<uint64_t*>(out + (static_cast<long long>(s) * outer + o) * kp + k) =
-        packed[s];
+  for (int i = 0; i < (S + 1) / 2; ++i) {
+    const int idx = threadIdx.x + 512 * i;
+    const int q = idx % 4, row = idx / 4, o = o0 + row % 64, k = k0 + 16 * q;
+    if (row >= S * 64 || o >= outer || k >= inner) continue;
+    *reinterpret_cast<uint4*>(out + (static_cast<long long>(row / 64) * outer + o) * kp + k) =
+        *reinterpret_cast<const uint4*>(smem + row * kRow + 16 * q);
   }
 }
 
@@ -522,8 +538,9 @@ __global__ void SumSqPContigKernel(View<double> x, int outer, int inner,
   const int o0 = blockIdx.y * kSumSqRowsP, o1 = min(outer, o0 + kSumSqRowsP);
   double s = 0.0;
   if (E != kZeroExp) {
+#pragma unroll 8
     for (int o = o0; o < o1; ++o) {
-      const double v = ldexp(x.data[o * x.rs + p * x.cs], -E);
+      const double v = Scale(x.data[o * x.rs + p * x.cs], -E);
       s = fma(v, v, s);
     }
   }
@@ -540,8 +557,9 @@ __global__ void SumSqOContigKernel(View<double> x, int outer, int inner,
   const int o0 = blockIdx.y * kSumSqRowsO, o1 = min(outer, o0 + kSumSqRowsO);
   double s = 0.0;
   if (E != kZeroExp) {
+#pragma unroll 8
     for (int o = o0 + lane; o < o1; o += 32) {
-      const double v = ldexp(x.data[o * x.rs + p * x.cs], -E);
+      const double v = Scale(x.data[o * x.rs + p * x.cs], -E);
       s = fma(v, v, s);
     }
   }
@@ -566,11 +584,23 @@ struct AutoArgs {
   const int* col_exp;
   int m, n, k;
   const int* emax;      // [0] E of op(A), [1] F of op(B)
-  const double* part_a;  // [chunks_a][k]
-  const double* part_b;  // [chunks_b][k]
-  int chunks_a, chunks_b;
+  const double* sum_a;  // [k] sums of squares over op(A)'s column p
+  const double* sum_b;  // [k] over op(B)'s row p
   int* slices_out;      // the chosen S (0: the plain path)
 };
+
+// sum[y k + p] = operand y's partial sums of p, in the chunks' order.
+__global__ void SumChunksKernel(const double* part_a, int chunks_a, const double* part_b,
+                                int chunks_b, int k, double* sum) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= k) return;
+  const double* part = blockIdx.y == 0 ? part_a : part_b;
+  const int chunks = blockIdx.y == 0 ? chunks_a : chunks_b;
+  double s = 0.0;
+#pragma unroll 8
+  for (int c = 0; c < chunks; ++c) s += part[static_cast<long long>(c) * k + p];
+  sum[static_cast<long long>(blockIdx.y) * k + p] = s;
+}
 
 // One block of 1024 threads: the statistic and the slice count.
 __global__ void AutoSlicesKernel(AutoArgs g) {
@@ -582,12 +612,7 @@ __global__ void AutoSlicesKernel(AutoArgs g) {
       if (g.row_exp[i] != kZeroExp) sa += ldexp(1.0, 2 * (g.row_exp[i] - E));
     for (int j = threadIdx.x; j < g.n; j += blockDim.x)
       if (g.col_exp[j] != kZeroExp) sb += ldexp(1.0, 2 * (g.col_exp[j] - F));
-    for (int p = threadIdx.x; p < g.k; p += blockDim.x) {
-      double ca = 0.0, rb = 0.0;
-      for (int c = 0; c < g.chunks_a; ++c) ca += g.part_a[static_cast<long long>(c) * g.k + p];
-      for (int c = 0; c < g.chunks_b; ++c) rb += g.part_b[static_cast<long long>(c) * g.k + p];
-      q = fma(ca, rb, q);
-    }
+    for (int p = threadIdx.x; p < g.k; p += blockDim.x) q = fma(g.sum_a[p], g.sum_b[p], q);
   }
   sa = BlockSum(sa, s);
   sb = BlockSum(sb, s);
@@ -770,7 +795,7 @@ int DgemmEmulated(int m, int n, int k, double alpha, View<double> a,
                                   : (n + kSumSqRowsP - 1) / kSumSqRowsP;
   const size_t int_bytes = (sizeof(int) * (m + n + 64) + 255) / 256 * 256;
   const size_t part_bytes =
-      automatic ? sizeof(double) * static_cast<size_t>(chunks_a + chunks_b) * k : 0;
+      automatic ? sizeof(double) * static_cast<size_t>(chunks_a + chunks_b + 2) * k : 0;
   char* acc = static_cast<char*>(Workspace(ws_acc, int_bytes + part_bytes));
   int* exps = reinterpret_cast<int*>(acc);
   int* row_exp = exps;
@@ -795,10 +820,11 @@ int DgemmEmulated(int m, int n, int k, double alpha, View<double> a,
     g.n = n;
     g.k = k;
     g.emax = flags + 2;
-    g.part_a = part_a;
-    g.part_b = part_b;
-    g.chunks_a = ca;
-    g.chunks_b = cb;
+    double* sums = part_b + static_cast<size_t>(chunks_b) * k;
+    SumChunksKernel<<<dim3((k + 127) / 128, 2), 128, 0, st>>>(part_a, ca, part_b, cb, k, sums);
+    CountLaunch();
+    g.sum_a = sums;
+    g.sum_b = sums + k;
     g.slices_out = flags + 1;
     AutoSlicesKernel<<<1, 1024, 0, st>>>(g);
     CountLaunch();
