@@ -387,16 +387,21 @@ __global__ void __launch_bounds__(kTcThreads) TrsmClusterKernel(TrsmClusterArgs<
   const bool rows_fast = p.tri.rs == 1;
   const int blocks = (p.r + 31) / 32;
   // Base triangle number t (in the order they are solved), in solve order:
-  // st[s][u] = T(row u, column s), s <= u.
+  // st[s][u] = T(row u, column s), s <= u. A thread copies the same four (s, u) of
+  // each, from the block's corner in solve order.
+  const long long step_r = p.lower ? p.tri.rs : -p.tri.rs, step_c = p.lower ? p.tri.cs : -p.tri.cs;
+  const int fast = threadIdx.x % 32, slow = threadIdx.x / 32;
   const auto load_base = [&](int t) {
     if (t >= blocks || rank >= nrhs) return;
     const int off = 32 * (p.lower ? t : blocks - 1 - t), n = min(32, p.r - off);
+    const int corner = p.lower ? off : off + n - 1;
+    const T* src = p.tri.data + corner * (p.tri.rs + p.tri.cs);
     T* st = tri[t & 1];
-    for (int idx = threadIdx.x; idx < 32 * 32; idx += kTcThreads) {
-      const int s = rows_fast ? idx / 32 : idx % 32, u = rows_fast ? idx % 32 : idx / 32;
-      if (s > u || u >= n || (s == u && p.unit)) continue;
-      const int row = off + (p.lower ? u : n - 1 - u), q = off + (p.lower ? s : n - 1 - s);
-      TcCopy(st + s * 33 + u, p.tri.data + row * p.tri.rs + q * p.tri.cs);
+#pragma unroll
+    for (int i = 0; i < 32; i += kTcThreads / 32) {
+      const int s = rows_fast ? slow + i : fast, u = rows_fast ? fast : slow + i;
+      if (s < u ? u < n : s == u && u < n && !p.unit)
+        TcCopy(st + s * 33 + u, src + u * step_r + s * step_c);
     }
   };
   load_base(0);

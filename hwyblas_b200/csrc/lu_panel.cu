@@ -42,9 +42,9 @@ template <typename T>
 constexpr int kPanelThreads = sizeof(T) == 16 ? 256 : 512;
 constexpr int kPanelLeast = 256;   // threads at least: the solves share all warps
 constexpr int kPanelCtas = 16;
-// Polls of a wait for the other CTAs' candidates (some 30 ns each): far above
-// any real wait.
-constexpr uint32_t kPanelPolls = 1u << 22;
+// Polls of a wait for the other CTAs' candidates, each suspended for at most
+// about 1 us (spinning warps slow the others down): far above any real wait.
+constexpr uint32_t kPanelPolls = 1u << 20;
 
 template <typename R>
 struct __align__(2 * sizeof(R)) Cx {
@@ -170,7 +170,7 @@ struct __align__(16) PanelSlot {
 
 template <typename T>
 struct PanelArgs {
-  int m, w, R, lanes;  // R: rows of a CTA
+  int m, w, R, S, lanes;  // R: rows of a CTA; S: their stride in shared memory
   T* a;
   long long lda;
   int* ipiv;
@@ -239,10 +239,10 @@ __device__ __forceinline__ bool MbarTest(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(SmemAddr(bar)), "r"(parity)
+      : "r"(SmemAddr(bar)), "r"(parity), "r"(1000u)
       : "memory");
   return ok != 0;
 }
@@ -423,15 +423,61 @@ __device__ __forceinline__ void PanelUpdateComplex(const Cx<R>* l, Cx<R>* x, int
   }
 }
 
+// Sixteen rows of the update on the FP64 tensor pipe (bound by instructions as FMAs:
+// 32 x 32 of 256 rows took 8 us): the m16n8k8 chain runs over q ascending; past n1,
+// -0 times +0 leaves every sum as it is. pos[i] >= least: row i is updated.
+__device__ __forceinline__ void PanelUpdateDmma(const double* l, double* x, int S,
+                                                const double* u, int n1, int n2, const int* pos,
+                                                int rows, int least) {
+  const int lane = threadIdx.x % 32, g = lane >> 2, t = lane & 3;
+  double acc[4][4];
+#pragma unroll
+  for (int b = 0; b < 4; ++b)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[b][e] = 0.0;
+#pragma unroll 2
+  for (int k0 = 0; k0 < n1; k0 += 8) {
+    const int q0 = k0 + t, q1 = q0 + 4;
+    const double* a0 = l + min(q0, n1 - 1) * S + g;
+    const double* a1 = l + min(q1, n1 - 1) * S + g;
+    const double f0 = q0 < n1 ? a0[0] : -0.0, f1 = q0 < n1 ? a0[8] : -0.0;
+    const double f2 = q1 < n1 ? a1[0] : -0.0, f3 = q1 < n1 ? a1[8] : -0.0;
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      if (b * 8 >= n2) break;
+      const int c = min(b * 8 + g, n2 - 1);
+      const double b0 = q0 < n1 ? u[q0 * kPanelLd<double> + c] : 0.0;
+      const double b1 = q1 < n1 ? u[q1 * kPanelLd<double> + c] : 0.0;
+      asm volatile(
+          "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
+          "{%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+          : "+d"(acc[b][0]), "+d"(acc[b][1]), "+d"(acc[b][2]), "+d"(acc[b][3])
+          : "d"(f0), "d"(f1), "d"(f2), "d"(f3), "d"(b0), "d"(b1));
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = g + 8 * h;
+    if (i >= rows || pos[i] < least) continue;
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = b * 8 + 2 * t + e;
+        if (c < n2) x[c * S + i] = -1.0 * acc[b][2 * h + e] + x[c * S + i];
+      }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T> p) {
   extern __shared__ __align__(16) unsigned char panel_smem[];
-  const int P = gridDim.x, cta = blockIdx.x, R = p.R, w = p.w;
+  const int P = gridDim.x, cta = blockIdx.x, R = p.R, RS = p.S, w = p.w;
   // [2][kPanelCtas] from the CTAs, then this CTA's own.
   PanelSlot<T>* slots = reinterpret_cast<PanelSlot<T>*>(panel_smem);
   PanelSlot<T>* own = slots + 2 * kPanelCtas;
   T* prow = reinterpret_cast<T*>(own + 1);                           // [w][kPanelLd] pivot rows
-  T* S = prow + w * kPanelLd<T>;                                     // [w][R] this CTA's rows
+  T* S = prow + w * kPanelLd<T>;                                     // [w][RS] this CTA's rows
   __shared__ T s_rinv[2][kPanelCtas];
   __shared__ unsigned long long s_wkey[2][kPanelThreads<T> / 32];
   __shared__ int s_wpos[2][kPanelThreads<T> / 32];
@@ -478,7 +524,7 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
   if (valid) {
     const T* src = p.a + place;
 #pragma unroll 4
-    for (int c = 0; c < w; ++c) CopyElement(S + c * R + tid, src + c * p.lda);
+    for (int c = 0; c < w; ++c) CopyElement(S + c * RS + tid, src + c * p.lda);
   }
   CpAsyncCommit();
   CpAsyncWait<0>();
@@ -495,7 +541,7 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
       T x[kPanelLeaf];
 #pragma unroll
       for (int k = 0; k < kPanelLeaf; ++k)
-        x[k] = valid && k < n1 ? S[(c0 + k) * R + tid] : Zero<T>();
+        x[k] = valid && k < n1 ? S[(c0 + k) * RS + tid] : Zero<T>();
 #pragma unroll 1
       for (int j = 0; j < n1; ++j) {
         const int jc = c0 + j, par = jc & 1;
@@ -588,7 +634,7 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
           // rank-1 update of the leaf's later columns, which move up by one.
           T l = Times(x[0], s_rinv[par][from & (kPanelCtas - 1)]);
           if (IsTiny(pivot)) l = IsZero(pivot) ? x[0] : Over(x[0], pivot);
-          S[jc * R + tid] = l;
+          S[jc * RS + tid] = l;
           const int len = p.m - jc - 1;
           if (len >= p.lanes) {
 #pragma unroll
@@ -618,8 +664,8 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
             const int col = lane + 32 * d;
             if (col >= w || (col >= c0 + r && col < c0 + n1)) continue;
             prow[(c0 + r) * kPanelLd<T> + col] =
-                P > 1 ? LoadRemote(MapRank(SmemAddr(row + col * R), owner), Zero<T>())
-                      : row[col * R];
+                P > 1 ? LoadRemote(MapRank(SmemAddr(row + col * RS), owner), Zero<T>())
+                      : row[col * RS];
           }
         }
         __syncthreads();
@@ -628,24 +674,30 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
       T* rows = prow + c0 * kPanelLd<T> + c0;
       PanelSolve<T>(rows, n1, n2);
       __syncthreads();
-      // Half the threads take the first cw columns of two rows each, the other
-      // half the rest.
-      const int cw = n2 > 16 ? 16 : 8, half = (R + 1) / 2;
-      const int blk = tid >= half ? 1 : 0, ra = tid - blk * half;
-      const int rb = min(ra + half, R - 1), nc = min(cw, n2 - blk * cw);
-      if (ra < half && nc > 0) {
-        const int cb = n1 + blk * cw;
-        const bool ina = s_pos[ra] >= c0 + n1;
-        const bool inb = ra + half < R && s_pos[rb] >= c0 + n1;
-        if constexpr (ElemOf<T>::kComplex)
-          PanelUpdateComplex(S + c0 * R, S + (c0 + cb) * R, R, rows + cb, n1, nc, ra, rb, ina,
-                             inb);
-        else if ((c0 + cb) % (16 / static_cast<int>(sizeof(T))) == 0)
-          PanelUpdate<T, true>(S + c0 * R, S + (c0 + cb) * R, R, rows + cb, n1, nc, cw, ra, rb,
-                               ina, inb);
-        else
-          PanelUpdate<T, false>(S + c0 * R, S + (c0 + cb) * R, R, rows + cb, n1, nc, cw, ra, rb,
-                                ina, inb);
+      if constexpr (sizeof(T) == 8 && !ElemOf<T>::kComplex) {
+        for (int r0 = warp * 16; r0 < R; r0 += nwarps * 16)
+          PanelUpdateDmma(S + c0 * RS + r0, S + (c0 + n1) * RS + r0, RS, rows + n1, n1, n2,
+                          s_pos + r0, R - r0, c0 + n1);
+      } else {
+        // Half the threads take the first cw columns of two rows each, the other
+        // half the rest.
+        const int cw = n2 > 16 ? 16 : 8, half = (R + 1) / 2;
+        const int blk = tid >= half ? 1 : 0, ra = tid - blk * half;
+        const int rb = min(ra + half, R - 1), nc = min(cw, n2 - blk * cw);
+        if (ra < half && nc > 0) {
+          const int cb = n1 + blk * cw;
+          const bool ina = s_pos[ra] >= c0 + n1;
+          const bool inb = ra + half < R && s_pos[rb] >= c0 + n1;
+          if constexpr (ElemOf<T>::kComplex)
+            PanelUpdateComplex(S + c0 * RS, S + (c0 + cb) * RS, RS, rows + cb, n1, nc, ra, rb, ina,
+                               inb);
+          else if ((c0 + cb) % (16 / static_cast<int>(sizeof(T))) == 0)
+            PanelUpdate<T, true>(S + c0 * RS, S + (c0 + cb) * RS, RS, rows + cb, n1, nc, cw, ra, rb,
+                                 ina, inb);
+          else
+            PanelUpdate<T, false>(S + c0 * RS, S + (c0 + cb) * RS, RS, rows + cb, n1, nc, cw, ra, rb,
+                                  ina, inb);
+        }
       }
       __syncthreads();
     }
@@ -659,7 +711,7 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
     if (valid && pos >= w) {
       T* dst = p.a + pos;
 #pragma unroll 8
-      for (int c = 0; c < w; ++c) StoreGlobal(dst + c * p.lda, S[c * R + tid]);
+      for (int c = 0; c < w; ++c) StoreGlobal(dst + c * p.lda, S[c * RS + tid]);
     }
     if (valid && pos != place && p.moves != nullptr) {
       const int e = atomicAdd(p.moves, 1);
@@ -671,10 +723,14 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
   if (P > 1) ClusterBarrier();
 }
 
+// Stride of a CTA's R rows in shared memory: 4 modulo 16, so that the tensor pipe's
+// fragments are free of bank conflicts, and room for whole blocks of 16.
+int PanelStride(int R) { return (R + 15) / 16 * 16 + 4; }
+
 template <typename T>
 size_t PanelSmem(int w, int R) {
   return (2 * kPanelCtas + 1) * sizeof(PanelSlot<T>) +
-         sizeof(T) * static_cast<size_t>(w) * (kPanelLd<T> + R);
+         sizeof(T) * static_cast<size_t>(w) * (kPanelLd<T> + PanelStride(R));
 }
 
 constexpr size_t kPanelSmemMax = 227 * 1024 - 4 * 1024;  // beside the static arrays
@@ -870,6 +926,7 @@ bool LaunchPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info
     return false;
   args.m = m;
   args.w = n;
+  args.S = PanelStride(args.R);
   args.lanes = sizeof(RealOf<T>) == 8 ? RefLanesDouble() : 2 * RefLanesDouble();
   args.a = a;
   args.lda = lda;
