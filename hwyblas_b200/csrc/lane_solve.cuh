@@ -15,7 +15,7 @@ namespace {
 template <bool kUnit, typename T, int N>
 __device__ __forceinline__ void LaneSolveSteps(const T* st, int ld, T inv, int r, T (&y)[N]) {
   const int lane = threadIdx.x % 32;
-#pragma unroll 2
+#pragma unroll 8
   for (int q = 0; q < r; ++q) {
     const T l = st[q * ld + lane];
 #pragma unroll
