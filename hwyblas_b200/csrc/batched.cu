@@ -700,7 +700,9 @@ __device__ void CtaLeaf(int m, int w, Mat<T> a, int* ipiv, int* info, int col0, 
 // moved rows go into the list, for every column of the matrix (the leaf's too).
 // The update shifts a row's registers, so that the current column is the first
 // (the loop is rolled). Searching and updating in memory, a column took several
-// round trips to L2.
+// round trips to L2: of n = 400 the taller half's leaves take 1300 us (CtaLeaf) where
+// the lower half's take 490 so, four CTAs an SM. 10,000 problems of 8 to 512 rows
+// without interchanges: 19.6 -> 18.8 ms, the moves included.
 template <typename T>
 __device__ void CtaLeafReg(int m, int w, Mat<T> a, int* ipiv, int* info, int col0, int lanes,
                            LuShared<T>& sh) {

@@ -614,8 +614,8 @@ __global__ void GetrfLeafTrailingKernel(int m, int w, int n, T* a,
 // decides an AXPY's rounding. Bound by the latency of the n dependent square
 // roots and reciprocals; a leaf is one warp, a lane one row, whose remaining
 // columns sit in registers that shift with every step (a rolled loop: its
-// instructions are fetched once). 64 columns: 27 us a leaf, plus solve and update
-// in launches of their own, -> the whole block in one launch.
+// instructions are fetched once). 64 columns: 35 us; two leaves took 27 us each
+// before, and the solve and the update between them were launches of their own.
 constexpr int kCholW = 64, kCholLd = kCholW + 1, kCholLeaf = 32, kCholThreads = 256;
 
 // The leaf at (c0, c0) of s; false after a non-positive (or NaN) diagonal.

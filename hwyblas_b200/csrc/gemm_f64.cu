@@ -845,8 +845,8 @@ __global__ void __launch_bounds__(256)
 // pipe, one 16 x 8 tile a warp; the KC chunks of k, whose chains are
 // independent, are dealt to the CTAs of a cluster, which then merge them in
 // order through distributed shared memory. One thread an element from global
-// memory (DgemmDirectKernel) waited on every term: 33 x 47 x 65 11 us,
-// 64 x 64 x 1000 45 us.
+// memory (DgemmDirectKernel) waited on every term: 33 x 47 x 65 11 us of kernel,
+// 6 so; 64 x 64 x 1000 58 us a call, 25 so.
 constexpr int kSmT = 32, kSmK = 64, kSmLd = kSmT + 4, kSmThreads = 256, kSmCluster = 8;
 constexpr int kSmStage = 2 * kSmK * kSmLd;  // doubles
 constexpr int kSmMaxParts = 16;             // chunks a CTA at most
@@ -1094,8 +1094,10 @@ size_t DgemmSplitBytes(int m, int n, int k) {
 namespace {
 // Products for DgemmSmallKernel: those of at most a few million multiply-adds
 // or with a side below 32, and larger ones whose (tile, chunk) pairs still fit
-// the SMs about twice, but for k <= 64 where DgemmShortKKernel can take them
-// (512 x 512 x 64: 27 us a call there, 32 here).
+// the SMs about twice (384^3 48 -> 30 us a call; beyond, each tile's loads cost
+// more than its products: 512 x 512 x 1024 69 us against 42 on the DMMA tiles),
+// but for k <= 64 where DgemmShortKKernel can take them (512 x 512 x 64: 27 us a
+// call there, 32 here).
 bool SmallTakes(int m, int n, int k, bool small, bool short_k) {
   const int nchunks = (k + 255) / 256, S = std::min(nchunks, kSmCluster);
   const long long ctas = static_cast<long long>((m + kSmT - 1) / kSmT) * ((n + kSmT - 1) / kSmT) * S;

@@ -172,7 +172,7 @@ enum KernelFamily : int {
   kFamilyNone = 0,
   kFamilyDmmaGemm = 1,   // DgemmDmmaKernel
   kFamilyOzakiGemm = 2,  // OzakiGemmKernel (all passes)
-  kFamilyLuLeaf = 3,     // GetrfLeafPanelKernel
+  kFamilyLuLeaf = 3,     // GetrfPanelKernel, GetrfLeafPanelKernel
 };
 cudaEvent_t KernelTimerStart(int family, cudaStream_t stream);
 void KernelTimerStop(cudaEvent_t start, cudaStream_t stream);

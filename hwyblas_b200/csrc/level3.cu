@@ -1,4 +1,4 @@
-// Level-3 routines around the GEMM kernels: the FP32 GEMM (FFMA on the CUDA
+// Level-3 routines around the GEMM kernels: the FP32 TRMM product (FFMA on the CUDA
 // cores, the reference's FP32 order with KC = 384), the recursive TRSM with
 // its base substitution kernel, SYRK, and the reference-semantics wrappers
 // (argument-independent quick returns and alpha scaling).
@@ -14,30 +14,10 @@ namespace hb {
 namespace {
 
 // ---------------------------------------------------------------------------
-// FP32 GEMM: 64 x 64 tile per 256-thread CTA, 4 x 4 outputs per thread, each
-// a sequential FFMA chain over k restarted every 384 (src/gemm_kernel-inl.h:72).
+// FP32 GEMM with a triangular operand (TRMM; the other products are in
+// gemm_f32.cu): 64 x 64 tile per 256-thread CTA, 4 x 4 outputs per thread, each a
+// sequential FFMA chain over k restarted every 384 (src/gemm_kernel-inl.h:72).
 constexpr int kSB = 64, kSK = 16;
-
-// `part` restricts C to one triangle (SYRK): elements outside it are neither
-// computed nor written; inside, the chain is the one of the full GEMM.
-__device__ __forceinline__ bool InPart(int part, int i, int j) {
-  return part == kAll || (part == kLower ? i >= j : i <= j);
-}
-
-// Whether C(i, j) lies in a micro-tile of the reference's AVX-512 float
-// kernel (MR 32, NR 12, MC 128, NC 4080) that crosses the diagonal: those
-// tiles merge as alpha*acc + beta*C with two roundings (src/gemm-inl.h:93-130;
-// src/gemm_kernel-inl.h:64-74).
-__device__ __forceinline__ bool InCrossingTileF(int part, int m, int n, int i, int j) {
-  constexpr int MR = 32, NR = 12, MC = 128, NC = 4080;
-  const int ic = i / MC * MC, mcb = min(MC, m - ic);
-  const int ir = (i - ic) / MR * MR, mr = min(MR, mcb - ir);
-  const int jc = j / NC * NC, ncb = min(NC, n - jc);
-  const int jr = (j - jc) / NR * NR, nr = min(NR, ncb - jr);
-  const int i0 = ic + ir, j0 = jc + jr;
-  if (part == kLower) return !(i0 > j0 + nr - 1);
-  return !(i0 + mr - 1 < j0);
-}
 
 // k range [*kb, *ke) the reference multiplies for C(i, j) when an operand is
 // triangular: NonZeroRange of the AVX-512 float micro-tile (MR 32, NR 12,
@@ -66,14 +46,11 @@ __device__ __forceinline__ void TriRangeF(int tri, int m, int n, int k, int i, i
 // reference skips the micro-tile (src/gemm-inl.h:202-209).
 __global__ void __launch_bounds__(256)
     SgemmKernel(int m, int n, int k, float alpha, View<float> a, View<float> b,
-                float beta, float* c, long long ldc, int part, int tri,
-                const int* guard) {
+                float beta, float* c, long long ldc, int tri, const int* guard) {
   if (guard != nullptr && *guard != 0) return;
   __shared__ float sa[kSK][kSB + 4];
   __shared__ float sb[kSK][kSB + 4];
   const int m0 = blockIdx.x * kSB, n0 = blockIdx.y * kSB;
-  // A tile wholly outside the triangle has nothing to do.
-  if ((part == kLower && m0 + kSB - 1 < n0) || (part == kUpper && m0 > n0 + kSB - 1)) return;
   const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
   float acc[4][4] = {}, cacc[4][4] = {};
   const int kchunk = 384;
@@ -103,19 +80,12 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
       for (int q = 0; q < 4; ++q) bv[q] = sb[kk][ty + 16 * q];
       const int kg = k0 + kk;
-      if (tri == kTriNone) {
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
+      for (int r = 0; r < 4; ++r)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(av[r], bv[q], acc[r][q]);
-      } else {
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (kg >= max(rkb[r], ckb[q]) && kg < min(rke[r], cke[q]))
-              acc[r][q] = fmaf(av[r], bv[q], acc[r][q]);
-      }
+        for (int q = 0; q < 4; ++q)
+          if (kg >= max(rkb[r], ckb[q]) && kg < min(rke[r], cke[q]))
+            acc[r][q] = fmaf(av[r], bv[q], acc[r][q]);
       if ((kg + 1) % kchunk == 0 || kg + 1 == k) {
         const bool first = kg < kchunk;
         const int c_lo = kg / kchunk * kchunk, c_hi = kg + 1;
@@ -125,20 +95,16 @@ __global__ void __launch_bounds__(256)
           for (int q = 0; q < 4; ++q) {
             const int i = m0 + tx + 16 * r, j = n0 + ty + 16 * q;
             const float rr = alpha * acc[r][q];
-            if (!first && tri != kTriNone &&
-                max(max(rkb[r], ckb[q]), c_lo) >= min(min(rke[r], cke[q]), c_hi)) {
+            if (!first && max(max(rkb[r], ckb[q]), c_lo) >= min(min(rke[r], cke[q]), c_hi)) {
               // Outside the element's k range: not merged.
             } else if (first) {
-              if (i < m && j < n && InPart(part, i, j)) {
+              if (i < m && j < n) {
                 if (beta == 0.f) {
                   cacc[r][q] = rr;
                 } else {
                   const float cin = c[i + j * ldc];
                   if (beta == 1.f) {
                     cacc[r][q] = rr + cin;
-                  } else if (part != kAll && InCrossingTileF(part, m, n, i, j)) {
-                    const float bc = beta * cin;
-                    cacc[r][q] = rr + bc;
                   } else {
                     cacc[r][q] = fmaf(cin, beta, rr);
                   }
@@ -158,7 +124,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = m0 + tx + 16 * r, j = n0 + ty + 16 * q;
-      if (i < m && j < n && InPart(part, i, j)) c[i + j * ldc] = cacc[r][q];
+      if (i < m && j < n) c[i + j * ldc] = cacc[r][q];
     }
 }
 
@@ -264,8 +230,8 @@ __global__ void __launch_bounds__(kBaseThreads)
 // chains, restarted every KC, and merges are the GEMM kernels'. Steps end with a cluster barrier, which is some 1.5 us less than a
 // grid barrier; X goes through L2. The right side is the left side of the
 // transposed system (each product's factors change places).
-// 512 rows: one right-hand side 168 us as a cooperative launch over the grid, 512
-// right-hand sides 140 us with 8 columns a CTA.
+// 512 rows: few right-hand sides 80 us (168 as a cooperative launch over the grid),
+// 64 a cluster 120 us (512 right-hand sides 140 us with 8 columns a CTA).
 constexpr int kTcRows = 512, kTcThreads = 256, kTcCtas = 8, kTcRhs = 64;
 constexpr int kTcStrip = 16, kTcStrips = kTcRows / kTcStrip / kTcCtas;  // a CTA's strips
 constexpr int kTcLd = kTcStrip + 4;  // conflict-free fragments
@@ -598,7 +564,6 @@ void Sgemm(int m, int n, int k, float alpha, View<float> a, View<float> b,
   }
   const dim3 grid((m + kSB - 1) / kSB, (n + kSB - 1) / kSB);
   SgemmKernel<<<grid, 256, 0, Ctx().stream>>>(m, n, k, alpha, a, b, beta, c, ldc,
-                                              static_cast<int>(part),
                                               static_cast<int>(tri), Ctx().guard);
   CountLaunch();
   LaunchFailed("sgemm");
