@@ -749,7 +749,7 @@ bool PanelShape(int m, int w, int most, int* ctas, int* rows) {
   const int least = (m + fit - 1) / fit;
   if (least > most) return false;
   // A row a thread: about 256 rows a CTA balance the exchange (more CTAs) with
-  // the updates (more rows).
+  // the updates (more rows); 160 measured 1 to 5 % slower (dgetrf n = 500 to 2500).
   const int want = std::max(least, std::min(most, (m + 255) / 256));
   *ctas = want;
   *rows = (m + want - 1) / want;
