@@ -51,7 +51,7 @@ struct ZParams {
   ZView<R> a, b;
   R* c;
   long long ldc;  // complex elements
-  const int* guard;
+  Guard guard;
   // HERK: only the triangle `part` of C (1 lower, 2 upper; 0 all) is
   // updated. Elements in micro-tiles of the reference (tmr x tnr, on its
   // grid) that cross the diagonal merge as its MergeTile does, with the
@@ -238,7 +238,7 @@ __device__ __forceinline__ void CpAsyncElem(void* smem_dst, const R* src, bool v
 // running value stays in C itself. FP32 only: FP64 runs ZgemmDmmaKernel.
 template <typename R, bool kConjA, bool kConjB>
 __global__ void __launch_bounds__(256, 2) ZgemmKernel(ZParams<R> p) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   using V = typename Vec2<R>::type;
   extern __shared__ __align__(16) unsigned char zsmem[];
   V* sa = reinterpret_cast<V*>(zsmem);                 // [2][kZK][kZM]
@@ -353,7 +353,7 @@ constexpr int kZdSmemBytes = kZdStages * 2 * kZK * kZdLd * 16;
 template <int kFa, bool kConjA, bool kConjB>
 __global__ void __launch_bounds__(512 / kFa, 1) ZgemmDmmaKernel(ZParams<double> p) {
   constexpr int kThreads = 512 / kFa;
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   extern __shared__ __align__(16) unsigned char zsmem[];
   double2* sa = reinterpret_cast<double2*>(zsmem);  // [stages][kZK][kZdLd]
   double2* sb = sa + kZdStages * kZK * kZdLd;       // [stages][kZK][kZdLd]
@@ -474,7 +474,7 @@ __global__ void __launch_bounds__(512 / kFa, 1) ZgemmDmmaKernel(ZParams<double> 
 // first-chunk rule, then every later chunk (ZMergeElement).
 template <typename R>
 __global__ void ZSplitMergeKernel(ZParams<R> p, int nchunks) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   const long long total = static_cast<long long>(p.m) * p.n;
   for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -495,8 +495,8 @@ constexpr int ZSmemBytes() {
 // product (c.re*b.re - c.im*b.im, c.re*b.im + c.im*b.re) (gemm.cc:48-64).
 template <typename R>
 __global__ void ZScaleKernel(int m, int n, R beta_re, R beta_im, R* c, long long ldc,
-                             const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                             Guard guard) {
+  if (guard.Stops()) return;
   const long long total = static_cast<long long>(m) * n;
   const bool zero = (beta_re == R(0) && beta_im == R(0));
   for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
@@ -553,8 +553,8 @@ __device__ __forceinline__ void ZLoadTriangle(const ZView<R>& tri, int lower, in
 template <typename R>
 __global__ void __launch_bounds__(128)
     ZTrsmBaseKernel(ZView<R> tri, int lower, int unit, int r, int rows, R* x,
-                    long long xs_row, long long xs_col, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                    long long xs_row, long long xs_col, Guard guard) {
+  if (guard.Stops()) return;
   // st[s][u] = T(q(s), j(u)) in solve order (conjugated for 'C').
   __shared__ R st_re[32][33], st_im[32][33];
   __shared__ R inv_re[32], inv_im[32];
@@ -630,8 +630,8 @@ constexpr int kZLaneThreads = 256, kZLaneRows = 2 * kZLaneThreads / 32;
 template <typename R>
 __global__ void __launch_bounds__(kZLaneThreads)
     ZTrsmLaneKernel(ZView<R> tri, int unit, int r, int rows, R* x, long long xs_row,
-                    long long xs_col, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                    long long xs_col, Guard guard) {
+  if (guard.Stops()) return;
   __shared__ R st_re[32][33], st_im[32][33];
   __shared__ R inv_re[32], inv_im[32];
   ZLoadTriangle<R>(tri, 0, unit, r, st_re, st_im, inv_re, inv_im);
@@ -974,8 +974,8 @@ __global__ void ZGetrfLeafTrailingKernel(int m, int w, int n, R* a, long long ld
 template <typename R>
 __global__ void __launch_bounds__(256)
     ZPotrfLeafKernel(int upper, int n, R* a, long long lda, int* info, int info_base,
-                     int lanes, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                     int lanes, Guard guard) {
+  if (guard.Stops()) return;
   __shared__ R sr[32][33], si[32][33];  // A(i, j)
   __shared__ R row_r[32], row_i[32];
   __shared__ R s_rinv;
@@ -1051,8 +1051,8 @@ __global__ void __launch_bounds__(256)
 // complex product, the diagonal first reduced to its real part.
 template <typename R>
 __global__ void ZScaleTriangleKernel(int n, int lower, R beta, R* c, long long ldc,
-                                     const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                                     Guard guard) {
+  if (guard.Stops()) return;
   const long long total = static_cast<long long>(n) * n;
   for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
        e += static_cast<long long>(gridDim.x) * blockDim.x) {
@@ -1664,8 +1664,8 @@ template <typename R>
 void ZPotrf(bool recursive, bool upper, int n, R* a, int lda, int* info) {
   if (n == 0) return;
   Context& ctx = Ctx();
-  const int* saved = ctx.guard;
-  ctx.guard = info;
+  const Guard saved = ctx.guard;
+  ctx.guard = Guard{info};
   const int nb = 64;
   if (recursive || nb >= n) {
     ZPotrf2Rec<R>(upper, n, a, lda, info, 0);

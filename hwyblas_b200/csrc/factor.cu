@@ -88,8 +88,8 @@ __global__ void IamaxKernel(int n, const T* x, long long incx, T* part_v,
 template <typename T>
 __global__ void LaswpKernel(int n, T* a, long long lda, int i1, int i2,
                             int inc, int ix0, int incx, const int* ipiv,
-                            const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                            Guard guard) {
+  if (guard.Stops()) return;
   const int col = blockIdx.x * blockDim.x + threadIdx.x;
   if (col >= n) return;
   T* ac = a + col * lda;
@@ -120,8 +120,8 @@ constexpr int kLaswpCols = 64;   // columns per block
 template <typename T>
 __global__ void __launch_bounds__(256)
     LaswpPermKernel(int n, T* a, long long lda, int k1, int k2,
-                    const int* ipiv, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                    const int* ipiv, Guard guard) {
+  if (guard.Stops()) return;
   __shared__ int pos[kSwapTable], src[kSwapTable];
   __shared__ int hkey[kSwapHash], hfirst[kSwapHash], spiv[kSwapMax], sslot[kSwapMax];
   __shared__ int wsum[8];
@@ -663,8 +663,8 @@ __device__ bool CholLeaf(T* s, T* col, T* sinv, int upper, int c0, int n, int la
 template <typename T>
 __global__ void __launch_bounds__(kCholThreads)
     PotrfBlockKernel(int upper, int n, T* a, long long lda, int* info, int info_base, int lanes,
-                     const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                     Guard guard) {
+  if (guard.Stops()) return;
   __shared__ T s[kCholW * kCholLd];  // s[i][j], i >= j
   __shared__ T col[2 * kCholLeaf], sinv[kCholW];
   __shared__ int alive;

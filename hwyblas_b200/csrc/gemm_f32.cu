@@ -124,10 +124,10 @@ template <int WM, int WN, bool kPart, int ModeA, int ModeB>
 __global__ void __launch_bounds__(F32Tile<WM, WN>::kThreads, 512 / F32Tile<WM, WN>::kThreads)
     SgemmTileKernel(int m, int n, int k, float alpha, const float* a, long long lda,
                     const float* b, long long ldb, float beta, float* c, long long ldc, int part,
-                    const int* guard) {
+                    Guard guard) {
   using Cfg = F32Tile<WM, WN>;
   constexpr int BM = Cfg::kBM, BN = Cfg::kBN, SA = Cfg::kSA, SB = Cfg::kSB;
-  if (guard != nullptr && *guard != 0) return;
+  if (guard.Stops()) return;
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   // A tile wholly outside the triangle has nothing to do.
   if (kPart && (part == kLower ? m0 + BM - 1 < n0 : m0 > n0 + BN - 1)) return;

@@ -60,7 +60,7 @@ struct GemmParams {
   double* partial;
   int nchunks;
   int* timeout_flag;
-  const int* guard;
+  Guard guard;
 };
 
 // k range [*kb, *ke) that the reference multiplies for C(i, j) when an
@@ -251,7 +251,7 @@ __global__ void __maxnreg__(168)
                     const __grid_constant__ CUtensorMap tm_b, GemmParams p) {
   // kTriKind: 0 no triangular operand, 1 op(A) triangular, 2 op(B).
   constexpr bool kTri = kTriKind != 0, kTriA = kTriKind == 1, kTriB = kTriKind == 2;
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   // Persistent: CTA b computes tiles b, b + gridDim.x, ... The producer
   // streams the k-slices across tile boundaries (the stage counter gs runs
   // over all of the CTA's k-slices), so the next tile's loads overlap this
@@ -529,7 +529,7 @@ __global__ void __maxnreg__(168)
 // triangular operand's range for the element is skipped; chunk 0 still
 // applies beta, with a zero accumulator when its range is empty).
 __global__ void __launch_bounds__(256) DgemmSplitMergeKernel(GemmParams p) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   const long long total = static_cast<long long>(p.m) * p.n;
   const long long plane = total;
   for (long long e = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; e < total;
@@ -607,7 +607,7 @@ template <bool kTA, bool kTB, bool kPart>
 __global__ void __launch_bounds__(kSkThreads, kSkPerSm)
     DgemmShortKKernel(GemmParams p, const double* __restrict__ a, long long lda,
                       const double* __restrict__ b, long long ldb) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   extern __shared__ __align__(16) double sk_smem[];
   double* sA = sk_smem;                   // sA[q][i] (kTA: sA[i][q]) = op(A)(m0 + i, q)
   double* sB = sA + kSkK * kSkLdAB;       // sB[j][q] (kTB: sB[q][j]) = op(B)(q, n0 + j)
@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(kSkThreads, kSkPerSm)
 // bits), without its TMA pipeline whose fixed costs dominate tiny shapes.
 __global__ void __launch_bounds__(256)
     DgemmDirectKernel(GemmParams p, View<double> a, View<double> b) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   const int i = blockIdx.x * 32 + threadIdx.x % 32;
   const int j = blockIdx.y * 8 + threadIdx.x / 32;
   if (!InPart(p, i, j)) return;
@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(256)
 // sums in order.
 __global__ void __launch_bounds__(256)
     DgemmDirectChunkKernel(GemmParams p, View<double> a, View<double> b, int tpe) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   __shared__ double part[256];
   const int epb = 256 / tpe;
   const int e = threadIdx.x / tpe, ch = threadIdx.x % tpe;
@@ -886,7 +886,9 @@ __device__ __forceinline__ double SmallMerge(const GemmParams& p, int i, int j, 
 
 __global__ void __launch_bounds__(kSmThreads, 3)
     DgemmSmallKernel(GemmParams p, View<double> a, View<double> b, int S) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  // A stopped call skips the stores only: no thread leaves before those that read
+  // its slabs or, in a cluster, its CTA's sums.
+  const bool stopped = p.guard.Stops();
   extern __shared__ __align__(16) double sm_smem[];
   double* parts = sm_smem + 2 * kSmStage;  // [chunk / S][column][row]
   const int rank = blockIdx.x % S, tile = blockIdx.x / S;
@@ -941,7 +943,7 @@ __global__ void __launch_bounds__(kSmThreads, 3)
       const int i = wr * 16 + g + (e >> 1) * 8, j = wc * 8 + 2 * t + (e & 1);
       if (S > 1) {
         parts[part * kSmT * kSmT + j * kSmT + i] = acc[e];
-      } else if (m0 + i < p.m && n0 + j < p.n && InPart(p, m0 + i, n0 + j)) {
+      } else if (!stopped && m0 + i < p.m && n0 + j < p.n && InPart(p, m0 + i, n0 + j)) {
         p.c[m0 + i + (n0 + j) * p.ldc] = SmallMerge(p, m0 + i, n0 + j, 0, p.alpha * acc[e], 0.0);
       }
       acc[e] = 0.0;
@@ -953,7 +955,7 @@ __global__ void __launch_bounds__(kSmThreads, 3)
   cluster.sync();
   for (int e = rank * kSmThreads + threadIdx.x; e < kSmT * kSmT; e += S * kSmThreads) {
     const int i = m0 + e % kSmT, j = n0 + e / kSmT;
-    if (i >= p.m || j >= p.n || !InPart(p, i, j)) continue;
+    if (stopped || i >= p.m || j >= p.n || !InPart(p, i, j)) continue;
     double cv = 0.0;
 #pragma unroll 4
     for (int c = 0; c < p.nchunks; ++c)
@@ -991,8 +993,8 @@ __global__ void CanonicalCopyKernel(View<T> x, int rows, int cols, T* dst,
 
 template <typename T>
 __global__ void ScaleKernel(int m, int n, T beta, T* c, long long ldc,
-                            int part, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                            int part, Guard guard) {
+  if (guard.Stops()) return;
   const long long total = static_cast<long long>(m) * n;
   for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) +
                        threadIdx.x;

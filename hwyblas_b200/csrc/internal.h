@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <climits>
 #include <cstddef>
 #include <functional>
 #include <cstdint>
@@ -45,6 +46,24 @@ inline View<T> ColMajor(const T* p, long long ld, bool trans = false) {
   return v;
 }
 
+// The stop condition of a driver that ends at its first failure: kernels do
+// nothing once *info (INFO, 1-based) names a column up to `limit`. Every thread
+// of a launch must see the same answer, for the threads of a block and the blocks
+// of a cluster work together: a launch that runs beside the one that may write
+// *info has a limit below every value that can be written meanwhile, and what
+// lies up to the limit is final before it starts.
+struct Guard {
+  const int* info = nullptr;
+  int limit = INT_MAX;
+#ifdef __CUDACC__
+  __device__ __forceinline__ bool Stops() const {
+    if (info == nullptr) return false;
+    const int v = *info;
+    return v != 0 && v <= limit;
+  }
+#endif
+};
+
 struct Context {
   cudaStream_t stream = nullptr;
   cudaStream_t own_stream = nullptr;
@@ -58,9 +77,8 @@ struct Context {
   // to copy back for it; [1] where INFO is copied to.
   int* host_status = nullptr;
   int* wait_flag = nullptr;  // host_status[0] as the device sees it
-  // If non-null, kernels return at once while *guard != 0 (used by drivers
-  // that must stop after a failure, e.g. Cholesky's non-positive minor).
-  const int* guard = nullptr;
+  // The running driver's stop condition (Cholesky's non-positive minor).
+  Guard guard;
   int last_error = 0;
   // Workspace bank of the work being enqueued: 0 on the context's stream, 1
   // on the side stream (see OnSide), so that the two streams never share a

@@ -48,8 +48,8 @@ constexpr int kTrti2Threads = 256;
 // the old ones and its writes.
 template <typename T>
 __global__ void __launch_bounds__(kTrti2Threads)
-    Trti2Kernel(int n, T* a, long long lda, int upper, int unit, T* tmp, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+    Trti2Kernel(int n, T* a, long long lda, int upper, int unit, T* tmp, Guard guard) {
+  if (guard.Stops()) return;
   const auto A = [&](int i, int j) -> T& { return a[i + j * lda]; };
   for (int step = 0; step < n; ++step) {
     const int j = upper ? step : n - 1 - step;
@@ -102,8 +102,8 @@ __global__ void __launch_bounds__(kTrti2Threads)
 template <typename T>
 __global__ void __launch_bounds__(64)
     Trti2BlocksKernel(int n, int nb, T* a, long long lda, int upper, int unit, T* orig,
-                      const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                      Guard guard) {
+  if (guard.Stops()) return;
   __shared__ T s[64][65];
   const int j0 = blockIdx.x * nb, jb = min(nb, n - j0), t = threadIdx.x;
   T* blk = a + j0 + static_cast<long long>(j0) * lda;
@@ -216,8 +216,8 @@ __global__ void GetriGemvKernel(int n, int j, T* a, long long lda, const T* work
 // The same for all columns in one CTA (n small).
 template <typename T>
 __global__ void __launch_bounds__(1024)
-    GetriUnblockedKernel(int n, T* a, long long lda, T* work, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+    GetriUnblockedKernel(int n, T* a, long long lda, T* work, Guard guard) {
+  if (guard.Stops()) return;
   for (int j = n - 1; j >= 0; --j) {
     for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
       work[i] = a[i + j * lda];

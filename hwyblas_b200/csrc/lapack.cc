@@ -190,16 +190,16 @@ void Potrf2Rec(bool upper, int n, T* a, int lda, int* info, int col0) {
 template <typename T>
 void Potrf2(bool upper, int n, T* a, int lda, int* info) {
   Context& ctx = Ctx();
-  const int* saved = ctx.guard;
-  ctx.guard = info;
+  const Guard saved = ctx.guard;
+  ctx.guard = Guard{info};
   Potrf2Rec<T>(upper, n, a, lda, info, 0);
   ctx.guard = saved;
 }
 
 void PotrfPanel(bool upper, int n, double* a, int lda, int* info, int col0) {
   Context& ctx = Ctx();
-  const int* saved = ctx.guard;
-  ctx.guard = info;
+  const Guard saved = ctx.guard;
+  ctx.guard = Guard{info};
   Potrf2Rec(upper, n, a, lda, info, col0);
   ctx.guard = saved;
 }
@@ -213,7 +213,9 @@ void PotrfPanel(bool upper, int n, double* a, int lda, int* info, int col0) {
 // the context's stream does the rest. The side stream's step j waits for
 // the context stream's step j - 1; the context stream's step j waits for
 // the side stream's diagonal block j. Every element's operations are the
-// reference's.
+// reference's. The context stream's step j runs beside the factorization of
+// block j + 1, which may fail meanwhile: the reference has done step j by then, so
+// that step stops only for a failure up to block j.
 template <typename T>
 void Potrf(bool upper, int n, T* a, int lda, int* info) {
   if (n == 0) return;
@@ -223,8 +225,8 @@ void Potrf(bool upper, int n, T* a, int lda, int* info) {
     return;
   }
   Context& ctx = Ctx();
-  const int* saved = ctx.guard;
-  ctx.guard = info;
+  const Guard saved = ctx.guard;
+  ctx.guard = Guard{info};
   SideStream& side = Side();
   const cudaStream_t main = ctx.stream;
   const cudaStream_t look = side.ok ? side.stream : main;
@@ -288,7 +290,9 @@ void Potrf(bool upper, int n, T* a, int lda, int* info) {
     });
     if (rest > next) {
       ctx.sm_cap = cap;
+      ctx.guard.limit = j + jb;
       beside(j, jb, j + jb + next, rest - next);
+      ctx.guard.limit = INT_MAX;
       ctx.sm_cap = 0;
     }
   }

@@ -46,8 +46,8 @@ __device__ __forceinline__ void TriRangeF(int tri, int m, int n, int k, int i, i
 // reference skips the micro-tile (src/gemm-inl.h:202-209).
 __global__ void __launch_bounds__(256)
     SgemmKernel(int m, int n, int k, float alpha, View<float> a, View<float> b,
-                float beta, float* c, long long ldc, int tri, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                float beta, float* c, long long ldc, int tri, Guard guard) {
+  if (guard.Stops()) return;
   __shared__ float sa[kSK][kSB + 4];
   __shared__ float sb[kSK][kSB + 4];
   const int m0 = blockIdx.x * kSB, n0 = blockIdx.y * kSB;
@@ -144,8 +144,8 @@ constexpr int kBaseThreads = 256, kBaseRows = 2 * kBaseThreads / 32, kBaseW = 64
 template <typename T>
 __global__ void __launch_bounds__(kBaseThreads)
     TrsmBaseKernel(View<T> tri, int lower, int unit, int r, int rows, T* x,
-                   long long xs_row, long long xs_col, const int* guard) {
-  if (guard != nullptr && *guard != 0) return;
+                   long long xs_row, long long xs_col, Guard guard) {
+  if (guard.Stops()) return;
   constexpr int ld = kBaseW + 1;
   __shared__ T st[kBaseW * ld];  // st[s][u] = T(col(s), col(u)) in solve order, s < u
   __shared__ T sinv[kBaseW];
@@ -256,7 +256,7 @@ struct TrsmClusterArgs {
   int lower, unit, r, other;
   T* x;         // element (row, right-hand side) at row * xs + rhs * xr
   long long xs, xr;
-  const int* guard;
+  Guard guard;
 };
 
 __device__ __forceinline__ void TcBarrier() {
@@ -344,7 +344,7 @@ __device__ __forceinline__ void TcTile(const T* a, const T* x, T* c, long long x
 
 template <typename T>
 __global__ void __launch_bounds__(kTcThreads) TrsmClusterKernel(TrsmClusterArgs<T> p) {
-  if (p.guard != nullptr && *p.guard != 0) return;
+  if (p.guard.Stops()) return;
   extern __shared__ __align__(16) unsigned char tc_smem[];
   T* tri[2] = {reinterpret_cast<T*>(tc_smem), reinterpret_cast<T*>(tc_smem) + 32 * 33};
   T* strips = tri[1] + 32 * 33;

@@ -28,6 +28,34 @@ def test_potrf_blocks(hb, orc, p, uplo, n, bad):
 
 
 @pytest.mark.parametrize("p", ["d", "s"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("n", [700, 1500, 3000])
+@pytest.mark.parametrize("block", ["second", "middle", "last"])
+def test_potrf_fails_beside_an_update(hb, orc, p, uplo, n, block):
+    """The block that fails is factored beside the rest of the step before it, which
+    the reference has done by then: A and INFO are its bits, whatever the two
+    streams' timing (hence the repetitions), and POSV leaves B alone."""
+    rng = np.random.default_rng(n)
+    g = rand(rng, n, n)
+    a = (g @ g.T / n + np.eye(n)).astype(REAL[p])
+    i = 64 * {"second": 1, "middle": n // 128, "last": (n - 1) // 64}[block] + 17
+    a[i, i] = -1.0
+    a = np.asfortranarray(a)
+    want = a.copy(order="F")
+    assert getattr(orc, f"{p}potrf")(uplo, n, want, n) == i + 1
+    b = rand(rng, n, 2, REAL[p])
+    for trial in range(10):
+        got, x = a.copy(order="F"), b.copy(order="F")
+        if trial % 2:
+            info = getattr(hb, f"{p}posv")(uplo, n, 2, got, n, x, n)
+        else:
+            info = getattr(hb, f"{p}potrf")(uplo, n, got, n)
+        assert info == i + 1
+        assert same_bits(got, want), (trial, first_diff(got, want))
+        assert same_bits(x, b)
+
+
+@pytest.mark.parametrize("p", ["d", "s"])
 @pytest.mark.parametrize("side", ["L", "R"])
 @pytest.mark.parametrize("uplo", ["L", "U"])
 @pytest.mark.parametrize("trans", ["N", "T"])
