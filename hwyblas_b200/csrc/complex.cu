@@ -1392,9 +1392,8 @@ void ZGetrfLeaf(int m, int n, R* a, int lda, int* ipiv, int* info, int info_base
   }
   const int rows = (m + P - 1) / P;
   const size_t smem = 2 * sizeof(R) * static_cast<size_t>(w) * rows;
-  static bool configured = false;
-  static int max_cluster = 0;
-  if (!configured) {
+  static PerDevice<int> clusters;
+  const int max_cluster = clusters.Get([] {
     const int smem_max = static_cast<int>(2 * sizeof(R) * kZLeafW * kZLeafMaxRows);
     cudaFuncSetAttribute(ZGetrfLeafKernel<R, false>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
@@ -1420,9 +1419,8 @@ void ZGetrfLeaf(int m, int n, R* a, int lda, int* ipiv, int* info, int info_base
       cudaGetLastError();
       size = 0;
     }
-    max_cluster = std::min(size, 16);
-    configured = true;
-  }
+    return std::min(size, 16);
+  });
   ZLeafArgs<R> args;
   args.m = m;
   args.w = w;

@@ -701,14 +701,11 @@ bool LaunchOzaki(const CUtensorMap& ma, const CUtensorMap& mb,
                  const OzakiParams& p, cudaStream_t st) {
   using Cfg = OzakiCfg<S, L0, L1, KB>;
   auto* kernel = OzakiGemmKernel<S, L0, L1, KB, kFinal, kReadW>;
-  static bool configured = false;
-  if (!configured) {
-    if (Failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    Cfg::kSmem),
-               "ozaki smem attribute"))
-      return false;
-    configured = true;
-  }
+  static PerDevice<cudaError_t> attr;
+  const auto set = [kernel] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+  };
+  if (Failed(attr.Get(set), "ozaki smem attribute")) return false;
   const long long tiles =
       static_cast<long long>((p.m + kEBM - 1) / kEBM) * ((p.n + kEBN - 1) / kEBN);
   cudaEvent_t t0 = KernelTimerStart(kFamilyOzakiGemm, st);

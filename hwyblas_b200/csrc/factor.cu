@@ -813,9 +813,7 @@ void GetrfLeaf(int m, int n, T* a, int lda, int* ipiv, int* info, int info_base,
   const size_t smem = static_cast<size_t>(w) * R * sizeof(T);
   const int smem_max = kLeafW * kLeafMaxRows * static_cast<int>(sizeof(T));
   const int smem_wide = 32 * kWideLeafRows * static_cast<int>(sizeof(T));
-  static int max_cluster = 0, max_cluster_wide = 0;
-  static bool configured = false;
-  auto cluster_limit = [](const void* fn, int smem_bytes) {
+  const auto cluster_limit = [](const void* fn, int smem_bytes) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kLeafMaxCluster);
     cfg.blockDim = dim3(kLeafThreads);
@@ -834,23 +832,25 @@ void GetrfLeaf(int m, int n, T* a, int lda, int* ipiv, int* info, int info_base,
     }
     return std::min(size, kLeafMaxCluster);
   };
-  if (!configured) {
+  static PerDevice<int> clusters, clusters_wide;
+  const int max_cluster = clusters.Get([&] {
     cudaFuncSetAttribute(GetrfLeafPanelKernel<T, false, kLeafW>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     cudaFuncSetAttribute(GetrfLeafPanelKernel<T, true, kLeafW>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max);
     cudaFuncSetAttribute(GetrfLeafPanelKernel<T, true, kLeafW>,
                          cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return cluster_limit(
+        reinterpret_cast<const void*>(GetrfLeafPanelKernel<T, true, kLeafW>), smem_max);
+  });
+  const int max_cluster_wide = clusters_wide.Get([&] {
     cudaFuncSetAttribute(GetrfLeafPanelKernel<T, true, 32>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, smem_wide);
     cudaFuncSetAttribute(GetrfLeafPanelKernel<T, true, 32>,
                          cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    max_cluster = cluster_limit(
-        reinterpret_cast<const void*>(GetrfLeafPanelKernel<T, true, kLeafW>), smem_max);
-    max_cluster_wide = cluster_limit(
+    return cluster_limit(
         reinterpret_cast<const void*>(GetrfLeafPanelKernel<T, true, 32>), smem_wide);
-    configured = true;
-  }
+  });
   if (wide && P > max_cluster_wide) {
     Failed(cudaErrorInvalidValue, "getrf wide leaf cluster");
     return;

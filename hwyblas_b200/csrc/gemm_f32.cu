@@ -240,10 +240,12 @@ struct TileCall {
 template <int WM, int WN, bool kPart, int ModeA, int ModeB>
 void LaunchModes(const TileCall& t) {
   using Cfg = F32Tile<WM, WN>;
-  static const cudaError_t attr =
-      cudaFuncSetAttribute(SgemmTileKernel<WM, WN, kPart, ModeA, ModeB>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
-  if (Failed(attr, "sgemm attributes")) return;
+  static PerDevice<cudaError_t> attr;
+  const auto set = [] {
+    return cudaFuncSetAttribute(SgemmTileKernel<WM, WN, kPart, ModeA, ModeB>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+  };
+  if (Failed(attr.Get(set), "sgemm attributes")) return;
   const dim3 grid((t.m + Cfg::kBM - 1) / Cfg::kBM, (t.n + Cfg::kBN - 1) / Cfg::kBN);
   SgemmTileKernel<WM, WN, kPart, ModeA, ModeB>
       <<<grid, Cfg::kThreads, Cfg::kSmem, Ctx().stream>>>(

@@ -1110,10 +1110,13 @@ bool SmallTakes(int m, int n, int k, bool small, bool short_k) {
 void DgemmSmall(int m, int n, int k, double alpha, View<double> a, View<double> b, double beta,
                 double* c, int ldc, Part part) {
   Context& ctx = Ctx();
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      DgemmSmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-      static_cast<int>(sizeof(double)) * (2 * kSmStage + kSmMaxParts * kSmT * kSmT));
-  if (Failed(attr, "dgemm small attributes")) return;
+  static PerDevice<cudaError_t> attr;
+  const auto set = [] {
+    return cudaFuncSetAttribute(
+        DgemmSmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        static_cast<int>(sizeof(double)) * (2 * kSmStage + kSmMaxParts * kSmT * kSmT));
+  };
+  if (Failed(attr.Get(set), "dgemm small attributes")) return;
   GemmParams p = {};
   p.m = m;
   p.n = n;
@@ -1190,8 +1193,8 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
     }
   }
   if (short_k) {
-    static bool sk_configured = false;
-    if (!sk_configured) {
+    static PerDevice<bool> configured;
+    configured.Get([] {
       const auto set = [](const void* f) {
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSkSmemBytes);
       };
@@ -1203,8 +1206,8 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
       set(reinterpret_cast<const void*>(DgemmShortKKernel<false, true, true>));
       set(reinterpret_cast<const void*>(DgemmShortKKernel<true, false, true>));
       set(reinterpret_cast<const void*>(DgemmShortKKernel<true, true, true>));
-      sk_configured = true;
-    }
+      return true;
+    });
     GemmParams p;
     p.m = m;
     p.n = n;
@@ -1271,8 +1274,8 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
   p.guard = ctx.guard;
   const long long tiles =
       static_cast<long long>((m + kBM - 1) / kBM) * ((n + kBN - 1) / kBN);
-  static bool configured = false;
-  if (!configured) {
+  static PerDevice<bool> configured;
+  configured.Get([] {
     const auto set = [](const void* f) {
       cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     };
@@ -1282,8 +1285,8 @@ void Dgemm(int m, int n, int k, double alpha, View<double> a, View<double> b,
     set(reinterpret_cast<const void*>(DgemmDmmaKernel<0, true>));
     set(reinterpret_cast<const void*>(DgemmDmmaKernel<1, true>));
     set(reinterpret_cast<const void*>(DgemmDmmaKernel<2, true>));
-    configured = true;
-  }
+    return true;
+  });
   const int tri_kind =
       tri == kTriNone ? 0 : (tri == kTriALower || tri == kTriAUpper) ? 1 : 2;
   // Few tiles and a long k (a narrow product: TRTRI's and GETRI's block

@@ -109,6 +109,35 @@ Context& Ctx();
 // Grows and returns slot `slot` of the thread's device workspace (at least
 // `bytes`, 256-byte aligned). Valid until the next call with the same slot.
 void* Workspace(int slot, size_t bytes);
+
+// What has to be set up or asked once a device, not once a process (function
+// attributes and occupancies are a device's): Get(f) is f() at its first use on the
+// calling thread's device, and the same value from then on. Two threads may both
+// call f for a device; it gives them the same.
+template <typename T>
+class PerDevice {
+ public:
+  template <typename F>
+  T Get(F f) {
+    const int device = Ctx().device;
+    if (device < 0 || device >= kMaxDevices) return f();
+    Slot& s = slots_[device];
+    if (!s.known.load(std::memory_order_acquire)) {
+      s.value.store(f(), std::memory_order_relaxed);
+      s.known.store(true, std::memory_order_release);
+    }
+    return s.value.load(std::memory_order_relaxed);
+  }
+
+ private:
+  static constexpr int kMaxDevices = 64;
+  struct Slot {
+    std::atomic<T> value{};
+    std::atomic<bool> known{false};
+  };
+  Slot slots_[kMaxDevices];
+};
+
 enum WorkspaceSlot : int {
   kWsStageA = 0,   // host-pointer staging
   kWsStageB = 1,

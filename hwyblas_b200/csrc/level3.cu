@@ -461,15 +461,16 @@ __global__ void __launch_bounds__(kTcThreads) TrsmClusterKernel(TrsmClusterArgs<
 template <typename T>
 bool TrsmCluster(bool left, View<T> tri, bool lower, bool unit, int r, int other, T* b, int ldb) {
   Context& ctx = Ctx();
-  static const bool ready = [] {
+  static PerDevice<bool> ready;
+  const auto set = [] {
     const bool ok =
         cudaFuncSetAttribute(reinterpret_cast<const void*>(TrsmClusterKernel<T>),
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              TcSmem<T>()) == cudaSuccess;
     if (!ok) cudaGetLastError();
     return ok;
-  }();
-  if (!ready) return false;
+  };
+  if (!ready.Get(set)) return false;
   TrsmClusterArgs<T> a;
   a.tri = tri;
   if (!left) std::swap(a.tri.rs, a.tri.cs);

@@ -897,7 +897,8 @@ bool LaunchPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info
   PanelArgs<T> args;
   int ctas = 0;
   if (n < 1 || n > kPanelW || m < n) return false;
-  static const int max_cluster = [] {
+  static PerDevice<int> clusters;
+  const int max_cluster = clusters.Get([] {
     const void* fn = reinterpret_cast<const void*>(GetrfPanelKernel<T>);
     if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(kPanelSmemMax)) != cudaSuccess ||
@@ -923,7 +924,7 @@ bool LaunchPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info
       size = 1;
     }
     return std::min(size, kPanelCtas);
-  }();
+  });
   // Beside a capped trailing update a cluster of at most 8 CTAs finds its SMs
   // in one GPC soonest; larger panels take what they need.
   if (!PanelShape<T>(m, n, std::min(max_cluster, 8), &ctas, &args.R) &&
@@ -964,9 +965,12 @@ template <typename T>
 void LaunchSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, const int* moves) {
   const int blocks = (left + kSwapCols - 1) / kSwapCols + (nc + kSwapCols - 1) / kSwapCols;
   if (blocks == 0) return;
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      PanelSwapTrsmKernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SwapSmem<T>());
-  if (Failed(attr, "panel interchanges attributes")) return;
+  static PerDevice<cudaError_t> attr;
+  const auto set = [] {
+    return cudaFuncSetAttribute(PanelSwapTrsmKernel<T>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, SwapSmem<T>());
+  };
+  if (Failed(attr.Get(set), "panel interchanges attributes")) return;
   SwapArgs<T> args;
   args.jb = jb;
   args.left = left;

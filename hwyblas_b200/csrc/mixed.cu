@@ -874,12 +874,11 @@ void InvertDiagBlocks(int n, const double* w, long long ldw, bool lower, bool un
                       double* inv) {
   const int nblk = (n + kTb - 1) / kTb;
   const int smem = 2 * kTb * (kTb + 1) * static_cast<int>(sizeof(double));
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(InvertDiagBlocksKernel,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    configured = true;
-  }
+  static PerDevice<cudaError_t> attr;
+  attr.Get([smem] {
+    return cudaFuncSetAttribute(InvertDiagBlocksKernel,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  });
   InvertDiagBlocksKernel<<<nblk, kTb, smem, Ctx().stream>>>(n, w, ldw, lower ? 1 : 0,
                                                             unit ? 1 : 0, inv);
   CountLaunch();
@@ -887,12 +886,12 @@ void InvertDiagBlocks(int n, const double* w, long long ldw, bool lower, bool un
 }
 
 void PermFromPivots(int n, const int* ipiv, int* perm) {
-  static bool configured = false;
-  if (!configured) {
-    cudaFuncSetAttribute(PermFromPivotsKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         2 * kPermSmem * static_cast<int>(sizeof(int)));
-    configured = true;
-  }
+  static PerDevice<cudaError_t> attr;
+  attr.Get([] {
+    return cudaFuncSetAttribute(PermFromPivotsKernel,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                2 * kPermSmem * static_cast<int>(sizeof(int)));
+  });
   const size_t smem = n <= kPermSmem ? 2 * sizeof(int) * n : 0;
   PermFromPivotsKernel<<<1, 1024, smem, Ctx().stream>>>(n, ipiv, perm);
   CountLaunch();
@@ -905,8 +904,8 @@ void PermFromPivots(int n, const int* ipiv, int* perm) {
 bool ChainTrsv(bool lower, int n, int nrhs, const double* w, long long ldw,
                const double* inv, double* x, long long ldx, unsigned int* flags) {
   Context& ctx = Ctx();
-  static int capacity = -1;
-  if (capacity < 0) {
+  static PerDevice<int> resident;
+  const int capacity = resident.Get([&ctx] {
     cudaFuncSetAttribute(ChainTrsvKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kChainSmem);
     cudaFuncSetAttribute(ChainTrsvKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -916,9 +915,9 @@ bool ChainTrsv(bool lower, int n, int nrhs, const double* w, long long ldw,
                                                   kChainSmem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&up, ChainTrsvKernel<false>, kChainThreads,
                                                   kChainSmem);
-    capacity = ctx.num_sms * std::min(lo, up);
     cudaGetLastError();
-  }
+    return ctx.num_sms * std::min(lo, up);
+  });
   const int nblk = (n + kTb - 1) / kTb;
   const int pmin = (nblk + kChainSlots - 1) / kChainSlots;
   if (capacity <= 0 || pmin > capacity) return false;
@@ -952,8 +951,8 @@ void BlockTrsv(bool lower, int n, int nrhs, const double* w, long long ldw,
                unsigned int* flags) {
   if (ChainTrsv(lower, n, nrhs, w, ldw, inv, x, ldx, flags)) return;
   Context& ctx = Ctx();
-  static int grid = 0;
-  if (grid == 0) {
+  static PerDevice<int> resident;
+  const int grid = resident.Get([&ctx] {
     cudaFuncSetAttribute(BlockTrsvKernel<true>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, kTrsvSmem);
     cudaFuncSetAttribute(BlockTrsvKernel<false>,
@@ -963,8 +962,8 @@ void BlockTrsv(bool lower, int n, int nrhs, const double* w, long long ldw,
                                                   kTrsvThreads, kTrsvSmem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&up, BlockTrsvKernel<false>,
                                                   kTrsvThreads, kTrsvSmem);
-    grid = ctx.num_sms * std::max(1, std::min({lo, up, 2}));
-  }
+    return ctx.num_sms * std::max(1, std::min({lo, up, 2}));
+  });
   int nn = n;
   long long lw = ldw, lx = ldx;
   int* flag = ctx.wait_flag;

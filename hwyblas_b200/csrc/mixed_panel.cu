@@ -723,8 +723,8 @@ __global__ void __launch_bounds__(kTnThreads, 1) TournamentLeafKernel(TnArgs p) 
 
 // Co-resident CTAs of the tournament leaf (one a SM with its shared memory).
 int TournamentCapacity() {
-  static int capacity = -1;
-  if (capacity < 0) {
+  static PerDevice<int> capacity;
+  return capacity.Get([] {
     cudaFuncSetAttribute(TournamentLeafKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          kTnSmem);
     int per_sm = 0;
@@ -733,9 +733,8 @@ int TournamentCapacity() {
       cudaGetLastError();
       per_sm = 0;
     }
-    capacity = std::min(Ctx().num_sms * per_sm, kTnMaxNodes - 12);
-  }
-  return capacity;
+    return std::min(Ctx().num_sms * per_sm, kTnMaxNodes - 12);
+  });
 }
 
 bool TournamentFits(int m) {

@@ -101,14 +101,11 @@ template <int kN>
 double I8PeakTops() {
   Context& ctx = Ctx();
   auto* kernel = I8PeakKernel<kN>;
-  static bool configured = false;
-  if (!configured) {
-    if (Failed(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    kProbeSmem),
-               "int8 peak probe smem"))
-      return 0.0;
-    configured = true;
-  }
+  static PerDevice<cudaError_t> attr;
+  const auto set = [kernel] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kProbeSmem);
+  };
+  if (Failed(attr.Get(set), "int8 peak probe smem")) return 0.0;
   const int iters = 20000;
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
