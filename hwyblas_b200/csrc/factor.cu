@@ -919,6 +919,7 @@ unsigned int SetLeafWaitLimit(unsigned int polls) {
   cudaMemcpyFromSymbol(&prev, g_leaf_poll_limit, sizeof(prev));
   const unsigned int v = polls == 0 ? kMaxPolls : polls;
   Failed(cudaMemcpyToSymbol(g_leaf_poll_limit, &v, sizeof(v)), "leaf wait limit");
+  SetPanelWaitLimit(polls);
   return prev;
 }
 

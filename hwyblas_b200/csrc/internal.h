@@ -293,8 +293,9 @@ bool ZGetrfPanel(int m, int n, R* a, int lda, int* ipiv, int ipiv_add, int* info
 template <typename R>
 void ZPanelSwapTrsm(int j, int jb, int left, int c0, int nc, R* a, int lda, const int* moves);
 // Sets the poll limit of the cooperative leaf's exchange on the current
-// device (0: the default); returns the previous one.
+// device (0: the default); returns the previous one. Sets the panel's too.
 unsigned int SetLeafWaitLimit(unsigned int polls);
+void SetPanelWaitLimit(unsigned int polls);  // lu_panel.cu; 0: the default
 // Potrf2 of a block of n <= 64 columns on device: sets *info to info_base + j + 1
 // and stops at the first non-positive (or NaN) diagonal, if *info is still 0.
 template <typename T>

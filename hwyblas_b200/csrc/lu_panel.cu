@@ -26,6 +26,7 @@
 // (Cx<float>, Cx<double>): the complex LU has the same recursion and leaves, on
 // |re| + |im| and the complex AXPY, product and quotient of complex.cuh.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 
 #include "complex.cuh"
@@ -46,9 +47,14 @@ template <typename T>
 constexpr int kPanelThreads = sizeof(T) == 16 ? 256 : 512;
 constexpr int kPanelLeast = 256;   // threads at least: the solves share all warps
 constexpr int kPanelCtas = 16;
-// Polls of a wait for the other CTAs' candidates, each suspended for at most
-// about 1 us (spinning warps slow the others down): far above any real wait.
-constexpr uint32_t kPanelPolls = 1u << 20;
+// Polls of a wait for the other CTAs' candidates, each asleep for at most 4 us
+// (whatever time is asked for; spinning warps slow the others down): about a second,
+// far above any real wait.
+constexpr uint32_t kPanelPolls = 1u << 18;
+// A limit set by hwyblas_set_leaf_wait_limit, 0: none. It counts polls that do not
+// sleep, in an instantiation of its own (kSpin): chosen at run time, the two polls
+// cost 8 % of a panel.
+std::atomic<uint32_t> g_panel_polls{0};
 
 template <typename R>
 struct __align__(2 * sizeof(R)) Cx {
@@ -182,6 +188,7 @@ struct PanelArgs {
   int* info;
   int info_base;
   int* moves;  // count, unused, then (position, row) of every row that moved
+  uint32_t polls;  // a wait's limit
   int* timeout_flag;
 };
 
@@ -239,16 +246,63 @@ template <typename R>
 __device__ __forceinline__ Cx<R> LoadRemote(uint32_t addr, Cx<R>) {
   return Cx<R>{LoadRemote(addr, R(0)), LoadRemote(addr + sizeof(R), R(0))};
 }
+template <bool kSpin>
 __device__ __forceinline__ bool MbarTest(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(SmemAddr(bar)), "r"(parity), "r"(1000u)
-      : "memory");
+  if constexpr (kSpin)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(SmemAddr(bar)), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(SmemAddr(bar)), "r"(parity)
+        : "memory");
   return ok != 0;
+}
+// The wait of a panel for phase `parity`; false (and the flags set) if it gives up.
+template <bool kSpin>
+__device__ __forceinline__ bool PanelWait(uint64_t* bar, uint32_t parity, uint32_t limit,
+                                          int* timeout_flag, int* quit) {
+  for (uint32_t polls = 0; !MbarTest<kSpin>(bar, parity);) {
+    if (++polls >= limit) {
+      atomicExch(timeout_flag, 1);
+      *quit = 1;
+      return false;
+    }
+  }
+  return true;
+}
+// Waits for the messages that are still on their way to a CTA that gave up: an
+// mbarrier takes those of the columns of one parity, `bytes` from every CTA a
+// column. sent[p]: the columns that CTA p has sent; armed: those this CTA has
+// armed. The last armed column's phase is given the bytes that nobody will
+// send, a later one (which the faster CTAs may have reached) is armed with the
+// bytes that were sent.
+__device__ void PanelDrain(uint64_t* bar, int parity, int armed, const int* sent, int P,
+                           uint32_t bytes, int* timeout_flag, int* quit) {
+  int c = armed > parity ? armed - 1 - ((armed - 1 - parity) & 1) : parity;
+  for (;; c += 2) {
+    int n = 0;
+    for (int p = 0; p < P; ++p) n += sent[p] > c;
+    if (n == 0) return;
+    if (c >= armed) {
+      MbarArriveExpectTx(bar, n * bytes);
+    } else if (n < P) {
+      asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(
+                       SmemAddr(bar)),
+                   "r"((P - n) * bytes)
+                   : "memory");
+    }
+    if (!PanelWait<false>(bar, (c >> 1) & 1, kPanelPolls, timeout_flag, quit)) return;
+  }
 }
 __device__ __forceinline__ void ClusterBarrier() {
   asm volatile(
@@ -473,7 +527,7 @@ __device__ __forceinline__ void PanelUpdateDmma(const double* l, double* x, int 
   }
 }
 
-template <typename T>
+template <typename T, bool kSpin>
 __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T> p) {
   extern __shared__ __align__(16) unsigned char panel_smem[];
   const int P = gridDim.x, cta = blockIdx.x, R = p.R, RS = p.S, w = p.w;
@@ -487,12 +541,18 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
   __shared__ int s_wpos[2][kPanelThreads<T> / 32];
   __shared__ int s_place[kPanelW], s_pos[kPanelThreads<T>], s_op[7][4];
   __shared__ __align__(8) uint64_t s_bar[2], s_rbar[2];
-  __shared__ int s_ops;
+  // s_quit: whether a wait of an even, an odd column gave up. Read behind the next
+  // column's barrier, which the other column's waits come after.
+  __shared__ int s_ops, s_sent[kPanelCtas], s_quit[2];
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, nwarps = blockDim.x / 32;
   const int place = cta * R + tid;
   const bool valid = tid < R && place < p.m;
   int pos = place;
 
+  if (tid < kPanelCtas) s_sent[tid] = w;
+  if (tid < 2) s_quit[tid] = 0;
+  // Pivots that stay in range if the panel ends early.
+  if (cta == 0 && tid < w) p.ipiv[tid] = tid + 1 + p.ipiv_add;
   if (tid == 0) {
     MbarInit(&s_bar[0], 1);
     MbarInit(&s_bar[1], 1);
@@ -536,9 +596,12 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
   if (P > 1) ClusterBarrier();
   else __syncthreads();
 
-  // A wait that gives up: the CTA skips the rest but keeps taking part in the
-  // cluster's barriers, so that no CTA exits while others read its rows.
+  // A wait that gives up (timed_out, a thread's own) ends the panel for its CTA at
+  // the next block barrier, where all threads learn of it (alive): it arms no more
+  // mbarriers and sends no more candidates, but takes part in the cluster's
+  // barriers and stays until nothing is on its way to it.
   bool timed_out = false, alive = true;
+  int armed = 0, sent = 0;  // columns that thread 0 has armed, that the CTA has sent
   for (int op = 0; op < s_ops; ++op) {
     const int c0 = s_op[op][1], n1 = s_op[op][2], n2 = s_op[op][3];
     if (s_op[op][0] != 0) {
@@ -547,9 +610,10 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
       for (int k = 0; k < kPanelLeaf; ++k)
         x[k] = valid && k < n1 ? S[(c0 + k) * RS + tid] : Zero<T>();
 #pragma unroll 1
-      for (int j = 0; j < n1; ++j) {
+      for (int j = 0; alive && j < n1; ++j) {
         const int jc = c0 + j, par = jc & 1;
-        if (P > 1 && tid == 0) {
+        if (P > 1 && tid == 0 && !timed_out) {
+          armed = jc + 1;
           MbarArriveExpectTx(&s_bar[par], P * static_cast<uint32_t>(sizeof(PanelSlot<T>)));
           MbarArriveExpectTx(&s_rbar[par], P * static_cast<uint32_t>(sizeof(T)));
         }
@@ -564,9 +628,15 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
           s_wpos[par][warp] = pos;
         }
         __syncthreads();
+        const unsigned long long wkey = lane < nwarps ? s_wkey[par][lane] : 0ull;
+        const int wpos = lane < nwarps ? s_wpos[par][lane] : 0x7fffffff;
+        if (s_quit[par ^ 1] != 0) {
+          alive = false;
+          break;
+        }
+        sent = jc + 1;
         // The block's, found by every warp; the warp that holds the row sends it.
-        const int cbest = WarpBest<kWideKey<T>>(lane < nwarps ? s_wkey[par][lane] : 0ull,
-                                      lane < nwarps ? s_wpos[par][lane] : 0x7fffffff);
+        const int cbest = WarpBest<kWideKey<T>>(wkey, wpos);
         if (warp == cbest) {
           if (lane == wbest) {
             own->key = key;
@@ -597,15 +667,8 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
         }
         int at = 2 * kPanelCtas, from = 0;  // the winner's slot
         if (P > 1) {
-          // After a wait that gave up the columns run on without waiting, to the
-          // leaf's end, where the block leaves together.
-          for (uint32_t polls = 0;
-               !timed_out && !MbarTest(&s_bar[par], (jc >> 1) & 1);) {
-            if (++polls >= kPanelPolls) {
-              atomicExch(p.timeout_flag, 1);
-              timed_out = true;
-            }
-          }
+          timed_out =
+              !PanelWait<kSpin>(&s_bar[par], (jc >> 1) & 1, p.polls, p.timeout_flag, &s_quit[par]);
           const PanelSlot<T>* slot = slots + par * kPanelCtas + lane;
           from = WarpBest<kWideKey<T>>(lane < P ? slot->key : 0ull, lane < P ? slot->pos : 0x7fffffff);
           at = par * kPanelCtas + (from & (kPanelCtas - 1));
@@ -616,7 +679,7 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
         const int piv = win->pos;
         const T pivot = win->row[0];
         if (tid < n1 - j) prow[jc * kPanelLd<T> + jc + tid] = win->row[tid];
-        if (tid == 32) {
+        if (tid == 32 && !timed_out) {
           s_place[jc] = win->place;
           if (cta == 0) {
             p.ipiv[jc] = piv + 1 + p.ipiv_add;
@@ -626,12 +689,9 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
         // A zero pivot is at position jc already.
         if (pos == piv) pos = jc;
         else if (pos == jc) pos = piv;
-        for (uint32_t polls = 0; P > 1 && !timed_out && !MbarTest(&s_rbar[par], (jc >> 1) & 1);) {
-          if (++polls >= kPanelPolls) {
-            atomicExch(p.timeout_flag, 1);
-            timed_out = true;
-          }
-        }
+        if (P > 1 && !timed_out)
+          timed_out =
+              !PanelWait<kSpin>(&s_rbar[par], (jc >> 1) & 1, p.polls, p.timeout_flag, &s_quit[par]);
         if (valid && pos > jc) {
           // The column below the pivot times its reciprocal (divided if the
           // pivot is below the safe minimum, kept if it is zero), then the
@@ -706,7 +766,7 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
       __syncthreads();
     }
   }
-  if (!__syncthreads_or(timed_out) && alive) {
+  if (alive) {
 #pragma unroll 4
     for (int i = tid; i < (w - cta + P - 1) / P * kPanelW; i += blockDim.x) {
       const int r = i % kPanelW, c = cta + i / kPanelW * P;
@@ -723,8 +783,23 @@ __global__ void __launch_bounds__(kPanelThreads<T>) GetrfPanelKernel(PanelArgs<T
       p.moves[3 + 2 * e] = place;
     }
   }
-  // No CTA exits while another may read or write its shared memory.
-  if (P > 1) ClusterBarrier();
+  if (P > 1) {
+    if (!alive && tid < P)
+      asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(
+                       MapRank(SmemAddr(&s_sent[cta]), tid)),
+                   "r"(sent)
+                   : "memory");
+    // No CTA exits while another may read its rows or write its counts; one whose
+    // waits all ended has received every candidate sent to it.
+    ClusterBarrier();
+    if (!alive && tid == 0) {
+      for (int par = 0; par < 2; ++par) {
+        PanelDrain(&s_bar[par], par, armed, s_sent, P, sizeof(PanelSlot<T>), p.timeout_flag,
+                   s_quit);
+        PanelDrain(&s_rbar[par], par, armed, s_sent, P, sizeof(T), p.timeout_flag, s_quit);
+      }
+    }
+  }
 }
 
 // Stride of a CTA's R rows in shared memory: 4 modulo 16, so that the tensor pipe's
@@ -899,13 +974,15 @@ bool LaunchPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info
   if (n < 1 || n > kPanelW || m < n) return false;
   static PerDevice<int> clusters;
   const int max_cluster = clusters.Get([] {
-    const void* fn = reinterpret_cast<const void*>(GetrfPanelKernel<T>);
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(kPanelSmemMax)) != cudaSuccess ||
-        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-            cudaSuccess) {
-      cudaGetLastError();
-      return 0;
+    const void* fn = reinterpret_cast<const void*>(GetrfPanelKernel<T, false>);
+    for (const void* f : {fn, reinterpret_cast<const void*>(GetrfPanelKernel<T, true>)}) {
+      if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(kPanelSmemMax)) != cudaSuccess ||
+          cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+              cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+      }
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kPanelCtas);
@@ -941,6 +1018,8 @@ bool LaunchPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info
   args.info = info;
   args.info_base = info_base;
   args.moves = moves;
+  const uint32_t limit = g_panel_polls.load(std::memory_order_relaxed);
+  args.polls = limit != 0 ? limit : kPanelPolls;
   args.timeout_flag = ctx.wait_flag;
   cudaEvent_t t0 = KernelTimerStart(kFamilyLuLeaf, ctx.stream);
   cudaLaunchConfig_t cfg = {};
@@ -955,10 +1034,14 @@ bool LaunchPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  Failed(cudaLaunchKernelEx(&cfg, GetrfPanelKernel<T>, args), "getrf panel");
+  if (cudaLaunchKernelEx(&cfg, limit != 0 ? GetrfPanelKernel<T, true> : GetrfPanelKernel<T, false>,
+                         args) != cudaSuccess) {
+    cudaGetLastError();  // not launched: the caller goes down the recursion
+    if (t0 != nullptr) cudaEventDestroy(t0);
+    return false;
+  }
   KernelTimerStop(t0, ctx.stream);
   CountLaunch();
-  LaunchFailed("getrf panel");
   return true;
 }
 template <typename T>
@@ -985,6 +1068,10 @@ void LaunchSwapTrsm(int j, int jb, int left, int c0, int nc, T* a, int lda, cons
   LaunchFailed("panel interchanges");
 }
 }  // namespace
+
+void SetPanelWaitLimit(unsigned int polls) {
+  g_panel_polls.store(polls, std::memory_order_relaxed);
+}
 
 template <typename T>
 bool GetrfPanel(int m, int n, T* a, int lda, int* ipiv, int ipiv_add, int* info, int info_base,

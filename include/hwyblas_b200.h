@@ -824,11 +824,13 @@ HWYBLAS_API double hwyblas_fp64_peak_tflops(void);
  * in the reference. */
 HWYBLAS_API double hwyblas_int8_peak_tops(void);
 /* Test hook for the bounded waits: sets how many times each CTA of the LU
- * panel's cooperative pivot exchange (panels of more than 16 x 1024 rows)
- * polls for its peers before it gives up, sets the timeout status (reported
- * as cudaErrorLaunchTimeout by hwyblas_last_cuda_error) and returns; 0
- * restores the default of 2^26. Applies to the current device; returns the
- * previous limit. No counterpart in the reference. */
+ * panel's pivot exchange polls for its peers before it gives up, sets the
+ * timeout status (reported as cudaErrorLaunchTimeout by
+ * hwyblas_last_cuda_error) and returns; 0 restores the defaults. Sets the
+ * limit of the one-launch panels (a process's; default 2^18 polls, each asleep
+ * for up to 4 microseconds, which a set limit's polls are not) and of the
+ * cooperative leaves of taller panels (the current device's; default 2^26),
+ * and returns the latter's previous value. No counterpart in the reference. */
 HWYBLAS_API unsigned int hwyblas_set_leaf_wait_limit(unsigned int polls);
 
 /* IDAMAX that allocates no memory: for callers that must not allocate
