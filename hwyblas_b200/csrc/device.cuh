@@ -13,6 +13,10 @@ namespace hb {
 // Polls before a wait gives up (a poll is tens of ns: far above any real
 // wait, far below a watchdog).
 constexpr uint32_t kMaxPolls = 1u << 26;
+// Polls (a power of two) between looks at the timeout flag in a wait that ends early
+// once another has given up: the flag lies in host memory, and no wait that ends
+// by itself should pay for the trip there.
+constexpr uint32_t kFlagPolls = 1u << 16;
 
 __device__ __forceinline__ uint32_t SmemAddr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -633,7 +633,7 @@ __global__ void __launch_bounds__(kChainThreads, 1)
                          : "l"(cflags + sweep)
                          : "memory");
             if (v == epoch) break;
-            if ((++polls & 255u) == 0 &&
+            if ((++polls & (kFlagPolls - 1)) == 0 &&
                 (*reinterpret_cast<volatile int*>(timeout_flag) != 0 || polls >= kMaxPolls)) {
               atomicExch(timeout_flag, 1);
               good = 0;

@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(kTnThreads, 1) TournamentLeafKernel(TnArgs p) 
       unsigned int d;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(d) : "l"(p.done) : "memory");
       if (d == p.epoch) break;
-      if ((++polls & 255u) == 0 &&
+      if ((++polls & (kFlagPolls - 1)) == 0 &&
           (*reinterpret_cast<volatile int*>(p.timeout_flag) != 0 || polls >= kMaxPolls)) {
         atomicExch(p.timeout_flag, 1);
         good = 0;
