@@ -1099,12 +1099,28 @@ namespace {
 // the SMs about twice (384^3 48 -> 30 us a call; beyond, each tile's loads cost
 // more than its products: 512 x 512 x 1024 69 us against 42 on the DMMA tiles),
 // but for k <= 64 where DgemmShortKKernel can take them (512 x 512 x 64: 27 us a
-// call there, 32 here).
+// call there, 32 here). A CTA multiplies its KC chunks one after another, so that a
+// long k is left to the kernels that spread the chunks over more CTAs. Beyond two
+// chunks a CTA (three for fewer than 16 tiles) that is the split DMMA tiles
+// (33 x 33 x 6000: 46 us here, 53 there; 128 x 128 x 6000 59 and 49, x 30000 256
+// and 90). With a side below 32 it is the chunk kernel, whose time is that of its
+// multiply-adds: beyond four chunks a CTA for tiles that are nearly empty
+// (1 x 1 x 12000: 64 and 53 us, 1 x 3000 x 12000 377 and 320; 1 x 32 x 12000 71 and
+// 77), beyond eight for few elements (16 x 16 x 20000: 95 and 70 us; 31 x 31 x 20000
+// 100 and 188).
 bool SmallTakes(int m, int n, int k, bool small, bool short_k) {
   const int nchunks = (k + 255) / 256, S = std::min(nchunks, kSmCluster);
-  const long long ctas = static_cast<long long>((m + kSmT - 1) / kSmT) * ((n + kSmT - 1) / kSmT) * S;
-  if ((nchunks + S - 1) / S > kSmMaxParts || ctas > (1LL << 30)) return false;
-  return small || (!short_k && ctas <= 2LL * Ctx().num_sms);
+  const int parts = (nchunks + S - 1) / S;
+  const long long tiles =
+      static_cast<long long>((m + kSmT - 1) / kSmT) * ((n + kSmT - 1) / kSmT);
+  if (parts > kSmMaxParts || tiles * S > (1LL << 30)) return false;
+  if (m < 32 || n < 32) {
+    const long long elements = static_cast<long long>(m) * n;
+    const int least = tiles > 1 && parts > 5 ? 64 : 24;  // elements a tile
+    return parts <= 4 || (elements >= least * tiles && (parts <= 8 || elements >= 512));
+  }
+  if (parts > (tiles < 16 ? 3 : 2)) return false;
+  return small || (!short_k && tiles * S <= 2LL * Ctx().num_sms);
 }
 
 void DgemmSmall(int m, int n, int k, double alpha, View<double> a, View<double> b, double beta,

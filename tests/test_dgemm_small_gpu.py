@@ -15,6 +15,10 @@ pytestmark = pytest.mark.gpu
     (1, 1, 1, 0), (31, 33, 63, 1), (32, 32, 64, 0), (33, 47, 65, 2), (64, 8, 255, 0),
     (40, 70, 256, 3), (65, 31, 257, 0), (3, 200, 511, 1), (64, 64, 513, 0), (33, 35, 2049, 1),
     (20, 20, 5000, 0), (300, 1, 3000, 0), (256, 256, 256, 0), (64, 96, 2560, 0),
+    # Either side of the lines for a long k: two to eight chunks a CTA.
+    (128, 100, 4096, 1), (128, 100, 4097, 1), (40, 33, 6144, 1), (40, 33, 6145, 1),
+    (31, 1, 8192, 0), (31, 1, 8193, 0), (1, 32, 10240, 1), (2, 40, 10241, 0), (8, 8, 16384, 0),
+    (8, 8, 16385, 0), (16, 32, 17000, 2), (31, 16, 17000, 0), (64, 1, 33000, 0),
 ])
 def test_dgemm_small_bitexact(hb, orc, ta, tb, m, n, k, pad):
     rng = np.random.default_rng(m + 7 * n + 11 * k)
