@@ -223,21 +223,19 @@ __global__ void __launch_bounds__(kBaseThreads)
 // launch. Bound by latency: up to 16 dependent base solves with an update after
 // each, so all that does not depend on X is on the chip beforehand. A cluster of
 // kTcCtas CTAs takes kTcRhs right-hand sides (their columns are independent): its
-// CTAs hold the triangle's 16-row strips in turn (at most 155 KB each) in shared
-// memory, copied once while the first base is solved, and the next base triangle
-// is copied while one is solved. A base solve gives each warp a right-hand side,
-// an update each warp 16 x 8 tiles of the strips its CTA holds; every element's
-// chains, restarted every KC, and merges are the GEMM kernels'. Steps end with a cluster barrier, which is some 1.5 us less than a
-// grid barrier; X goes through L2. The right side is the left side of the
-// transposed system (each product's factors change places).
+// CTAs hold the triangle's 16-row strips in turn (at most 180 KiB each in FP64, 196.5
+// with the base triangles) in shared memory, copied once while the first base is
+// solved, and the next base triangle is copied while one is solved. A base solve gives
+// each warp a right-hand side, an update each warp 16 x 8 tiles of the strips its CTA
+// holds; every element's chains, restarted every KC, and merges are the GEMM kernels'.
+// Steps end with a cluster barrier, which is some 1.5 us less than a grid barrier; X
+// goes through L2. The right side is the left side of the transposed system (each
+// product's factors change places).
 // 512 rows: few right-hand sides 80 us (168 as a cooperative launch over the grid),
 // 64 a cluster 120 us (512 right-hand sides 140 us with 8 columns a CTA).
 constexpr int kTcRows = 512, kTcThreads = 256, kTcCtas = 8, kTcRhs = 64;
 constexpr int kTcStrip = 16, kTcStrips = kTcRows / kTcStrip / kTcCtas;  // a CTA's strips
 constexpr int kTcLd = kTcStrip + 4;  // conflict-free fragments
-// Sixteen clusters are one wave of the GPU: 900 right-hand sides 143 us (172 as base
-// solves and products), 1500 in a second wave 267 us (192).
-constexpr int kTcMaxOther = 1024;
 
 template <typename T>
 constexpr int kTcKc = sizeof(T) == 8 ? 256 : 384;
@@ -461,27 +459,6 @@ __global__ void __launch_bounds__(kTcThreads) TrsmClusterKernel(TrsmClusterArgs<
 template <typename T>
 bool TrsmCluster(bool left, View<T> tri, bool lower, bool unit, int r, int other, T* b, int ldb) {
   Context& ctx = Ctx();
-  static PerDevice<bool> ready;
-  const auto set = [] {
-    const bool ok =
-        cudaFuncSetAttribute(reinterpret_cast<const void*>(TrsmClusterKernel<T>),
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             TcSmem<T>()) == cudaSuccess;
-    if (!ok) cudaGetLastError();
-    return ok;
-  };
-  if (!ready.Get(set)) return false;
-  TrsmClusterArgs<T> a;
-  a.tri = tri;
-  if (!left) std::swap(a.tri.rs, a.tri.cs);
-  a.lower = left == lower ? 1 : 0;
-  a.unit = unit ? 1 : 0;
-  a.r = r;
-  a.other = other;
-  a.x = b;
-  a.xs = left ? 1 : ldb;
-  a.xr = left ? ldb : 1;
-  a.guard = ctx.guard;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((other + kTcRhs - 1) / kTcRhs * kTcCtas);
   cfg.blockDim = dim3(kTcThreads);
@@ -494,6 +471,34 @@ bool TrsmCluster(bool left, View<T> tri, bool lower, bool unit, int r, int other
   attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
+  // Right-hand sides of one wave: the clusters that the GPU holds at a time (15 here, by
+  // the SMs of its GPCs). A second wave takes nearly as long again, where base solves
+  // and products take little more: 512 rows and 960 right-hand sides 144 us, 1024 267 us
+  // in two waves and 173 as solves and products (65 rows 37, 52 and 45).
+  static PerDevice<int> wave;
+  const auto fit = [&cfg] {
+    const void* fn = reinterpret_cast<const void*>(TrsmClusterKernel<T>);
+    int clusters = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<T>()) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    return clusters * kTcRhs;
+  };
+  if (other > wave.Get(fit)) return false;
+  TrsmClusterArgs<T> a;
+  a.tri = tri;
+  if (!left) std::swap(a.tri.rs, a.tri.cs);
+  a.lower = left == lower ? 1 : 0;
+  a.unit = unit ? 1 : 0;
+  a.r = r;
+  a.other = other;
+  a.x = b;
+  a.xs = left ? 1 : ldb;
+  a.xr = left ? ldb : 1;
+  a.guard = ctx.guard;
   Failed(cudaLaunchKernelEx(&cfg, TrsmClusterKernel<T>, a), "trsm subtree");
   CountLaunch();
   return !LaunchFailed("trsm subtree");
@@ -521,9 +526,7 @@ void TrsmRec(bool left, View<T> tri, bool lower, bool unit, int r, int other,
     TrsmSolve<T>(left, tri, lower, unit, r, other, b, ldb);
     return;
   }
-  if (r <= kTcRows && other <= kTcMaxOther &&
-      TrsmCluster<T>(left, tri, lower, unit, r, other, b, ldb))
-    return;
+  if (r <= kTcRows && TrsmCluster<T>(left, tri, lower, unit, r, other, b, ldb)) return;
   const int r1 = std::max(32, (r / 2) / 32 * 32);
   const int r2 = r - r1;
   const View<T> t11 = tri;

@@ -124,10 +124,11 @@ def test_complex_blocked(hb, orc, p, m, n, ties):
 @pytest.mark.parametrize("uplo", ["L", "U"])
 @pytest.mark.parametrize("trans", ["N", "T"])
 @pytest.mark.parametrize("r,other", [(65, 1), (96, 9), (288, 64), (450, 3), (500, 70), (511, 8),
-                                     (512, 130), (700, 17)])
+                                     (512, 130), (700, 17), (200, 960), (200, 961)])
 def test_trsm_subtrees(hb, orc, p, side, uplo, trans, r, other):
     """Subtrees in one launch: partial blocks, more right-hand sides than a
-    cluster takes, updates deeper than a KC chunk (upper, r = 500 and 511)."""
+    cluster takes, updates deeper than a KC chunk (upper, r = 500 and 511), as many
+    right-hand sides as fit a wave of clusters and one more."""
     rng = np.random.default_rng(r + other)
     m, n = (r, other) if side == "L" else (other, r)
     a = rand(rng, r, r, REAL[p]) / REAL[p](np.sqrt(r))
