@@ -219,6 +219,77 @@ __global__ void __launch_bounds__(kBaseThreads)
   }
 }
 
+// The base solve (r <= 32) with one thread a row: the row in registers in solve order
+// (static indices), the triangle in shared memory, two columns a pass. Bound by the
+// loads once there are rows enough for the SMs; TrsmBaseKernel, a lane an element, is
+// bound by its shuffles by then (right side, 32 x 400000: 312 us, 93 so).
+template <typename T>
+__global__ void __launch_bounds__(128)
+    TrsmRowsKernel(View<T> tri, int lower, int unit, int r, int rows, T* x, long long xs_row,
+                   long long xs_col, Guard guard) {
+  if (guard.Stops()) return;
+  __shared__ T st[32][33];  // st[s][u] = T(col(s), col(u)) in solve order, s < u
+  __shared__ T sinv[32];
+  for (int idx = threadIdx.x; idx < 32 * 32; idx += blockDim.x) {
+    const int s = idx / 32, u = idx % 32;
+    T v = T(0);
+    if (s < r && u < r && (s < u || (s == u && !unit))) {
+      const int q = lower ? r - 1 - s : s, j = lower ? r - 1 - u : u;
+      v = tri.data[q * tri.rs + j * tri.cs];
+    }
+    st[s][u] = v;
+    if (s == u) sinv[s] = s < r && !unit ? T(1) / v : T(1);
+  }
+  __syncthreads();
+  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= rows) return;
+  T* xr = x + row * xs_row;
+  T y[32];
+#pragma unroll
+  for (int s = 0; s < 32; ++s)
+    y[s] = s < r ? xr[(lower ? r - 1 - s : s) * xs_col] : T(0);
+#pragma unroll
+  for (int step = 0; step < 32; step += 2) {
+    if (step >= r) break;
+    T acc0 = y[step], acc1 = y[step + 1];
+#pragma unroll
+    for (int s = 0; s < step; ++s) {
+      acc0 = fma(-y[s], st[s][step], acc0);
+      acc1 = fma(-y[s], st[s][step + 1], acc1);
+    }
+    if (!unit) acc0 = acc0 * sinv[step];
+    y[step] = acc0;
+    acc1 = fma(-acc0, st[step][step + 1], acc1);
+    if (!unit) acc1 = acc1 * sinv[step + 1];
+    y[step + 1] = acc1;
+  }
+#pragma unroll
+  for (int s = 0; s < 32; ++s)
+    if (s < r) xr[(lower ? r - 1 - s : s) * xs_col] = y[s];
+}
+
+// Rows from which a base solve goes to TrsmRowsKernel: where its few long-running
+// threads (27 us a call whatever the number of rows) meet the lanes' time. A call with
+// 32 columns, lanes and rows in us: right side FP64 8000 29 and 28, 16000 34 and 27,
+// FP32 12000 27 and 26; left side, whose loads are not coalesced here, FP64 12000 32
+// and 30, FP32 24000 33 and 34, 32000 36 and 34.
+template <typename T>
+int RowsFrom(bool left) {
+  if (sizeof(T) == 8) return left ? 12000 : 8000;
+  return left ? 24000 : 12000;
+}
+
+// Rows from which a node of 33 to 64 columns is two such solves and a product in
+// launches of their own. Lanes and launches in us: FP64 right side 64 columns 16000 52 and
+// 44, 400000 733 and 250, 33 columns 16000 43 and 42; left side 32000 81 and 66, 24000
+// 55 and 55 (33 columns); FP32 right side 32000 60 and 51, left side 48 columns 64000
+// 88 and 82, 64 columns 100000 137 and 150, 400000 469 and 431.
+template <typename T>
+int SplitFrom(bool left, int r) {
+  if (sizeof(T) == 8) return left ? 24000 : 16000;
+  return !left ? 32000 : r <= 48 ? 64000 : 256000;
+}
+
 // A subtree of the TRSM recursion (65 to kTcRows rows of the triangle) in one
 // launch. Bound by latency: up to 16 dependent base solves with an update after
 // each, so all that does not depend on X is on the chip beforehand. A cluster of
@@ -522,7 +593,7 @@ void LaunchGemm<float>(int m, int n, int k, float alpha, View<float> a,
 template <typename T>
 void TrsmRec(bool left, View<T> tri, bool lower, bool unit, int r, int other,
              T* b, int ldb) {
-  if (r <= kBaseW) {
+  if (r <= 32 || (r <= kBaseW && other < SplitFrom<T>(left, r))) {
     TrsmSolve<T>(left, tri, lower, unit, r, other, b, ldb);
     return;
   }
@@ -594,8 +665,13 @@ void TrsmSolve(bool left, View<T> tri, bool lower, bool unit, int r, int other,
     xs_row = 1;
     xs_col = ldb;
   }
-  TrsmBaseKernel<T><<<(other + kBaseRows - 1) / kBaseRows, kBaseThreads, 0, Ctx().stream>>>(
-      t, lo ? 1 : 0, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
+  if (r <= 32 && other >= RowsFrom<T>(left)) {
+    TrsmRowsKernel<T><<<(other + 127) / 128, 128, 0, Ctx().stream>>>(
+        t, lo ? 1 : 0, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
+  } else {
+    TrsmBaseKernel<T><<<(other + kBaseRows - 1) / kBaseRows, kBaseThreads, 0, Ctx().stream>>>(
+        t, lo ? 1 : 0, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
+  }
   CountLaunch();
   LaunchFailed("trsm base");
 }

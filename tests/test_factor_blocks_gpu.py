@@ -75,6 +75,28 @@ def test_trsm_bases(hb, orc, p, side, uplo, trans, diag, r):
         assert same_bits(x1, x2), (other, first_diff(x1, x2))
 
 
+@pytest.mark.parametrize("p", ["d", "s"])
+@pytest.mark.parametrize("side", ["L", "R"])
+@pytest.mark.parametrize("uplo", ["L", "U"])
+@pytest.mark.parametrize("diag", ["N", "U"])
+@pytest.mark.parametrize("r", [1, 2, 15, 31, 32, 33, 47, 64])
+def test_trsm_bases_many_rows(hb, orc, p, side, uplo, diag, r):
+    """Either side of the lines between a lane an element and a thread a row, and
+    between one launch and three."""
+    lines = {("d", "L"): (12000, 24000), ("d", "R"): (8000, 16000), ("s", "L"): (24000, 64000),
+             ("s", "R"): (12000, 32000)}[p, side]
+    rng = np.random.default_rng(r)
+    a = rand(rng, r, r, REAL[p]) / REAL[p](np.sqrt(r))
+    a = np.asfortranarray(a + np.diag(np.full(r, 1.5)).astype(REAL[p]))
+    for other in (lines[r > 32] - 1, lines[r > 32] + 1):
+        m, n = (r, other) if side == "L" else (other, r)
+        b = rand(rng, m + 1, n, REAL[p])
+        x1, x2 = b.copy(order="F"), b.copy(order="F")
+        getattr(hb, f"{p}trsm")(side, uplo, "N", diag, m, n, 1.0, a, r, x1, m + 1)
+        getattr(orc, f"{p}trsm")(side, uplo, "N", diag, m, n, REAL[p](1.0), a, r, x2, m + 1)
+        assert same_bits(x1, x2), (other, first_diff(x1, x2))
+
+
 def check_zgetrf(hb, orc, p, a, recursive):
     m, n = a.shape
     a1, a2 = a.copy(order="F"), a.copy(order="F")
