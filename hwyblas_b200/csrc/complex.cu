@@ -1206,13 +1206,18 @@ static void ZTrsmRec(bool left, ZView<R> tri, bool lower, bool unit, int r, int 
       xs_row = 1;
       xs_col = ldb;
     }
-    if (!lo) {
+    // From so many rows on a thread a row is faster for an upper T too (times in us,
+    // lanes and rows, 32 columns: right side, FP64 4000 35 and 34, 100000 237 and 69, FP32
+    // 4000 32 and 32; left side, whose loads are not coalesced there, FP64 8000 40 and
+    // 40, FP32 12000 40 and 38).
+    const int rows_from = !left ? 4000 : sizeof(R) == 8 ? 8000 : 12000;
+    if (!lo && other < rows_from) {
       ZTrsmLaneKernel<R>
           <<<(other + kZLaneRows - 1) / kZLaneRows, kZLaneThreads, 0, Ctx().stream>>>(
               t, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
     } else {
       ZTrsmBaseKernel<R><<<(other + 127) / 128, 128, 0, Ctx().stream>>>(
-          t, 1, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
+          t, lo ? 1 : 0, unit ? 1 : 0, r, other, b, xs_row, xs_col, Ctx().guard);
     }
     CountLaunch();
     LaunchFailed("complex trsm base");

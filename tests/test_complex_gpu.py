@@ -157,6 +157,25 @@ def test_ztrsm_bitexact(hb, orc, p, side, uplo, trans, diag):
 
 
 @pytest.mark.parametrize("p", ["z", "c"])
+@pytest.mark.parametrize("side,uplo,trans", [("L", "L", "N"), ("R", "U", "N"), ("L", "U", "C"),
+                                             ("R", "L", "T")])
+@pytest.mark.parametrize("r", [1, 31, 32, 40])
+def test_ztrsm_many_rows(hb, orc, p, side, uplo, trans, r):
+    """Base solves either side of the lines between a lane an element and a thread a row."""
+    line = 4000 if side == "R" else 8000 if p == "z" else 12000
+    rng = np.random.default_rng(r)
+    t = np.complex128 if p == "z" else np.complex64
+    a = np.asfortranarray((crand(rng, r, r, t) / np.sqrt(r) + 2 * np.eye(r)).astype(t))
+    for other in (line - 1, line):
+        m, n = (r, other) if side == "L" else (other, r)
+        b = crand(rng, m + 1, n, t)
+        b1, b2 = b.copy(order="F"), b.copy(order="F")
+        hb.ztrsm(p, side, uplo, trans, "N", m, n, 1.0, a, r, b1, m + 1)
+        assert orc.ztrsm(side, uplo, trans, "N", m, n, 1.0, a, r, b2, m + 1) == 0
+        assert same_bits(creal(b1), creal(b2)), other
+
+
+@pytest.mark.parametrize("p", ["z", "c"])
 def test_ztrsm_diagonal_reciprocals(hb, orc, p):
     """The device's 1/t(j, j) against the C++ runtime's complex quotient (the
     reference's), through diagonal triangles: magnitudes 2^-40..2^40 and
