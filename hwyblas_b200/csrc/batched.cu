@@ -605,7 +605,6 @@ struct LuShared {
   T rinv;
   // The rows that a leaf's interchanges moved: new and old position.
   int moves, dst[kMovesMax], src[kMovesMax];
-  int perm[kPermMax];  // a solve's row order
 };
 
 // LU leaf of an m x w block (w <= 16, m >= w): partial pivoting with the
@@ -906,7 +905,8 @@ __device__ void CtaGetrf(int n, Mat<T> a, int* ipiv, int* info, int lanes,
 }
 
 // All n interchanges of a solve on B's columns (backward: from the last): replayed
-// on the row order in shared memory, then each column is one gather.
+// on the row order, then a batch of whole columns is one gather. The order and the
+// pivots are in the triangle's place, 16 bits each.
 template <typename T>
 __device__ void CtaSolveSwaps(bool backward, int n, int nrhs, Mat<T> b, const int* ipiv,
                               LuShared<T>& sh) {
@@ -916,35 +916,41 @@ __device__ void CtaSolveSwaps(bool backward, int n, int nrhs, Mat<T> b, const in
     else CtaLaswp(nrhs, b, 1, n, ipiv);
     return;
   }
-  static_assert(sizeof(sh.st) >= sizeof(sh.perm), "the pivots fit the triangle's place");
-  int* piv = reinterpret_cast<int*>(sh.st);
+  static_assert(sizeof(sh.st) >= 2 * kPermMax * sizeof(unsigned short), "they fit there");
+  unsigned short* perm = reinterpret_cast<unsigned short*>(sh.st);
+  unsigned short* piv = perm + kPermMax;
+  bool moves = false;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    sh.perm[i] = i;
-    piv[i] = ipiv[i];
+    const int p = ipiv[i] - 1;
+    moves |= p != i;
+    perm[i] = static_cast<unsigned short>(i);
+    piv[i] = static_cast<unsigned short>(p);
   }
-  __syncthreads();
+  if (!__syncthreads_or(moves)) return;
   if (threadIdx.x == 0) {
     for (int s = 0; s < n; ++s) {
-      const int i = backward ? n - 1 - s : s, p = piv[i] - 1;
+      const int i = backward ? n - 1 - s : s, p = piv[i];
       if (p == i) continue;
-      const int t = sh.perm[i];
-      sh.perm[i] = sh.perm[p];
-      sh.perm[p] = t;
+      const unsigned short t = perm[i];
+      perm[i] = perm[p];
+      perm[p] = t;
     }
   }
   __syncthreads();
-  for (int c = 0; c < nrhs; ++c) {
+  const int per = kPer * blockDim.x / n;  // columns of a batch
+  for (int c0 = 0; c0 < nrhs; c0 += per) {
+    const int items = min(per, nrhs - c0) * n;
     T v[kPer];
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      if (i < n) v[k] = b(sh.perm[i], c);
+      const int idx = threadIdx.x + k * blockDim.x;
+      if (idx < items) v[k] = b(perm[idx % n], c0 + idx / n);
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-      const int i = threadIdx.x + k * blockDim.x;
-      if (i < n && sh.perm[i] != i) b(i, c) = v[k];
+      const int idx = threadIdx.x + k * blockDim.x;
+      if (idx < items && perm[idx % n] != idx % n) b(idx % n, c0 + idx / n) = v[k];
     }
   }
   __syncthreads();

@@ -26,3 +26,33 @@ def test_batched_lu_interchanges(hb, cuda, p):
         for n, x, y, q, r in zip(sizes, got, want, piv, wpiv):
             assert torch.equal(q, r), n
             assert torch.equal(x, y), n
+
+
+@pytest.mark.parametrize("p", ["d", "s"])
+@pytest.mark.parametrize("trans", ["N", "T"])
+@pytest.mark.parametrize("config", [64, 256])
+def test_batched_solve_interchanges(hb, cuda, p, trans, config):
+    """Whole columns a batch (small n, many right-hand sides), one column or less a
+    thread, more rows than the order in shared memory holds; no interchange at all."""
+    torch = cuda
+    t = torch.float64 if p == "d" else torch.float32
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    sizes = [1, 2, 7, 16, 63, 64, 65, 255, 256, 257, 512, 513, 1000, 1024, 1025, 100]
+    rhs = [40, 33, 40, 17, 3, 40, 5, 2, 9, 3, 2, 3, 1, 2, 2, 6]
+    a = [torch.rand(n * n, dtype=t, device="cuda", generator=gen) * 2 - 1 for n in sizes]
+    a[-1].view(100, 100).diagonal().add_(200)  # pivots on the diagonal
+    piv = [torch.zeros(n, dtype=torch.int32, device="cuda") for n in sizes]
+    b = [torch.rand(n * r, dtype=t, device="cuda", generator=gen) for n, r in zip(sizes, rhs)]
+    getrf, getrs = (hb.dgetrf, hb.dgetrs) if p == "d" else (hb.sgetrf, hb.sgetrs)
+    want = [x.clone() for x in b]
+    for n, r, x, q, y in zip(sizes, rhs, a, piv, want):
+        assert getrf(n, n, x, n, q) == 0
+        assert getrs(trans, n, r, x, n, q, y, n) == 0
+    old = hb.lib().hwyblas_batched_set_config(config)
+    try:
+        assert hb.getrs_batched(trans, sizes, rhs, a, sizes, piv, b, sizes, precision=p) == 0
+    finally:
+        hb.lib().hwyblas_batched_set_config(old)
+    torch.cuda.synchronize()
+    for n, x, y in zip(sizes, b, want):
+        assert torch.equal(x, y), n
