@@ -121,7 +121,12 @@ struct DmmaTile {
   static constexpr int kLoadB = kDmmaKb * kTN / kThreads;
 };
 
-template <int WM, int WN, int NB>
+// kNarrow: of a tile that C does not fill, a warp issues only the MMAs whose 16 x 8
+// block holds elements, so that the other warps have the tensor pipe to themselves.
+// For solves with few right-hand sides (n = 512, 8 of them, 200 problems: 385 us
+// without, 297 with); in the LU and the GEMM the question costs more than it saves
+// (GEMM n = 512, 200 problems: 4.07 ms with, 3.78 without; LU 4.69 and 4.46).
+template <int WM, int WN, int NB, bool kNarrow>
 __device__ void CtaGemmDmma(int m, int n, int k, double alpha, Mat<double> a, Mat<double> b,
                             double beta, Mat<double> c, double* sA, double* sB) {
   using Cfg = DmmaTile<WM, WN, NB>;
@@ -129,8 +134,6 @@ __device__ void CtaGemmDmma(int m, int n, int k, double alpha, Mat<double> a, Ma
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int wm = warp % WM, wn = warp / WM;
   const int g = lane >> 2, t = lane & 3;
-  // A warp issues only the MMAs whose 16 x 8 block holds elements of C: at the
-  // ragged edge the other warps have the tensor pipe to themselves.
   // Operand loads: along the contiguous index of each operand.
   const bool a_rows = a.rs == 1;  // A(i, q) contiguous in i
   const bool b_rows = b.rs == 1;  // B(q, j) contiguous in q
@@ -183,13 +186,13 @@ __device__ void CtaGemmDmma(int m, int n, int k, double alpha, Mat<double> a, Ma
           __syncthreads();
           if (kb0 + kDmmaKb < k) fetch(kb0 + kDmmaKb);
           const int steps =
-              m0 + wm * 16 < m ? (min(pe, kb0 + kDmmaKb) - kb0 + 7) / 8 : 0;
+              !kNarrow || m0 + wm * 16 < m ? (min(pe, kb0 + kDmmaKb) - kb0 + 7) / 8 : 0;
           for (int ks = 0; ks < steps; ++ks) {
             const double* pa = sA + (ks * 8 + t) * SA + wm * 16 + g;
             const double a0 = pa[0], a1 = pa[8], a2 = pa[4 * SA], a3 = pa[4 * SA + 8];
 #pragma unroll
             for (int nb = 0; nb < NB; ++nb) {
-              if (n0 + (wn * NB + nb) * 8 >= n) break;
+              if (kNarrow && n0 + (wn * NB + nb) * 8 >= n) break;
               const double* pb = sB + (ks * 8 + t) * SB + wn * 8 * NB + nb * 8 + g;
               BatchDmma(acc[nb], a0, a1, a2, a3, pb[0], pb[4 * SB]);
             }
@@ -338,8 +341,8 @@ __device__ void CtaGemmReg(int m, int n, int k, T alpha, Mat<T> a, Mat<T> b, T b
 
 // The GEMM a batched factorization or solve calls for its updates: the
 // per-element chains (any type, any CTA size) or, in FP64, the tensor-pipe
-// tiles for blocks of at least 16 x 16 (the CTA has the tile's warps). Both
-// give every element the same bits.
+// tiles for blocks of at least 16 rows and 4 columns (the CTA has the tile's
+// warps). Both give every element the same bits.
 template <typename T>
 struct ElemGemm {
   __device__ void operator()(int m, int n, int k, T alpha, Mat<T> a, Mat<T> b, T beta,
@@ -361,7 +364,7 @@ struct RegGemm {
   }
 };
 
-template <int WM, int WN, int NB>
+template <int WM, int WN, int NB, bool kNarrow>
 struct TileGemm {
   double* sA;
   double* sB;
@@ -370,7 +373,7 @@ struct TileGemm {
     if (m < 16 || n < 4)
       CtaGemm<double>(m, n, k, alpha, a, b, beta, c);
     else
-      CtaGemmDmma<WM, WN, NB>(m, n, k, alpha, a, b, beta, c, sA, sB);
+      CtaGemmDmma<WM, WN, NB, kNarrow>(m, n, k, alpha, a, b, beta, c, sA, sB);
   }
 };
 
@@ -1090,7 +1093,7 @@ __global__ void __launch_bounds__(DmmaTile<WM, WN, NB>::kThreads, MinBlocks)
   __shared__ double sA[kDmmaKb * Cfg::kSA];
   __shared__ double sB[kDmmaKb * Cfg::kSB];
   __shared__ int slot;
-  RunProblems<Kind>(p, TileGemm<WM, WN, NB>{sA, sB}, sh, &slot);
+  RunProblems<Kind>(p, TileGemm<WM, WN, NB, Kind != kDevGetrf>{sA, sB}, sh, &slot);
 }
 
 template <typename T, int Threads>
@@ -1151,7 +1154,7 @@ __global__ void __launch_bounds__(DmmaTile<WM, WN, NB>::kThreads,
     if (m < 16 || n < 16) {
       CtaGemm<double>(m, n, k, p.alpha, a, b, p.beta, c);
     } else {
-      CtaGemmDmma<WM, WN, NB>(m, n, k, p.alpha, a, b, p.beta, c, sA, sB);
+      CtaGemmDmma<WM, WN, NB, false>(m, n, k, p.alpha, a, b, p.beta, c, sA, sB);
     }
   }
 }
