@@ -97,7 +97,7 @@ def test_trsm_bases_many_rows(hb, orc, p, side, uplo, diag, r):
         assert same_bits(x1, x2), (other, first_diff(x1, x2))
 
 
-def check_zgetrf(hb, orc, p, a, recursive):
+def check_zgetrf(hb, orc, p, a, recursive, columns=None):
     m, n = a.shape
     a1, a2 = a.copy(order="F"), a.copy(order="F")
     p1, p2 = np.zeros(min(m, n), np.int32), np.zeros(min(m, n), np.int32)
@@ -106,7 +106,7 @@ def check_zgetrf(hb, orc, p, a, recursive):
     assert i1 == i2
     assert np.array_equal(p1, p2), np.flatnonzero(p1 != p2)[:4]
     r = REAL["d" if p == "z" else "s"]
-    b1, b2 = a1.T.view(r), a2.T.view(r)  # row by row: column by column of a
+    b1, b2 = a1.T.view(r)[:columns], a2.T.view(r)[:columns]  # row by row: column by column of a
     assert same_bits(b1, b2), first_diff(b1, b2)
 
 
@@ -139,6 +139,22 @@ def test_complex_blocked(hb, orc, p, m, n, ties):
                               .astype(a.dtype))
         a[:, 5] = a[:, 3]
     check_zgetrf(hb, orc, p, a, False)
+
+
+@pytest.mark.parametrize("p", ["z", "c"])
+@pytest.mark.parametrize("m", [40, 600])
+@pytest.mark.parametrize("place", ["first", "middle", "all"])
+@pytest.mark.parametrize("re,im", [(np.nan, 0), (0, np.nan), (np.inf, 1), (0, -np.inf),
+                                   (np.inf, np.nan)])
+def test_complex_panel_special_values(hb, orc, p, m, place, re, im):
+    """NaN anywhere; infinities in the last column, whose search they go through (what
+    the C runtime recovers from quotients of infinities is not reproduced)."""
+    rng = np.random.default_rng(m)
+    infinite = np.isinf([re, im]).any()
+    a = crand(rng, p, m, 21 if infinite else 36)
+    rows = {"first": [0], "middle": [m // 2], "all": list(range(m))}[place]
+    a[rows, 20] = complex(re, im)
+    check_zgetrf(hb, orc, p, a, True, columns=20 if infinite else None)
 
 
 @pytest.mark.parametrize("p", ["d", "s"])

@@ -14,6 +14,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k,pad", [
     (1, 1, 1, 0), (63, 31, 15, 1), (64, 32, 16, 0), (65, 33, 17, 3), (130, 129, 383, 2),
     (128, 64, 384, 4), (129, 100, 385, 0), (200, 70, 800, 5),
+    # 128 x 64 tiles, either side of the 24 from which they are taken.
+    (512, 384, 64, 0), (512, 385, 33, 1), (640, 320, 385, 4), (513, 449, 385, 3),
+    (640, 640, 400, 0), (129, 770, 50, 2),
     (1601, 1540, 20, 3), (1664, 1536, 400, 0),  # at least 148 tiles of 128 x 128
 ])
 def test_sgemm_tiles_bitexact(hb, orc, ta, tb, m, n, k, pad):
@@ -52,7 +55,7 @@ def test_sgemm_tiles_device_alignment(hb, orc, cuda, offset):
 
 
 @pytest.mark.parametrize("uplo", ["L", "U"])
-@pytest.mark.parametrize("n,k", [(65, 17), (300, 400), (2000, 30)])
+@pytest.mark.parametrize("n,k", [(65, 17), (300, 400), (600, 385), (2000, 30)])
 def test_ssyrk_tiles_bitexact(hb, orc, uplo, n, k):
     rng = np.random.default_rng(n + k)
     a, c = rand(rng, n, k, np.float32), rand(rng, n, n, np.float32)
