@@ -1267,23 +1267,34 @@ int ThreadsOf(int config) {
                                : config;
 }
 
+// three: three CTAs of 256 threads an SM, which spill registers, instead of two.
 template <int Kind, typename T>
-void* LuKernelOf(int config) {
+void* LuKernelOf(int config, bool three) {
   if constexpr (sizeof(T) == 8) {
     if (config == kDmma32) return reinterpret_cast<void*>(BatchedLuDmmaKernel<Kind, 2, 2, 2, 4>);
-    if (config == kDmma64) return reinterpret_cast<void*>(BatchedLuDmmaKernel<Kind, 4, 2, 4, 2>);
+    if (config == kDmma64)
+      return three ? reinterpret_cast<void*>(BatchedLuDmmaKernel<Kind, 4, 2, 4, 3>)
+                   : reinterpret_cast<void*>(BatchedLuDmmaKernel<Kind, 4, 2, 4, 2>);
   }
   if (config == 64) return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 64, 8>);
   if (config == 128) return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 128, 4>);
   if (config == kDense128) return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 128, 6>);
-  return reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 256, 2>);
+  return three ? reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 256, 3>)
+               : reinterpret_cast<void*>(BatchedLuKernel<Kind, T, 256, 2>);
 }
 
+// Three CTAs of 256 threads an SM are for batches that two do not hold at a time, as
+// long as three do (FP64 n = 400, 300 problems: LU 5.11 ms with two, 3.96 with three, and
+// 800 problems 9.06 and 9.28; solves of 40 right-hand sides, 300 problems 719 and 683 us,
+// 800 1253 and 1449); FP32 solves, which spill less, from there on (n = 400, 40 right-hand
+// sides: 300 problems 513 and 397 us, 800 888 and 817).
 template <typename T>
-void* KernelOf(int kind, int config) {
-  if (kind == kBatchGetrf) return LuKernelOf<kDevGetrf, T>(config);
-  if (kind == kBatchGetrs) return LuKernelOf<kDevGetrs, T>(config);
-  if (kind == kBatchTrsm) return LuKernelOf<kDevTrsm, T>(config);
+void* KernelOf(int kind, int config, int count, int sms) {
+  const bool three = count > 2 * sms && (count <= 3 * sms ||
+                                         (sizeof(T) == 4 && kind != kBatchGetrf));
+  if (kind == kBatchGetrf) return LuKernelOf<kDevGetrf, T>(config, three);
+  if (kind == kBatchGetrs) return LuKernelOf<kDevGetrs, T>(config, three);
+  if (kind == kBatchTrsm) return LuKernelOf<kDevTrsm, T>(config, three);
   if (sizeof(T) == 8 && config == kDmma32)
     return reinterpret_cast<void*>(BatchedGemmDmmaKernel<2, 2, 2>);
   if (sizeof(T) == 8 && config == kDmma64)
@@ -1422,7 +1433,7 @@ bool LaunchBatch(int kind, const HostBatch<T>& bt, int config, int** dev_info,
   args.beta = bt.beta;
   args.flags = bt.flags;
   args.lanes = sizeof(T) == 8 ? RefLanesDouble() : 2 * RefLanesDouble();
-  void* fn = KernelOf<T>(kind, config);
+  void* fn = KernelOf<T>(kind, config, count, ctx.num_sms);
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, 0);
   const int grid = std::max(1, std::min(count, ctx.num_sms * std::max(per_sm, 1)));

@@ -56,3 +56,38 @@ def test_batched_solve_interchanges(hb, cuda, p, trans, config):
     torch.cuda.synchronize()
     for n, x, y in zip(sizes, b, want):
         assert torch.equal(x, y), n
+
+
+@pytest.mark.parametrize("p", ["d", "s"])
+@pytest.mark.parametrize("config", [256, 1002])
+@pytest.mark.parametrize("count", [290, 300, 450])
+def test_batched_ctas_an_sm(hb, cuda, p, config, count):
+    """Batches that two CTAs of 256 threads an SM hold, that three do, and larger ones:
+    LU, solve and TRSM equal to the 64-thread configuration's."""
+    torch = cuda
+    if p == "s" and config == 1002:
+        pytest.skip("FP64 only")
+    t = torch.float64 if p == "d" else torch.float32
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    n = 72
+    a0 = torch.rand(count, n, n, dtype=t, device="cuda", generator=gen) * 2 - 1
+    b0 = torch.rand(count, 5, n, dtype=t, device="cuda", generator=gen)
+    sizes, rhs = [n] * count, [5] * count
+
+    def run(cfg):
+        a, b, x = a0.clone(), b0.clone(), b0.clone()
+        piv = torch.zeros(count, n, dtype=torch.int32, device="cuda")
+        old = hb.lib().hwyblas_batched_set_config(cfg)
+        try:
+            info = hb.getrf_batched(sizes, list(a), sizes, list(piv), precision=p)
+            hb.getrs_batched("N", sizes, rhs, list(a), sizes, list(piv), list(b), sizes, precision=p)
+            hb.trsm_batched("L", "L", "N", "U", sizes, rhs, 1.0, list(a), sizes, list(x), sizes,
+                            precision=p)
+        finally:
+            hb.lib().hwyblas_batched_set_config(old)
+        torch.cuda.synchronize()
+        assert info == [0] * count
+        return a, piv, b, x
+
+    for got, want in zip(run(config), run(64)):
+        assert torch.equal(got, want)
