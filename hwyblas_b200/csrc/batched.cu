@@ -431,8 +431,10 @@ __device__ void CtaTrsmBase(Mat<T> t, bool lower, bool unit, int r, int other, T
     sinv[s] = (s < r && !unit) ? T(1) / st[s][s] : T(1);
   }
   __syncthreads();
-  if (2 * other <= static_cast<int>(blockDim.x)) {
-    // Few rows: two a warp, a lane an element, instead of a thread a row.
+  if ((sizeof(T) == 8 ? 4 : 2) * other <= static_cast<int>(blockDim.x)) {
+    // Few rows: two a warp, a lane an element, instead of a thread a row. (Up to four
+    // rounds of the CTA's warps in FP64, whose shuffles are two each, eight in FP32:
+    // FP64 n = 200, 64 rows on 4 warps 432 us with eight rounds, 354 a thread a row.)
     const int lane = threadIdx.x % 32;
     const long long at = (lower ? r - 1 - lane : lane) * xs_col;
     for (int row = threadIdx.x / 32 * 2; row < other; row += blockDim.x / 16) {
