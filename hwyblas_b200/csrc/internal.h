@@ -57,9 +57,8 @@ struct Guard {
   int limit = INT_MAX;
 #ifdef __CUDACC__
   __device__ __forceinline__ bool Stops() const {
-    if (info == nullptr) return false;
-    const int v = *info;
-    return v != 0 && v <= limit;
+    return info != nullptr &&
+           static_cast<unsigned>(*info - 1) < static_cast<unsigned>(limit);
   }
 #endif
 };
