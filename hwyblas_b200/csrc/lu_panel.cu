@@ -17,7 +17,7 @@
 // What bounds a column now is one warp's chain of instructions, some 1700 cycles at
 // 256 rows: two rows a thread, with one busy warp a scheduler, made 256 x 64
 // 96 us instead of 79. 4096 x 64: 400 us as leaves, interchanges, solves and
-// products, 119 us so. Per column: the warps' maxima by
+// products, 113 us so. Per column: the warps' maxima by
 // redux on the bits of |x|, one block barrier, the block's candidate row sent
 // to every CTA of the cluster by st.async (one one-way trip; the receiving
 // mbarrier counts the bytes), and every warp picks the winner by itself.
