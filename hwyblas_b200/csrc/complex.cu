@@ -847,7 +847,10 @@ __global__ void __launch_bounds__(kZLeafThreads) ZGetrfLeafKernel(ZLeafArgs<R> p
         }
       }
       __syncthreads();
-      if (s_abort) return;
+      if (s_abort) {  // pivots that stay in range for the interchanges that follow
+        if (cta == 0 && threadIdx.x >= j && threadIdx.x < w) p.ipiv[threadIdx.x] = threadIdx.x + 1;
+        return;
+      }
       for (int idx = threadIdx.x; idx < P * kZSlot; idx += blockDim.x)
         s_cand[idx] = *(volatile const R*)&p.xchg[par * P * kZSlot + idx];
     }

@@ -495,7 +495,10 @@ __global__ void __launch_bounds__(kLeafThreads)
         }
       }
       __syncthreads();
-      if (s_abort) return;
+      if (s_abort) {  // pivots that stay in range for the interchanges that follow
+        if (cta == 0 && threadIdx.x >= j && threadIdx.x < w) p.ipiv[threadIdx.x] = threadIdx.x + 1;
+        return;
+      }
       for (int idx = threadIdx.x; idx < P * slot_len; idx += blockDim.x)
         s_cand[idx] = *(volatile const T*)&cand[par * P * slot_len + idx];
       __syncthreads();

@@ -19,12 +19,14 @@ CUDA_ERROR_LAUNCH_TIMEOUT = 702  # cudaErrorLaunchTimeout
 DEFAULT_POLLS = 1 << 26
 
 
-def test_leaf_wait_times_out_reports_and_recovers(hb, orc):
+@pytest.mark.parametrize("n", [16, 40])
+def test_leaf_wait_times_out_reports_and_recovers(hb, orc, n):
     lib = hb.lib()
     rng = np.random.default_rng(12)
     # 59 CTAs of 1024 rows: beyond the 16-CTA cluster, so the cooperative
-    # variant with polled global slots runs.
-    m, n = 60000, 16
+    # variant with polled global slots runs. One leaf, and leaves with
+    # interchanges by their pivots between them.
+    m = 60000
     a0 = rand(rng, m, n)
     lib.hwyblas_last_cuda_error()  # clear
     prev = lib.hwyblas_set_leaf_wait_limit(1)
@@ -34,6 +36,7 @@ def test_leaf_wait_times_out_reports_and_recovers(hb, orc):
         ipiv = np.zeros(n, np.int32)
         hb.dgetrf2(m, n, a, m, ipiv)
         assert lib.hwyblas_last_cuda_error() == CUDA_ERROR_LAUNCH_TIMEOUT
+        assert ipiv.min() >= 1 and ipiv.max() <= m
     finally:
         assert lib.hwyblas_set_leaf_wait_limit(0) == 1
     a1, a2 = a0.copy(order="F"), a0.copy(order="F")
